@@ -840,9 +840,14 @@ k_emit(const K* __restrict__ keys, uint32_t n, const uint4* __restrict__ knode, 
     }
     if (gn)
     {
+        // a NaN plane (from a NaN vertex) makes the traversal take the general box test
+        bool nan = false;
+        for (int k = 0; k < 3; k++) { nan |= b.mn[k] != b.mn[k] || b.mx[k] != b.mx[k]; }
+        if (nan) { *reinterpret_cast<uint32_t*>(root + 1) = 1u; }
         // the traversal layout (a tree without SAH subtrees): this node's box, reference and
-        // count in its parent's 64-byte record -- the left child's half is floats 0-5 and words
-        // 12 / 14, the right child's floats 6-11 and words 13 / 15 -- or the entry record (the root)
+        // count in its parent's 64-byte record -- the left child's half is floats 0-5 (the two
+        // planes of each axis together) and words 12 / 14, the right child's floats 6-11 and words
+        // 13 / 15 -- or the entry record (the root)
         const uint32_t ref = is_m ? pre : (stri ? stri[f] : f);
         const uint32_t cnt = is_m ? 0u : (LEAF_BIT | (l - f + 1u));
         const uint32_t par = parent[x];
@@ -863,12 +868,12 @@ k_emit(const K* __restrict__ keys, uint32_t n, const uint4* __restrict__ knode, 
         uint32_t* gu = reinterpret_cast<uint32_t*>(g);
         if (left)
         {
-            g[0] = b.mn[0]; g[1] = b.mn[1]; g[2] = b.mn[2]; g[3] = b.mx[0]; g[4] = b.mx[1]; g[5] = b.mx[2];
+            g[0] = b.mn[0]; g[1] = b.mx[0]; g[2] = b.mn[1]; g[3] = b.mx[1]; g[4] = b.mn[2]; g[5] = b.mx[2];
             gu[12] = ref; gu[14] = cnt;
         }
         else
         {
-            g[6] = b.mn[0]; g[7] = b.mn[1]; g[8] = b.mn[2]; g[9] = b.mx[0]; g[10] = b.mx[1]; g[11] = b.mx[2];
+            g[6] = b.mn[0]; g[7] = b.mx[0]; g[8] = b.mn[1]; g[9] = b.mx[1]; g[10] = b.mn[2]; g[11] = b.mx[2];
             gu[13] = ref; gu[15] = cnt;
         }
     }
@@ -1082,7 +1087,7 @@ __global__ void __launch_bounds__(BLK)
 k_clear(uint32_t n, uint32_t* __restrict__ parent, uint8_t* __restrict__ kflag, uint32_t* __restrict__ wnode,
         uint32_t* __restrict__ wtri, uint8_t* __restrict__ kpos, uint32_t* __restrict__ scene, uint32_t n_scene_boxes,
         uint32_t* __restrict__ hist, uint32_t* __restrict__ counters, uint32_t* __restrict__ status,
-        uint32_t* __restrict__ lookback, uint32_t n_lookback, uint32_t* __restrict__ tile_counters)
+        uint32_t* __restrict__ lookback, uint32_t n_lookback, uint32_t* __restrict__ tile_counters, uint32_t* __restrict__ odd)
 {
     const uint32_t i = blockIdx.x * BLK + threadIdx.x;
     if (i < n_lookback) { lookback[i] = 0u; }  // the radix sort's look-back words (all its passes)
@@ -1098,7 +1103,7 @@ k_clear(uint32_t n, uint32_t* __restrict__ parent, uint8_t* __restrict__ kflag, 
         const int t = threadIdx.x;
         for (int k = t; k < 9 * 256; k += BLK) { hist[k] = 0u; }
         if (t < 16) { counters[t] = 0u; }
-        if (t == 0) { *status = 0u; }
+        if (t == 0) { *status = 0u; *odd = 0u; }
     }
 }
 
@@ -1161,7 +1166,7 @@ int build_typed(rt_bvh* B, const rt_vertex* d_verts, uint32_t V, const rt_triang
         k_clear<<<blocks_for(std::max<uint32_t>(std::max<uint32_t>(N + 1, 6 * n_boxes), (uint32_t)n_lookback)), BLK, 0, st>>>(
             N, S.parent.as<uint32_t>(), S.kflag.as<uint8_t>(), S.wnode.as<uint32_t>(), S.wtri.as<uint32_t>(),
             S.bnd.as<uint8_t>(), S.scene.as<uint32_t>(), n_boxes, S.hist.as<uint32_t>(), counters, status,
-            S.sort.lookback.as<uint32_t>(), (uint32_t)n_lookback, S.sort.tile_counters.as<uint32_t>());
+            S.sort.lookback.as<uint32_t>(), (uint32_t)n_lookback, S.sort.tile_counters.as<uint32_t>(), reinterpret_cast<uint32_t*>(B->rootbuf.as<TraceRoot>() + 1));
         count_launch();
         k_vertices<<<blocks_for(V), BLK, 0, st>>>(d_verts, B->verts.as<rt_vertex>(), V);
         count_launch();
@@ -1515,7 +1520,7 @@ int build_bvh_batch(rt_bvh* B, const rt_vertex* d_verts, uint32_t V, const rt_tr
     if (cap < N) { cap = N; }
     const size_t max_nodes = (size_t)cap * 2 - 1;  // bvh_bfs.cpp:58
     if (B->tripos.ensure((size_t)cap * 48) ||  // written by k_emit_tris in builds without SAH subtrees
-        B->gnodes.ensure(max_nodes * sizeof(rt_gnode)) || B->rootbuf.ensure(sizeof(TraceRoot)) ||  // and by k_emit
+        B->gnodes.ensure(max_nodes * sizeof(rt_gnode)) || B->rootbuf.ensure(ROOT_RECORD_BYTES) ||  // and by k_emit
         B->nodes.ensure(max_nodes * sizeof(rt_bvh_node)) || B->tris.ensure((size_t)cap * sizeof(rt_triangle)) ||
         B->prim.ensure((size_t)cap * 4) || B->verts.ensure((size_t)V * sizeof(rt_vertex)))
     {

@@ -142,9 +142,9 @@ int exclusive_scan_u32(const uint32_t* in, uint32_t* out, uint32_t n, uint32_t* 
 // leaf child (ref = first triangle), 0 for an inner child (ref = node index).
 struct rt_gnode
 {
-    float4 a;  // l.min.x l.min.y l.min.z l.max.x
-    float4 b;  // l.max.y l.max.z r.min.x r.min.y
-    float4 c;  // r.min.z r.max.x r.max.y r.max.z
+    float4 a;  // l.min.x l.max.x l.min.y l.max.y
+    float4 b;  // l.min.z l.max.z r.min.x r.max.x
+    float4 c;  // r.min.y r.max.y r.min.z r.max.z
     uint4  d;  // l.ref   r.ref   l.cnt   r.cnt
 };
 

@@ -92,6 +92,10 @@ struct TraceRoot
     uint32_t ref, cnt;
 };
 
+// The root buffer: the entry record, then a word that is nonzero when a node box holds NaN (a NaN
+// vertex's, or a loaded file's).
+constexpr size_t ROOT_RECORD_BYTES = sizeof(TraceRoot) + 16;
+
 struct TraceCtx
 {
     const rt_gnode*    gn;
@@ -99,6 +103,7 @@ struct TraceCtx
     const rt_triangle* tris;
     const rt_vertex*   verts;
     const TraceRoot*   root;  // device record written by the layout kernel
+    const uint32_t*    odd;   // nonzero: a box holds NaN
     uint32_t           ww;    // 1: while-while loop (leaves of 6 or more triangles on average)
     const rt_wnode*    wn;    // the 8-wide layout (trace_ray_wide; built on request)
     const uint32_t*    wid;   // wide node index of each binary node that is a wide node
@@ -163,8 +168,8 @@ __device__ __forceinline__ THit trace_ray_oneloop(const TraceCtx& T, const Trace
             const rt_gnode* g = T.gn + ref;
             const float4 a = __ldg(&g->a), b = __ldg(&g->b), c = __ldg(&g->c);
             const uint4 dd = __ldg(&g->d);
-            const float tl = ray_box(o, inv, tmin, best, a.x, a.y, a.z, a.w, b.x, b.y);
-            const float tr = ray_box(o, inv, tmin, best, b.z, b.w, c.x, c.y, c.z, c.w);
+            const float tl = ray_box(o, inv, tmin, best, a.x, a.z, b.x, a.y, a.w, b.y);
+            const float tr = ray_box(o, inv, tmin, best, b.z, c.x, c.z, b.w, c.y, c.w);
             // push the farther child first so the nearer one pops first; left first on ties
             uint32_t fr, fc, nr, nc;
             float ft, nt;
@@ -230,8 +235,8 @@ __device__ __forceinline__ THit trace_ray_ww(const TraceCtx& T, const TraceRoot&
             const rt_gnode* g = T.gn + cref;
             const float4 a = __ldg(&g->a), b = __ldg(&g->b), c = __ldg(&g->c);
             const uint4 dd = __ldg(&g->d);
-            const float tl = ray_box(o, inv, tmin, best, a.x, a.y, a.z, a.w, b.x, b.y);
-            const float tr = ray_box(o, inv, tmin, best, b.z, b.w, c.x, c.y, c.z, c.w);
+            const float tl = ray_box(o, inv, tmin, best, a.x, a.z, b.x, a.y, a.w, b.y);
+            const float tr = ray_box(o, inv, tmin, best, b.z, c.x, c.z, b.w, c.y, c.w);
             // the farther child waits on the stack, the nearer one is next; left first on ties
             uint32_t fr, fc, nr, nc;
             float ft, nt;

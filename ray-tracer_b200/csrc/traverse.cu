@@ -16,10 +16,11 @@
 // strict "t < bestT" update (:112-142), so the first triangle at the minimal distance wins as
 // in the reference and hits carry identical triangle indices (trace_core.cuh).
 //
-// The kernel is persistent: each warp claims 32 rays at a time from a global counter until
-// the batch is exhausted, so long incoherent rays do not leave SMs idle at the tail.
-#include "trace_core.cuh"
+// The kernel is persistent: warps claim rays from a global counter as their lanes finish, and
+// test leaves together (trace_warp.cuh).
+#include "trace_warp.cuh"
 
+#include <algorithm>
 #include <mutex>
 #include <vector>
 
@@ -38,7 +39,7 @@ constexpr int TBLK = 128;
 // thread 0 also writes the traversal entry record of node 0.
 __global__ void k_make_gnodes(const rt_bvh_node* __restrict__ nodes, uint32_t n_nodes, uint32_t n_tris,
                               const uint32_t* __restrict__ d_counts, rt_gnode* __restrict__ gn, TraceRoot* __restrict__ root,
-                              uint32_t* __restrict__ status)
+                              uint32_t* __restrict__ odd, uint32_t* __restrict__ status)
 {
     const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
     if (d_counts) { n_nodes = d_counts[0]; n_tris = d_counts[1]; }
@@ -66,12 +67,16 @@ __global__ void k_make_gnodes(const rt_bvh_node* __restrict__ nodes, uint32_t n_
     }
     const rt_bvh_node l = nodes[nd.a], r = nodes[nd.b];
     rt_gnode g;
-    g.a = make_float4(l.bmin[0], l.bmin[1], l.bmin[2], l.bmax[0]);
-    g.b = make_float4(l.bmax[1], l.bmax[2], r.bmin[0], r.bmin[1]);
-    g.c = make_float4(r.bmin[2], r.bmax[0], r.bmax[1], r.bmax[2]);
+    g.a = make_float4(l.bmin[0], l.bmax[0], l.bmin[1], l.bmax[1]);
+    g.b = make_float4(l.bmin[2], l.bmax[2], r.bmin[0], r.bmax[0]);
+    g.c = make_float4(r.bmin[1], r.bmax[1], r.bmin[2], r.bmax[2]);
     g.d = make_uint4(l.is_leaf ? l.a : nd.a, r.is_leaf ? r.a : nd.b, l.is_leaf ? (LEAF_BIT | l.b) : 0u,
                      r.is_leaf ? (LEAF_BIT | r.b) : 0u);
     gn[i] = g;
+    // a NaN plane makes the traversal take the general box test
+    bool nan = false;
+    for (int k = 0; k < 3; k++) { nan |= l.bmin[k] != l.bmin[k] || l.bmax[k] != l.bmax[k] || r.bmin[k] != r.bmin[k] || r.bmax[k] != r.bmax[k]; }
+    if (nan) { *odd = 1u; }
 }
 
 __global__ void k_make_tripos(const rt_triangle* __restrict__ tris, uint32_t n, const uint32_t* __restrict__ d_counts,
@@ -129,14 +134,88 @@ __global__ void k_depth(const rt_bvh_node* __restrict__ nodes, uint32_t n, const
     atomicMax(depth, d);
 }
 
+// The hit record of a finished ray.
+__device__ __forceinline__ void write_hit(const TraceCtx& T, float4* __restrict__ hits, uint64_t ri, bool hit, bool overflow,
+                                          float t, float u, float v, uint32_t tri, uint32_t* __restrict__ status)
+{
+    float4 h0 = make_float4(0.f, 0.f, 0.f, 0.f), h1 = make_float4(0.f, 0.f, 0.f, 0.f);
+    uint32_t flags = 0;
+    if (hit)
+    {
+        const f3 nrm = hit_normal(T, tri, u, v);
+        h0 = make_float4(t, u, v, __uint_as_float(tri));
+        h1 = make_float4(nrm.x, nrm.y, nrm.z, 0.f);
+        flags = RT_HIT_FLAG_HIT;
+    }
+    if (overflow) { flags |= RT_HIT_FLAG_OVERFLOW; atomicOr(status, ST_STACK); }
+    h1.w = __uint_as_float(flags);
+    hits[2 * ri] = h0;
+    hits[2 * ri + 1] = h1;
+}
+
 // rt_ray records in, rt_hit records out (two 128-bit accesses each). n_dev, when set, holds
 // the ray count on the device (the wavefront path tracer's queue length). ROOTS: ray i
-// traces the subtree roots[rscene[i]] (a scene of a batched build).
-template <int MODE, int STK, bool ROOTS, bool WIDE = false>
-__global__ void __launch_bounds__(256)
+// traces the subtree roots[rscene[i]] (a scene of a batched build). A warp holds at most
+// `per_warp` rays at a time.
+template <int MODE, int STK, bool ROOTS>
+__global__ void __launch_bounds__(256, 4)
 k_trace(TraceCtx T, const float4* __restrict__ rays, float4* __restrict__ hits, uint64_t n, const uint32_t* __restrict__ n_dev,
         unsigned long long* __restrict__ counter, uint32_t* __restrict__ status, const TraceRoot* __restrict__ roots,
-        const uint32_t* __restrict__ rscene)
+        const uint32_t* __restrict__ rscene, int per_warp)
+{
+    extern __shared__ __align__(16) unsigned char smem[];
+    constexpr unsigned FULL = 0xffffffffu;
+    WarpShare& S = reinterpret_cast<WarpShare*>(smem)[threadIdx.x >> 5];
+    const int lane = (int)(threadIdx.x & 31u);
+    const unsigned lanes = per_warp >= 32 ? FULL : (1u << per_warp) - 1u;
+    const int refill = per_warp >= 32 ? REFILL : (per_warp + 1) / 2;
+    if (n_dev) { n = *n_dev; }
+    const bool odd_tree = *T.odd != 0u;
+    LaneTrace<MODE, STK> L;
+    uint2 stk[STK];
+    L.live = false;
+    bool pending = false, more = true;  // this lane has a result to write; rays are left
+    for (;;)
+    {
+        const unsigned idle = __ballot_sync(FULL, !L.live) & lanes;
+        if (idle == lanes || (more && __popc(idle) >= refill))
+        {
+            if (!L.live && pending)
+            {
+                pending = false;
+                const float4 h = S.hit[lane];
+                write_hit(T, hits, S.id[lane], L.hit, L.overflow, L.best, h.x, h.y, __float_as_uint(h.z), status);
+            }
+            if (!more) { break; }
+            unsigned long long base = 0;
+            if (lane == 0) { base = atomicAdd(counter, (unsigned long long)__popc(idle)); }
+            base = __shfl_sync(FULL, base, 0);
+            if (base + __popc(idle) >= n) { more = false; }
+            if ((idle >> lane) & 1u)
+            {
+                const uint64_t ri = base + __popc(idle & ((1u << lane) - 1u));
+                if (ri < n)
+                {
+                    const float4 r0 = rays[2 * ri], r1 = rays[2 * ri + 1];
+                    if (ROOTS) { L.start(S, roots[rscene[ri]], r0, r1, odd_tree); } else { L.start(S, *T.root, r0, r1, odd_tree); }
+                    S.id[lane] = ri;
+                    pending = true;
+                }
+            }
+            __syncwarp();
+            continue;
+        }
+        warp_walk<MODE, STK>(L, stk, T, S, lanes, more, refill);
+        warp_leaves<MODE, STK>(L, stk, T, S);
+    }
+}
+
+// The 8-wide layout's kernel: each warp claims 32 rays at a time until the batch is exhausted.
+template <int MODE, bool ROOTS>
+__global__ void __launch_bounds__(256)
+k_trace_wide(TraceCtx T, const float4* __restrict__ rays, float4* __restrict__ hits, uint64_t n,
+             const uint32_t* __restrict__ n_dev, unsigned long long* __restrict__ counter, uint32_t* __restrict__ status,
+             const TraceRoot* __restrict__ roots, const uint32_t* __restrict__ rscene, int)
 {
     const int lane = threadIdx.x & 31;
     if (n_dev) { n = *n_dev; }
@@ -152,40 +231,25 @@ k_trace(TraceCtx T, const float4* __restrict__ rays, float4* __restrict__ hits, 
         if (ri >= n) { continue; }
         const float4 r0 = rays[2 * ri], r1 = rays[2 * ri + 1];
         const TraceRoot& R = ROOTS ? roots[rscene[ri]] : R0;
-        const f3 o = mk3(r0.x, r0.y, r0.z), d = mk3(r1.x, r1.y, r1.z);
-        THit H;
-        if constexpr (WIDE) { H = trace_ray_wide<MODE, STK>(T, R, o, d, r0.w, r1.w); }  // one entry per wide level
-        else { H = trace_ray<MODE, STK>(T, R, o, d, r0.w, r1.w); }
-        float4 h0 = make_float4(0.f, 0.f, 0.f, 0.f), h1 = make_float4(0.f, 0.f, 0.f, 0.f);
-        uint32_t flags = 0;
-        if (H.hit)
-        {
-            const f3 nrm = hit_normal(T, H.tri, H.u, H.v);
-            h0 = make_float4(H.t, H.u, H.v, __uint_as_float(H.tri));
-            h1 = make_float4(nrm.x, nrm.y, nrm.z, 0.f);
-            flags = RT_HIT_FLAG_HIT;
-        }
-        if (H.overflow) { flags |= RT_HIT_FLAG_OVERFLOW; atomicOr(status, ST_STACK); }
-        h1.w = __uint_as_float(flags);
-        hits[2 * ri] = h0;
-        hits[2 * ri + 1] = h1;
+        const THit H = trace_ray_wide<MODE, STACK>(T, R, mk3(r0.x, r0.y, r0.z), mk3(r1.x, r1.y, r1.z), r0.w, r1.w);
+        write_hit(T, hits, ri, H.hit, H.overflow, H.t, H.u, H.v, H.tri, status);
     }
 }
 
 using TraceFn = void (*)(TraceCtx, const float4*, float4*, uint64_t, const uint32_t*, unsigned long long*, uint32_t*,
-                         const TraceRoot*, const uint32_t*);
+                         const TraceRoot*, const uint32_t*, int);
 
 TraceFn trace_fn(uint32_t flags, int stack, bool roots, bool wide)
 {
     if (wide)
     {
-        if (roots) { return (flags & 3u) == 0 ? k_trace<0, STACK, true, true> : nullptr; }
+        if (roots) { return (flags & 3u) == 0 ? k_trace_wide<0, true> : nullptr; }
         switch (flags & 3u)
         {
-        case 0: return k_trace<0, STACK, false, true>;
-        case 1: return k_trace<1, STACK, false, true>;
-        case 2: return k_trace<2, STACK, false, true>;
-        default: return k_trace<3, STACK, false, true>;
+        case 0: return k_trace_wide<0, false>;
+        case 1: return k_trace_wide<1, false>;
+        case 2: return k_trace_wide<2, false>;
+        default: return k_trace_wide<3, false>;
         }
     }
     if (stack <= 32)
@@ -208,7 +272,7 @@ std::mutex g_occ_mu;
 struct OccKey { TraceFn fn; int block; int v; };
 std::vector<OccKey> g_occ;
 
-int blocks_per_sm(TraceFn fn, int block)
+int blocks_per_sm(TraceFn fn, int block, size_t smem)
 {
     std::lock_guard<std::mutex> lk(g_occ_mu);
     for (const OccKey& k : g_occ)
@@ -216,7 +280,7 @@ int blocks_per_sm(TraceFn fn, int block)
         if (k.fn == fn && k.block == block) { return k.v; }
     }
     int v = 0;
-    if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&v, fn, block, 0) != cudaSuccess) { cudaGetLastError(); v = 1; }
+    if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&v, fn, block, smem) != cudaSuccess) { cudaGetLastError(); v = 1; }
     if (v < 1) { v = 1; }
     g_occ.push_back(OccKey{ fn, block, v });
     return v;
@@ -232,6 +296,7 @@ TraceCtx make_trace_ctx(const rt_bvh* B)
     T.tris = B->tris.as<rt_triangle>();
     T.verts = B->verts.as<rt_vertex>();
     T.root = B->rootbuf.as<TraceRoot>();
+    T.odd = reinterpret_cast<const uint32_t*>(T.root + 1);
     T.ww = B->trace_ww ? 1u : 0u;
     T.wn = B->wnodes.as<rt_wnode>();
     T.wid = B->wid.as<uint32_t>();
@@ -242,14 +307,15 @@ int launch_traversal_layout(rt_bvh* B, cudaStream_t st, uint32_t max_nodes, uint
                             uint32_t* vstatus, bool tripos_ready, bool gnodes_ready)
 {
     if (B->gnodes.ensure((size_t)max_nodes * sizeof(rt_gnode)) || B->tripos.ensure((size_t)(max_tris ? max_tris : 1) * 48) ||
-        B->rootbuf.ensure(sizeof(TraceRoot)))
+        B->rootbuf.ensure(ROOT_RECORD_BYTES))
     {
         return RT_E_CUDA;
     }
     if (!gnodes_ready)
     {
+        uint32_t* odd = reinterpret_cast<uint32_t*>(B->rootbuf.as<TraceRoot>() + 1);  // zeroed by the caller
         k_make_gnodes<<<(max_nodes + 255) / 256, 256, 0, st>>>(B->nodes.as<rt_bvh_node>(), max_nodes, max_tris, d_counts,
-                                                               B->gnodes.as<rt_gnode>(), B->rootbuf.as<TraceRoot>(), vstatus);
+                                                               B->gnodes.as<rt_gnode>(), B->rootbuf.as<TraceRoot>(), odd, vstatus);
         count_launch();
     }
     if (max_tris && !tripos_ready)
@@ -264,7 +330,8 @@ int launch_traversal_layout(rt_bvh* B, cudaStream_t st, uint32_t max_nodes, uint
 int make_traversal_layout(rt_bvh* B, cudaStream_t st)
 {
     if (B->n_nodes == 0) { return fail(RT_E_EMPTY, "empty BVH"); }
-    if (B->trace_status.ensure(64)) { return RT_E_CUDA; }
+    if (B->trace_status.ensure(64) || B->rootbuf.ensure(ROOT_RECORD_BYTES)) { return RT_E_CUDA; }
+    RT_CUDA(cudaMemsetAsync(B->rootbuf.as<TraceRoot>() + 1, 0, 4, st));
     uint32_t* vstatus = B->trace_status.as<uint32_t>() + 12;
     RT_CUDA(cudaMemsetAsync(vstatus, 0, 4, st));
     if (int e = launch_traversal_layout(B, st, B->n_nodes, B->n_tris, nullptr, vstatus)) { return e; }
@@ -282,16 +349,23 @@ int trace_launch(const rt_bvh* B, const void* d_rays, void* d_hits, uint64_t n, 
     if (!fn) { return fail(RT_E_INVALID, "no trace kernel for this mode and stack depth"); }
     const int block = opt.block > 0 ? opt.block : TBLK;
     if (block % 32 || block > 256) { return fail(RT_E_INVALID, "trace block must be a multiple of 32, at most 256"); }
-    uint64_t grid = (uint64_t)device_sm_count() * (uint64_t)blocks_per_sm(fn, block);
+    const size_t smem = B->trace_wide ? 0 : (size_t)(block / 32) * sizeof(WarpShare);
+    uint64_t grid = (uint64_t)device_sm_count() * (uint64_t)blocks_per_sm(fn, block, smem);
+    int per_warp = 32;
     if (!n_dev)
     {
-        const uint64_t want = (n + block - 1) / block;
+        // Few rays are spread over the resident warps, down to one ray per warp: the lanes without
+        // a ray still test its leaves' triangles (1,000 rays, 5,120-triangle hybrid tree: see
+        // trace_warp.cuh).
+        const uint64_t warps = grid * (uint64_t)(block / 32);
+        if (!B->trace_wide && n < warps * 32) { per_warp = (int)std::max<uint64_t>(1, (n + warps - 1) / warps); }
+        const uint64_t want = (n + (uint64_t)per_warp * (block / 32) - 1) / ((uint64_t)per_warp * (block / 32));
         if (grid > want) { grid = want; }
     }
     if (grid == 0) { return RT_OK; }
     const TraceCtx T = make_trace_ctx(B);
-    fn<<<(uint32_t)grid, block, 0, st>>>(T, static_cast<const float4*>(d_rays), static_cast<float4*>(d_hits), n, n_dev,
-                                         d_counter, d_status, opt.roots, opt.rscene);
+    fn<<<(uint32_t)grid, block, smem, st>>>(T, static_cast<const float4*>(d_rays), static_cast<float4*>(d_hits), n, n_dev,
+                                            d_counter, d_status, opt.roots, opt.rscene, per_warp);
     count_launch();
     return check_launch("trace");
 }

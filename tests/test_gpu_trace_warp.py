@@ -1,0 +1,69 @@
+"""The warp-cooperative trace kernel at the sizes and inputs where it can go wrong: ray counts around
+a warp and below one ray per resident warp, leaves of one to hundreds of triangles, rays and
+vertices that are not finite. Bar: bit-equal to the oracle's restatement of bvh::trace."""
+import numpy as np
+import pytest
+
+import rtb200
+from oracle import Baked
+from rtb200 import scenes
+from test_gpu_trace import compare, rays_for
+
+pytestmark = pytest.mark.gpu
+
+
+def build(kind, preset, **kw):
+    if kind == "soup":
+        v, t = scenes.soup(3001, seed=5, lo=1e-2, hi=2e-1)
+    else:  # runs of equal triangles: leaves far above 32 pairs
+        v, t = scenes.soup(40, seed=6, lo=1e-1, hi=3e-1)
+        t = np.repeat(t, 37, axis=0)
+    return v, t, rtb200.Bvh.build(v, t, rtb200.make_cfg(preset, **kw))
+
+
+@pytest.mark.parametrize("kind,preset,kw", [("soup", "lbvh63", {}), ("soup", "sah4", {}), ("soup", "lbvh63", dict(max_leaf=200)),
+                                            ("soup", "lbvh63", dict(max_leaf=1)), ("runs", "lbvh63", dict(max_leaf=500)),
+                                            ("runs", "hybrid", {})])
+@pytest.mark.parametrize("flags", [0, 1, 2, 3])
+def test_leaf_sizes(orc, kind, preset, kw, flags):
+    v, t, b = build(kind, preset, **kw)
+    nodes, tris, verts = b.download()
+    rays = rays_for(v, 6001, seed=11)
+    compare(b.trace(rays, flags), orc.trace(Baked(nodes, tris, verts), rays, flags=flags, threads=8), f"{kind}/{preset}/{kw}/{flags}")
+
+
+@pytest.mark.parametrize("n", [1, 2, 31, 32, 33, 1000, 4735, 4737, 151551, 151553])
+def test_ray_counts(orc, n):
+    v, t, b = build("soup", "hybrid")
+    nodes, tris, verts = b.download()
+    rays = rays_for(v, max(n, 8), seed=n)[:n]
+    compare(b.trace(rays), orc.trace(Baked(nodes, tris, verts), rays, threads=8), f"n={n}")
+
+
+@pytest.mark.parametrize("flags", [0, 1])
+def test_rays_that_are_not_finite(orc, flags):
+    v, t, b = build("soup", "lbvh63")
+    nodes, tris, verts = b.download()
+    rays = rays_for(v, 8192, seed=3)
+    rng = np.random.default_rng(4)
+    bad = np.array([np.nan, np.inf, -np.inf, 0.0, -0.0, 1e-45, -1e-45, 3e38, -3e38], np.float32)
+    at = rng.integers(0, 8, 4096)
+    rays[np.arange(4096), at] = bad[rng.integers(0, len(bad), 4096)]
+    hits = b.trace(rays, flags)
+    h, out, tri, counters, overflow = orc.trace(Baked(nodes, tris, verts), rays, flags=flags, threads=8)
+    # x86 and CUDA give a NaN different sign bits: a NaN weight equals any NaN
+    got = np.stack([hits["t"], hits["u"], hits["v"], hits["n"][:, 0], hits["n"][:, 1], hits["n"][:, 2]], axis=1)
+    both = np.isnan(got) & np.isnan(out)
+    out = np.where(both, got, out)
+    compare(hits, (h, out, tri, counters, overflow), f"flags {flags}")
+
+
+@pytest.mark.parametrize("preset", ["lbvh63", "hybrid"])
+def test_vertices_that_are_not_finite(orc, preset):
+    v, t = scenes.soup(600, seed=8, lo=1e-2, hi=2e-1)
+    rng = np.random.default_rng(9)
+    v[rng.integers(0, v.shape[0], 6), rng.integers(0, 3, 6)] = np.nan
+    b = rtb200.Bvh.build(v, t, preset)
+    nodes, tris, verts = b.download()
+    rays = rays_for(np.nan_to_num(v), 8192, seed=10)
+    compare(b.trace(rays), orc.trace(Baked(nodes, tris, verts), rays, threads=8), preset)
