@@ -133,18 +133,16 @@ void rt_bvh_free(rt_bvh* bvh);
 #define RT_TRACE_ANY_HIT     1u  /* stop at the first accepted triangle */
 #define RT_TRACE_WATERTIGHT  2u  /* watertight test (Woop, Benthin, Wald 2013), no culling */
 
-/* Traversal loop form of a handle (no counterpart in the reference): 0 the one-loop form of
- * traverse() (bvh_traverse.cpp:91-178), 1 the while-while form (lanes of a warp walk inner
- * nodes, then test leaves, together), -1 the default: while-while when leaves hold 6 or more
- * triangles on average. Both visit the same nodes in the same order and give identical hits;
- * only their speed differs. 2: the 8-wide layout (128-byte nodes of up to eight children with
- * 8-bit quantised, conservative child boxes), built now and again after every rebuild of the
- * handle; rt_trace and the wavefront path tracer's trace stage use it (the plain per-pixel
- * renderer keeps the binary loop). It is not the reference's visiting
- * order: the closest hit's distance is the same, but on an exact tie in distance the reported
- * triangle may differ, and a triangle that the binary boxes cull -- one an exact box test
- * loses by rounding at a face, or, in trees with spatial splits, one outside a collapsed
- * intermediate node's box -- may be found. */
+/* Traversal form of a handle (no counterpart in the reference): -1, 0 and 1 the reference's
+ * visiting order over the binary tree (traverse(), bvh_traverse.cpp:91-178) with identical hits;
+ * they choose the loop of rt_adjoint's traversal (0 one loop, 1 while-while, -1 while-while when
+ * leaves hold 6 or more triangles on average), traces and renders have one form for all. 2: the 8-wide layout (128-byte
+ * nodes of up to eight children with 8-bit quantised, conservative child boxes), built now and
+ * again after every rebuild of the handle; rt_trace uses it (renders keep the binary tree). It is
+ * not the reference's visiting order: the closest hit's distance is the same, but on an exact tie
+ * in distance the reported triangle may differ, and a triangle that the binary boxes cull -- one
+ * an exact box test loses by rounding at a face, or, in trees with spatial splits, one outside a
+ * collapsed intermediate node's box -- may be found. */
 int rt_bvh_trace_loop(rt_bvh* bvh, int form);
 /* The wide layout of a handle in form 2 (no counterpart in the reference): *n_wide nodes of
  * 128 bytes each -- {float p[3]; uint32 meta (x / y / z scale exponents in bits 0-23, inner-
@@ -185,6 +183,10 @@ typedef struct rt_render_cfg
 void rt_camera_lookat(const float pos[3], const float target[3], float fov_deg, rt_render_cfg* cfg);
 void rt_camera_quat(const float pos[3], const float q_wxyz[4], float focal, rt_render_cfg* cfg);
 
+/* Both modes trace all paths with one persistent kernel and add a pixel's samples in sample order,
+ * so they give the same image; RT_RENDER_WAVEFRONT takes the handle's tuned launch parameters
+ * (rt_autotune_wavefront), RT_RENDER_PLAIN the defaults. Calls on one handle may come from several
+ * streams and host threads: they share the handle's scratch one after another. */
 enum rt_render_mode { RT_RENDER_PLAIN = 0, RT_RENDER_WAVEFRONT = 1 };
 
 /* Renders the image (rgb: W*H*3 float, row y = 0 at the bottom as in the reference's buffer
@@ -249,18 +251,17 @@ int rt_bvh_scenes(const rt_bvh* bvh, uint32_t* n_scenes, uint32_t* info4);
  * entries never overflows). */
 int rt_bvh_depth(rt_bvh* bvh, uint32_t* depth);
 
-/* Launch parameters of the wavefront path tracer. */
+/* Launch parameters of the path tracer. */
 typedef struct rt_wavefront_params
 {
-    uint32_t trace_block;  /* threads per block of the persistent trace kernel (32..256) */
-    uint32_t chunk_paths;  /* paths in flight per generate/extend/shade round */
+    uint32_t trace_block;  /* threads per block of the path kernel (32..256) */
+    uint32_t chunk_paths;  /* paths per launch; whole samples of all pixels are grouped up to it */
     uint32_t stack_depth;  /* traversal stack entries: 64, or 32 when the tree is at most 31 deep */
-    uint32_t shade_block;  /* threads per block of the shade kernel */
+    uint32_t shade_block;  /* threads per block of the kernel that adds up the samples */
 } rt_wavefront_params;
 
-/* Renders every scene of a batched handle in one wavefront kernel set, replayed from a CUDA
- * graph captured on first use of a configuration. cfgs[s]: camera and seed of scene s;
- * size, spp, bounces, roulette, background and sample offset come from cfgs[0]. shading:
+/* Renders every scene of a batched handle in the same launches. cfgs[s]: camera and seed of scene
+ * s; size, spp, bounces, roulette, background and sample offset come from cfgs[0]. shading:
  * materials over all scenes, mat_of_tri / tri_albedo per baked triangle of the handle.
  * rgb (rgb2 optional): n_scenes * H * W * 3 floats, scene-major (device). Scene s gets the
  * samples that rt_render_ex of scene s alone with cfgs[s] takes (same random numbers).

@@ -126,17 +126,10 @@ static void free_bvh(rt_bvh* b)
                        &b->s.sah_scan_in, &b->s.sah_scan_out, &b->s.sah_node_ids, &b->s.sah_roots_lvl, &b->s.sah_root_ord, &b->s.root_sort.keys_alt,
                        &b->s.root_sort.vals_alt, &b->s.root_sort.lookback, &b->s.root_sort.tile_counters,
                        &b->s.in_verts, &b->s.in_tris, &b->s.gtris, &b->s.batch_off, &b->s.sah_budget, &b->s.sah_wide, &b->s.sah_tmp2, &b->s.sah_pos2, &b->s.wide_flag, &b->s.wide_par, &b->wnodes, &b->wid, &b->scene_info, &b->scene_roots,
-                       &b->wf_cams };
+                       &b->wf_buf };
     for (DevBuf* x : bufs) { x->release(); }
     b->rootbuf.release();
-    for (int k = 0; k < 2; k++) { b->wf_rays[k].release(); b->wf_state[k].release(); b->wf_scene[k].release(); }
-    b->wf_hits.release(); b->wf_acc.release(); b->wf_ctr.release();
-    if (b->wf_exec) { cudaGraphExecDestroy(b->wf_exec); b->wf_exec = nullptr; }
-    for (cudaEvent_t& e : b->wf_ev)
-    {
-        if (e) { cudaEventDestroy(e); e = nullptr; }
-    }
-    if (b->wf_stream) { cudaStreamDestroy(b->wf_stream); b->wf_stream = nullptr; }
+    if (b->wf_ev) { cudaEventDestroy(b->wf_ev); b->wf_ev = nullptr; }
     if (b->bake_exec) { cudaGraphExecDestroy(b->bake_exec); b->bake_exec = nullptr; }
     for (cudaEvent_t& e : b->bake_ev)
     {

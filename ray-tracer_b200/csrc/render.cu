@@ -3,18 +3,19 @@
 // std::mt19937 stream, and the material extensions the benchmark scenes need (per-triangle
 // albedo, emitters, mirrors; the reference has albedo 0.8 and no emitters).
 //
-// Two schedules compute the same samples from the same random numbers:
-//  RT_RENDER_PLAIN      one thread per pixel runs all its samples (the reference's loop order,
-//                       so the per-pixel sums add up in sample order);
-//  RT_RENDER_WAVEFRONT  generate / extend / shade queues: all paths of a chunk of samples advance
-//                       one bounce per step; extend is the persistent trace kernel over the
-//                       compacted ray queue, shade writes the next queue and retires finished
-//                       paths into the image with atomics.
-// The wavefront also renders the scenes of a batched build together (rt_render_batch): a path
-// carries its scene, extend traces it from that scene's root, and each scene has its own
-// camera and seed, so scene s of a batch gets the samples a render of scene s alone gets. Its
-// launch sequence is replayed from a CUDA graph captured once per configuration, and its
-// block size, queue chunk and stack depth can be chosen by rt_autotune_wavefront.
+// One persistent kernel (k_paths) traces every (pixel, sample) path: a warp's lanes hold 32 paths
+// at different bounces, walk the tree and test leaves together (trace_warp.cuh), and lanes whose
+// ray is done are shaded together -- emission, next direction, roulette -- and go on with their next
+// ray or a new path. Each path's radiance goes to a buffer, and k_sum adds a pixel's samples in
+// sample order (the reference's loop order), so images do not depend on the schedule.
+// RT_RENDER_PLAIN and RT_RENDER_WAVEFRONT differ in nothing but the paths per launch
+// (rt_wavefront_params). Scenes of a batched build (rt_render_batch) are rendered by the same
+// launch: a path starts at its scene's root with that scene's camera and seed.
+//
+// Why not queues of rays between a trace and a shade kernel per bounce, as before: every such
+// step lasts at least as long as its longest ray (0.3-0.6 ms), which was more than half of the
+// time of a 1080p image at 8 bounces; and why not a thread per pixel: a 256 x 256 image fills
+// 0.4 of the chip that way.
 //
 // Random numbers: Philox4x32-10 (Salmon et al., SC'11) keyed by (seed, 0x5EED), counter
 // (pixel, sample, 0, 0) for the pixel jitter and (pixel, sample, bounce + 1, 0) for the
@@ -27,10 +28,11 @@
 // counter-based random numbers, and at vertex k the radiance still to come,
 // L - sum_{i<=k} T_i E_i, divided by the albedo there is dL/dalbedo_k. The RNG is recomputed,
 // not stored, so memory stays O(pixels). Russian-roulette probabilities are held constant.
-#include "trace_core.cuh"
+#include "trace_warp.cuh"
 
 #include <algorithm>
 #include <cstring>
+#include <mutex>
 #include <vector>
 
 namespace rtb
@@ -182,6 +184,151 @@ __device__ __forceinline__ bool scatter(const RP& P, uint32_t seed, const Surf& 
     return true;
 }
 
+// Shades a traced ray of a path: adds the emission (or background) it reached to `sum` and, where the
+// path goes on, makes its next ray r0 = {o, tmin}, r1 = {d, tmax}. sf: the surface hit.
+__device__ __forceinline__ bool shade(const TraceCtx& T, const RP& P, const Shade& sh, uint32_t seed, uint32_t pix, uint32_t sidx,
+                                      uint32_t bounce, bool hit, float t, float4 uvt, f3 o, f3 d, f3& tp, f3& sum, Surf& sf,
+                                      float4& r0, float4& r1)
+{
+    if (!hit)
+    {
+        sum = add3(sum, mul3(tp, environment(P, d)));
+        return false;
+    }
+    const uint32_t tri = __float_as_uint(uvt.z);
+    sf = surface(sh, tri);
+    sum = add3(sum, mul3(tp, sf.emission));
+    const f3 n = hit_normal(T, tri, uvt.x, uvt.y);
+    f3 nd;
+    if (!scatter(P, seed, sf, n, d, pix, sidx, bounce, tp, nd) || bounce >= P.max_bounce) { return false; }
+    const f3 no = add3(o, muls(d, t));
+    r0 = make_float4(no.x, no.y, no.z, 1e-4f);
+    r1 = make_float4(nd.x, nd.y, nd.z, bits2f(0x7f800000u));
+    return true;
+}
+
+// What one launch of k_paths works on. Items are numbered sample by sample, scene by scene, and in
+// 8 x 4 pixel tiles (neighbouring lanes start with neighbouring pixels); items of a tile that lie
+// outside the image are skipped.
+struct PathJob
+{
+    RP               P;
+    Shade            sh;
+    const Cam*       cams;     // per scene (nullptr: P.cam)
+    const TraceRoot* roots;    // per scene (nullptr: the handle's root)
+    uint32_t         S;        // scenes
+    uint32_t         tiles_x, scene_items;
+    uint32_t         sample0;  // sample of item 0, from P.sample_offset
+    uint32_t         first, n; // this launch's items
+    float*           rad;      // radiance per path: [sample - sample0][scene][pixel][3]
+};
+
+// Shared memory of one warp's paths.
+struct PathShare
+{
+    WarpShare w;
+    float4    tp[32];  // throughput, image pixel (scene * W * H + pixel)
+    float4    sum[32]; // radiance so far, sample
+};
+// The radiance of every path.
+template <int STK>
+__global__ void __launch_bounds__(256, 4)
+k_paths(const TraceCtx T, const __grid_constant__ PathJob J, uint32_t* __restrict__ counter, int per_warp)
+{
+    extern __shared__ __align__(16) unsigned char smem[];
+    constexpr unsigned FULL = 0xffffffffu;
+    PathShare& S = reinterpret_cast<PathShare*>(smem)[threadIdx.x >> 5];
+    const int lane = (int)(threadIdx.x & 31u);
+    const unsigned lanes = per_warp >= 32 ? FULL : (1u << per_warp) - 1u;
+    const int refill = per_warp >= 32 ? REFILL : (per_warp + 1) / 2;
+    const bool odd_tree = *T.odd != 0u;
+    const uint32_t npix = J.P.W * J.P.H;
+    LaneTrace<0, STK> L;
+    uint2 stk[STK];
+    L.live = false;
+    bool pending = false, more = true;  // this lane has a ray (to shade when it is done); items are left
+    for (;;)
+    {
+        // lanes whose ray is done are shaded, and those whose path is done get a new one, once enough
+        // of them wait; when no paths are left, once half of the lanes still at work do
+        const unsigned idle = __ballot_sync(FULL, !L.live) & lanes;
+        const unsigned takers = more ? lanes : __ballot_sync(FULL, pending);
+        const int serve = more ? refill : (__popc(takers) + 1) / 2;
+        if (__popc(idle & takers) >= serve)
+        {
+            const bool mine = (idle >> lane) & 1u;
+            bool go = false;  // r0, r1: the lane's next ray
+            float4 r0 = make_float4(0.f, 0.f, 0.f, 0.f), r1 = r0;
+            uint32_t bounce = 0;
+            // shade what the finished rays hit
+            if (mine && pending)
+            {
+                pending = false;
+                const float4 a = S.w.a[lane], b = S.w.b[lane], h = S.w.hit[lane], ts = S.tp[lane], ss = S.sum[lane];
+                f3 tp = mk3(ts.x, ts.y, ts.z), sum = mk3(ss.x, ss.y, ss.z);
+                const uint32_t gpix = __float_as_uint(ts.w), sidx = __float_as_uint(ss.w);
+                const uint32_t sc = gpix / npix;
+                const size_t at = 3 * ((size_t)(sidx - J.P.sample_offset - J.sample0) * J.S * npix + gpix);
+                bounce = (uint32_t)S.w.id[lane];
+                Surf sf;
+                go = shade(T, J.P, J.sh, J.cams ? J.cams[sc].seed : J.P.cam.seed, gpix - sc * npix, sidx, bounce, L.hit, L.best, h,
+                           mk3(a.x, a.y, a.z), mk3(b.x, b.y, b.z), tp, sum, sf, r0, r1);
+                if (go)
+                {
+                    S.tp[lane] = make_float4(tp.x, tp.y, tp.z, ts.w);
+                    S.sum[lane] = make_float4(sum.x, sum.y, sum.z, ss.w);
+                    bounce++;
+                }
+                else { J.rad[at] = sum.x; J.rad[at + 1] = sum.y; J.rad[at + 2] = sum.z; }
+            }
+            // new paths for the others
+            const bool want = mine && !go;
+            const unsigned wants = __ballot_sync(FULL, want);
+            if (more && wants)
+            {
+                uint32_t base = 0;
+                if (lane == 0) { base = atomicAdd(counter, (uint32_t)__popc(wants)); }
+                base = __shfl_sync(FULL, base, 0);
+                if (base + (uint32_t)__popc(wants) >= J.n) { more = false; }
+                const uint32_t g = base + (uint32_t)__popc(wants & ((1u << lane) - 1u));
+                if (want && g < J.n)
+                {
+                    const uint32_t G = J.first + g, per_sample = J.scene_items * J.S;
+                    const uint32_t s = G / per_sample, rem = G - s * per_sample, sc = rem / J.scene_items;
+                    const uint32_t q = rem - sc * J.scene_items, tile = q >> 5, ty = tile / J.tiles_x;
+                    const uint32_t x = (tile - ty * J.tiles_x) * 8u + (q & 7u), y = ty * 4u + ((q >> 3) & 3u);
+                    const uint32_t pix = y * J.P.W + x, gpix = sc * npix + pix;
+                    if (x < J.P.W && y < J.P.H)
+                    {
+                        const uint32_t sidx = J.P.sample_offset + J.sample0 + s;
+                        f3 o, d;
+                        primary(J.P, J.cams ? J.cams[sc] : J.P.cam, x, y, pix, sidx, o, d);
+                        r0 = make_float4(o.x, o.y, o.z, 1e-3f);
+                        r1 = make_float4(d.x, d.y, d.z, bits2f(0x7f800000u));
+                        S.tp[lane] = make_float4(1.f, 1.f, 1.f, __uint_as_float(gpix));
+                        S.sum[lane] = make_float4(0.f, 0.f, 0.f, __uint_as_float(sidx));
+                        bounce = 0;
+                        go = true;
+                    }
+                }
+            }
+            if (go)
+            {
+                const TraceRoot* R = T.root;
+                if (J.roots) { R = J.roots + __float_as_uint(S.tp[lane].w) / npix; }
+                L.start(S.w, *R, r0, r1, odd_tree);
+                S.w.id[lane] = bounce;
+                pending = true;
+            }
+            __syncwarp();
+            if (!more && !__any_sync(FULL, pending)) { break; }
+            continue;
+        }
+        warp_walk<0, STK>(L, stk, T, S.w, takers, serve);
+        warp_leaves<0, STK>(L, stk, T, S.w);
+    }
+}
+
 // The radiance of one sample of one pixel (primaryRay + pathTrace).
 __device__ __forceinline__ f3 path_sample(const TraceCtx& T, const RP& P, const Shade& S, uint32_t x, uint32_t y,
                                           uint32_t pix, uint32_t sidx)
@@ -208,25 +355,6 @@ __device__ __forceinline__ f3 path_sample(const TraceCtx& T, const RP& P, const 
         tmin = 1e-4f;
     }
     return L;
-}
-
-__global__ void __launch_bounds__(128)
-k_render_plain(TraceCtx T, RP P, Shade S, float* __restrict__ rgb, float* __restrict__ rgb2)
-{
-    const uint32_t x = blockIdx.x * 16 + (threadIdx.x & 15);
-    const uint32_t y = blockIdx.y * 8 + (threadIdx.x >> 4);
-    if (x >= P.W || y >= P.H) { return; }
-    const uint32_t pix = y * P.W + x;
-    f3 acc = mk3(0.f, 0.f, 0.f), acc2 = mk3(0.f, 0.f, 0.f);
-    for (uint32_t s = 0; s < P.spp; s++)
-    {
-        const f3 L = path_sample(T, P, S, x, y, pix, P.sample_offset + s);
-        acc = add3(acc, L);
-        acc2 = add3(acc2, mul3(L, L));
-    }
-    const float fs = (float)P.spp;
-    rgb[3 * pix] = acc.x / fs; rgb[3 * pix + 1] = acc.y / fs; rgb[3 * pix + 2] = acc.z / fs;
-    if (rgb2) { rgb2[3 * pix] = acc2.x / fs; rgb2[3 * pix + 1] = acc2.y / fs; rgb2[3 * pix + 2] = acc2.z / fs; }
 }
 
 // dst[3 key + c] += v.c for every lane with `valid`, lanes of the warp with equal keys summed
@@ -264,6 +392,10 @@ __device__ __forceinline__ void warp_add3(float* __restrict__ dst, uint32_t key,
     }
 }
 
+// Why a thread per pixel and per-lane traversal stay here: a material's emission gradient is one
+// 32-bit sum of millions of terms, off by 1.5e-4 from the exact one at 512 x 512 x 32, and where it
+// ends up depends on which tiles are at work together; schedules that trace 3-5 times faster move
+// it by up to 3e-5.
 // Path-replay adjoint, one thread per pixel (the plain schedule). Lanes run the replay's
 // bounce loop in step so the gradient adds can be combined per warp; pixels whose dL/dI is
 // zero are skipped.
@@ -327,97 +459,25 @@ k_adjoint(TraceCtx T, RP P, Shade S, const float* __restrict__ dimg, float* __re
     }
 }
 
-// ---- wavefront ----
-// ray queue: rt_ray records (o, tmin, d, tmax); path state: (tp.xyz, image pixel), (L.xyz,
-// sample); scene queue: the scene of each ray (batched renders). Image pixel = scene * W * H
-// + pixel of the scene. Paths are numbered sample-major: g = (sample * S + scene) * W * H + pixel.
-
+// Adds the samples of every pixel channel in sample order: acc (+)= rad[0 .. n), and their squares;
+// the last call divides by the sample count.
 __global__ void __launch_bounds__(256)
-k_wf_generate(RP P, const Cam* __restrict__ cams, uint32_t S, uint64_t g0, uint32_t n_paths, float4* __restrict__ rays,
-              float4* __restrict__ state, uint32_t* __restrict__ rscene, uint32_t* __restrict__ count)
+k_sum(const float* __restrict__ rad, uint64_t channels, uint32_t n, bool start, bool end, float spp, float* __restrict__ rgb,
+      float* __restrict__ rgb2)
 {
-    const uint32_t i = blockIdx.x * 256 + threadIdx.x;
-    if (i == 0) { *count = n_paths; }
-    if (i >= n_paths) { return; }
-    const uint64_t npix = (uint64_t)P.W * P.H;
-    const uint64_t g = g0 + i;
-    const uint32_t s = (uint32_t)(g / (npix * S));
-    const uint64_t rem = g - (uint64_t)s * npix * S;
-    const uint32_t sc = (uint32_t)(rem / npix);
-    const uint32_t pix = (uint32_t)(rem - (uint64_t)sc * npix);
-    const uint32_t x = pix % P.W, y = pix / P.W;
-    const Cam C = cams ? cams[sc] : P.cam;
-    f3 o, d;
-    primary(P, C, x, y, pix, P.sample_offset + s, o, d);
-    rays[2 * i] = make_float4(o.x, o.y, o.z, 1e-3f);
-    rays[2 * i + 1] = make_float4(d.x, d.y, d.z, bits2f(0x7f800000u));
-    state[2 * i] = make_float4(1.f, 1.f, 1.f, __uint_as_float((uint32_t)(sc * npix + pix)));
-    state[2 * i + 1] = make_float4(0.f, 0.f, 0.f, __uint_as_float(P.sample_offset + s));
-    if (rscene) { rscene[i] = sc; }
-}
-
-__device__ __forceinline__ void retire(float* acc, float* acc2, uint32_t gpix, f3 L)
-{
-    atomicAdd(&acc[3 * (size_t)gpix], L.x); atomicAdd(&acc[3 * (size_t)gpix + 1], L.y); atomicAdd(&acc[3 * (size_t)gpix + 2], L.z);
-    if (acc2)
+    for (uint64_t i = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x; i < channels; i += (uint64_t)gridDim.x * blockDim.x)
     {
-        atomicAdd(&acc2[3 * (size_t)gpix], L.x * L.x); atomicAdd(&acc2[3 * (size_t)gpix + 1], L.y * L.y);
-        atomicAdd(&acc2[3 * (size_t)gpix + 2], L.z * L.z);
-    }
-}
-
-__global__ void __launch_bounds__(256)
-k_wf_shade(TraceCtx T, RP P, Shade S, const Cam* __restrict__ cams, uint32_t bounce, const uint32_t* __restrict__ count_in,
-           const float4* __restrict__ rays, const float4* __restrict__ state, const float4* __restrict__ hits,
-           float4* __restrict__ rays_out, float4* __restrict__ state_out, uint32_t* __restrict__ rscene_out,
-           uint32_t* __restrict__ count_out, float* __restrict__ acc, float* __restrict__ acc2)
-{
-    const uint32_t n = *count_in;
-    const uint32_t npix = P.W * P.H;
-    for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x)
-    {
-        const float4 r0 = rays[2 * i], r1 = rays[2 * i + 1];
-        const float4 s0 = state[2 * i], s1 = state[2 * i + 1];
-        const float4 h0 = hits[2 * i], h1 = hits[2 * i + 1];
-        const uint32_t gpix = __float_as_uint(s0.w), sidx = __float_as_uint(s1.w);
-        f3 tp = mk3(s0.x, s0.y, s0.z), L = mk3(s1.x, s1.y, s1.z);
-        const f3 o = mk3(r0.x, r0.y, r0.z), d = mk3(r1.x, r1.y, r1.z);
-        const uint32_t flags = __float_as_uint(h1.w);
-        if (!(flags & RT_HIT_FLAG_HIT))
+        float acc = start ? 0.f : rgb[i], acc2 = start || !rgb2 ? 0.f : rgb2[i];
+#pragma unroll 4
+        for (uint32_t s = 0; s < n; s++)
         {
-            L = add3(L, mul3(tp, environment(P, d)));
-            retire(acc, acc2, gpix, L);
-            continue;
+            const float v = __ldcs(&rad[(uint64_t)s * channels + i]);
+            acc += v;
+            acc2 += v * v;
         }
-        const uint32_t sc = gpix / npix, pix = gpix - sc * npix;
-        const uint32_t seed = cams ? cams[sc].seed : P.cam.seed;
-        const f3 nrm = mk3(h1.x, h1.y, h1.z);
-        const Surf sf = surface(S, __float_as_uint(h0.w));
-        L = add3(L, mul3(tp, sf.emission));
-        f3 nd;
-        const bool alive = scatter(P, seed, sf, nrm, d, pix, sidx, bounce, tp, nd);
-        if (!alive || bounce >= P.max_bounce)
-        {
-            retire(acc, acc2, gpix, L);
-            continue;
-        }
-        const f3 no = add3(o, muls(d, h0.x));
-        const uint32_t j = atomicAdd(count_out, 1u);
-        rays_out[2 * j] = make_float4(no.x, no.y, no.z, 1e-4f);
-        rays_out[2 * j + 1] = make_float4(nd.x, nd.y, nd.z, bits2f(0x7f800000u));
-        state_out[2 * j] = make_float4(tp.x, tp.y, tp.z, s0.w);
-        state_out[2 * j + 1] = make_float4(L.x, L.y, L.z, s1.w);
-        if (rscene_out) { rscene_out[j] = sc; }
+        rgb[i] = end ? acc / spp : acc;
+        if (rgb2) { rgb2[i] = end ? acc2 / spp : acc2; }
     }
-}
-
-__global__ void k_wf_finish(const float* __restrict__ acc, const float* __restrict__ acc2, uint64_t n, float spp,
-                            float* __restrict__ rgb, float* __restrict__ rgb2)
-{
-    const uint64_t i = (uint64_t)blockIdx.x * 256 + threadIdx.x;
-    if (i >= n) { return; }
-    rgb[i] = acc[i] / spp;
-    if (rgb2) { rgb2[i] = acc2[i] / spp; }
 }
 
 Cam make_cam(const rt_render_cfg& c)
@@ -442,99 +502,13 @@ RP make_rp(const rt_render_cfg& c, const rt_shading& sh)
     return P;
 }
 
-// One wavefront render: S scenes (1 for a plain handle), per-scene cameras on the device
-// (nullptr: P.cam) and subtree roots (nullptr: the handle's root).
-struct WfJob
-{
-    RP              P;
-    const Cam*      cams;
-    uint32_t        S;
-    Shade           sh;
-    const TraceRoot* roots;
-    float*          rgb;
-    float*          rgb2;
-};
-
-constexpr uint32_t kMaxBounceQueues = 64;
-
-int wf_buffers(rt_bvh* B, const WfJob& J, const rt_wavefront_params& W)
-{
-    const uint64_t chunk = W.chunk_paths;
-    const uint64_t nimg = (uint64_t)J.S * J.P.W * J.P.H * 3;
-    for (int k = 0; k < 2; k++)
-    {
-        if (B->wf_rays[k].ensure(chunk * 32) || B->wf_state[k].ensure(chunk * 32) ||
-            (J.S > 1 && B->wf_scene[k].ensure(chunk * 4)))
-        {
-            return RT_E_CUDA;
-        }
-    }
-    if (B->wf_hits.ensure(chunk * 32) || B->wf_acc.ensure(nimg * 4 * 2) ||
-        B->wf_ctr.ensure((size_t)kMaxBounceQueues * 16 + 64) || B->trace_status.ensure(64))
-    {
-        return RT_E_CUDA;
-    }
-    return RT_OK;
-}
-
-// Issues every launch of the render on st: no host synchronisation and no allocation, so the
-// sequence can be captured into a CUDA graph. Returns the kernel launches issued via *n_kernels.
-int wf_issue(rt_bvh* B, const WfJob& J, const rt_wavefront_params& W, cudaStream_t st, uint32_t* n_kernels)
-{
-    const TraceCtx T = make_trace_ctx(B);
-    const RP& P = J.P;
-    const uint64_t npix = (uint64_t)P.W * P.H;
-    const uint64_t total = npix * J.S * P.spp;
-    const uint64_t nimg = npix * J.S * 3;
-    const uint32_t nb = P.max_bounce + 2;
-    float* acc = B->wf_acc.as<float>();
-    float* acc2 = J.rgb2 ? acc + nimg : nullptr;
-    uint32_t* counts = B->wf_ctr.as<uint32_t>();  // per bounce queue length
-    unsigned long long* tctr = reinterpret_cast<unsigned long long*>(counts + 2 * kMaxBounceQueues);  // per bounce trace counter
-    uint32_t* status = B->trace_status.as<uint32_t>() + 4;
-    const int sms = device_sm_count();
-    const int sblk = W.shade_block ? (int)W.shade_block : 256;
-    uint32_t nk = 0;
-    RT_CUDA(cudaMemsetAsync(acc, 0, nimg * 4 * (J.rgb2 ? 2 : 1), st));
-    TraceLaunch tl;
-    tl.block = (int)W.trace_block;
-    tl.stack = (int)W.stack_depth;
-    tl.roots = J.roots;
-    for (uint64_t g0 = 0; g0 < total; g0 += W.chunk_paths)
-    {
-        const uint32_t n_paths = (uint32_t)std::min<uint64_t>(W.chunk_paths, total - g0);
-        RT_CUDA(cudaMemsetAsync(counts, 0, (size_t)kMaxBounceQueues * 16, st));
-        k_wf_generate<<<(n_paths + 255) / 256, 256, 0, st>>>(P, J.cams, J.S, g0, n_paths, B->wf_rays[0].as<float4>(),
-                                                              B->wf_state[0].as<float4>(),
-                                                              J.S > 1 ? B->wf_scene[0].as<uint32_t>() : nullptr, counts);
-        nk++;
-        int cur = 0;
-        for (uint32_t b = 0; b <= P.max_bounce; b++)
-        {
-            tl.rscene = J.S > 1 ? B->wf_scene[cur].as<uint32_t>() : nullptr;
-            if (int e = trace_launch(B, B->wf_rays[cur].p, B->wf_hits.p, 0, counts + b, 0u, st, status, tctr + b, tl)) { return e; }
-            k_wf_shade<<<sms * 2048 / sblk, sblk, 0, st>>>(T, P, J.sh, J.cams, b, counts + b, B->wf_rays[cur].as<float4>(),
-                                                         B->wf_state[cur].as<float4>(), B->wf_hits.as<float4>(),
-                                                         B->wf_rays[cur ^ 1].as<float4>(), B->wf_state[cur ^ 1].as<float4>(),
-                                                         J.S > 1 ? B->wf_scene[cur ^ 1].as<uint32_t>() : nullptr,
-                                                         counts + b + 1, acc, acc2);
-            nk += 2;
-            cur ^= 1;
-        }
-        if (int e = check_launch("wavefront")) { return e; }
-        (void)nb;
-    }
-    k_wf_finish<<<(uint32_t)((nimg + 255) / 256), 256, 0, st>>>(acc, acc2, nimg, (float)P.spp, J.rgb, J.rgb2);
-    nk++;
-    if (n_kernels) { *n_kernels = nk; }
-    return check_launch("wavefront finish");
-}
+constexpr uint32_t MAX_WAVEFRONT_BOUNCE = 62;
 
 rt_wavefront_params default_params()
 {
     rt_wavefront_params W;
-    W.trace_block = 128;
-    W.chunk_paths = 1u << 22;
+    W.trace_block = 256;
+    W.chunk_paths = 1u << 25;
     W.stack_depth = 64;
     W.shade_block = 256;
     return W;
@@ -549,51 +523,109 @@ int check_params(const rt_wavefront_params& W)
     return RT_OK;
 }
 
-// Replays the job from the handle's cached CUDA graph (captured on first use of a
-// configuration) on the handle's own stream, ordered after / before the caller's stream.
-int wf_run_graph(rt_bvh* B, const WfJob& J, const rt_wavefront_params& W, cudaStream_t st)
+// The scratch of one render: radiance of the paths in flight, per-scene cameras and
+// the item counter. It belongs to the handle and is passed from call to call through an event, so
+// calls on other streams and host threads queue up behind one another; a call that is being
+// captured into a graph owns its scratch as memory nodes of that graph.
+class PathScratch
 {
-    if (int e = wf_buffers(B, J, W)) { return e; }
-    // the graph bakes in kernel arguments and buffer addresses: all of them form its key
-    // (and the traversal form: binary one-loop / while-while, or the 8-wide layout)
-    const void* ptrs[] = { B->wf_rays[0].p, B->wf_rays[1].p, B->wf_state[0].p, B->wf_state[1].p, B->wf_scene[0].p,
-                           B->wf_scene[1].p, B->wf_hits.p, B->wf_acc.p, B->wf_ctr.p, B->trace_status.p, B->gnodes.p,
-                           B->tripos.p, B->tris.p, B->verts.p, B->rootbuf.p, B->scene_roots.p, B->wnodes.p, B->wid.p };
-    const uint32_t form[2] = { B->trace_ww ? 1u : 0u, B->trace_wide ? 1u : 0u };
-    std::vector<unsigned char> key(sizeof(WfJob) + sizeof(W) + sizeof(ptrs) + sizeof(form));
-    std::memset(key.data(), 0, key.size());
-    std::memcpy(key.data(), &J, sizeof(WfJob));
-    std::memcpy(key.data() + sizeof(WfJob), &W, sizeof(W));
-    std::memcpy(key.data() + sizeof(WfJob) + sizeof(W), ptrs, sizeof(ptrs));
-    std::memcpy(key.data() + sizeof(WfJob) + sizeof(W) + sizeof(ptrs), form, sizeof(form));
-    if (!B->wf_stream)
+    rt_bvh*                      B_;
+    cudaStream_t                 st_;
+    bool                         capturing_ = false;
+    std::unique_lock<std::mutex> lk_;
+    void*                        mem_ = nullptr;
+
+public:
+    PathScratch(rt_bvh* B, cudaStream_t st) : B_(B), st_(st), lk_(B->wf_mu) {}
+    int get(size_t bytes, void** p)
     {
-        RT_CUDA(cudaStreamCreateWithFlags(&B->wf_stream, cudaStreamNonBlocking));
-        RT_CUDA(cudaEventCreateWithFlags(&B->wf_ev[0], cudaEventDisableTiming));
-        RT_CUDA(cudaEventCreateWithFlags(&B->wf_ev[1], cudaEventDisableTiming));
+        cudaStreamCaptureStatus cs = cudaStreamCaptureStatusNone;
+        RT_CUDA(cudaStreamIsCapturing(st_, &cs));
+        capturing_ = cs != cudaStreamCaptureStatusNone;
+        if (capturing_)
+        {
+            RT_CUDA(cudaMallocAsync(&mem_, bytes, st_));
+            *p = mem_;
+            return RT_OK;
+        }
+        if (!B_->wf_ev) { RT_CUDA(cudaEventCreateWithFlags(&B_->wf_ev, cudaEventDisableTiming)); }
+        else { RT_CUDA(cudaStreamWaitEvent(st_, B_->wf_ev, 0)); }
+        if (B_->wf_buf.ensure(bytes)) { return RT_E_CUDA; }
+        *p = B_->wf_buf.p;
+        return RT_OK;
     }
-    if (!B->wf_exec || key != B->wf_key)
+    bool capturing() const { return capturing_; }
+    ~PathScratch()
     {
-        if (B->wf_exec) { cudaGraphExecDestroy(B->wf_exec); B->wf_exec = nullptr; }
-        RT_CUDA(cudaStreamBeginCapture(B->wf_stream, cudaStreamCaptureModeThreadLocal));
-        uint32_t nk = 0;
-        const int e = wf_issue(B, J, W, B->wf_stream, &nk);
-        cudaGraph_t g = nullptr;
-        const cudaError_t ce = cudaStreamEndCapture(B->wf_stream, &g);
-        if (e) { if (g) { cudaGraphDestroy(g); } return e; }
-        if (ce != cudaSuccess) { return fail(RT_E_CUDA, std::string("graph capture: ") + cudaGetErrorString(ce)); }
-        const cudaError_t ie = cudaGraphInstantiate(&B->wf_exec, g, 0);
-        cudaGraphDestroy(g);
-        if (ie != cudaSuccess) { B->wf_exec = nullptr; return fail(RT_E_CUDA, std::string("graph instantiate: ") + cudaGetErrorString(ie)); }
-        B->wf_key = key;
-        B->wf_kernels = nk;
+        if (mem_) { cudaFreeAsync(mem_, st_); }
+        else if (!capturing_ && B_->wf_ev) { cudaEventRecord(B_->wf_ev, st_); }
     }
-    RT_CUDA(cudaEventRecord(B->wf_ev[0], st));
-    RT_CUDA(cudaStreamWaitEvent(B->wf_stream, B->wf_ev[0], 0));
-    RT_CUDA(cudaGraphLaunch(B->wf_exec, B->wf_stream));
-    count_launch(B->wf_kernels);
-    RT_CUDA(cudaEventRecord(B->wf_ev[1], B->wf_stream));
-    RT_CUDA(cudaStreamWaitEvent(st, B->wf_ev[1], 0));
+};
+
+using PathFn = void (*)(TraceCtx, PathJob, uint32_t*, int);
+
+int launch_paths(PathFn fn, const TraceCtx& T, const PathJob& J, uint32_t* counter, uint32_t block, cudaStream_t st)
+{
+    const size_t smem = (size_t)(block / 32) * sizeof(PathShare);
+    const int per_sm = blocks_per_sm(reinterpret_cast<const void*>(fn), (int)block, smem);
+    // few items are spread over the resident warps (as few rays are by trace_launch)
+    const uint64_t warps = (uint64_t)device_sm_count() * (uint64_t)per_sm * (block / 32);
+    const uint64_t per_warp = std::min<uint64_t>(32, (J.n + warps - 1) / warps);
+    const uint64_t grid = std::min<uint64_t>((uint64_t)device_sm_count() * (uint64_t)per_sm,
+                                             (J.n + per_warp * (block / 32) - 1) / (per_warp * (block / 32)));
+    RT_CUDA(cudaMemsetAsync(counter, 0, 4, st));
+    fn<<<(uint32_t)grid, block, smem, st>>>(T, J, counter, (int)per_warp);
+    count_launch();
+    return check_launch("paths");
+}
+
+// Renders J's scenes. Samples are taken in groups
+// whose paths fit W.chunk_paths (at least one sample of every pixel), each group launched in pieces
+// of at most that many paths.
+int run_paths(const rt_bvh* B, PathJob J, const Cam* h_cams, const rt_wavefront_params& W, float* rgb, float* rgb2,
+              cudaStream_t st)
+{
+    const uint64_t npix = (uint64_t)J.P.W * J.P.H;
+    const uint64_t tiles_x = ((uint64_t)J.P.W + 7) / 8, items = tiles_x * (((uint64_t)J.P.H + 3) / 4) * 32;
+    if (items * J.S > 0xffffffffull) { return fail(RT_E_CAPACITY, "more than 2^32 pixels"); }
+    J.tiles_x = (uint32_t)tiles_x;
+    J.scene_items = (uint32_t)items;
+    const uint64_t per_sample = items * J.S;
+    const uint64_t group = std::max<uint64_t>(1, std::min<uint64_t>(W.chunk_paths / per_sample, J.P.spp));
+    const uint64_t rad_bytes = (group * npix * J.S * 12 + 255) / 256 * 256, cam_bytes = (J.S * sizeof(Cam) + 255) / 256 * 256;
+    PathScratch scratch(const_cast<rt_bvh*>(B), st);
+    void* mem = nullptr;
+    if (int e = scratch.get(rad_bytes + cam_bytes + 256, &mem)) { return e; }
+    J.rad = static_cast<float*>(mem);
+    Cam* cams = reinterpret_cast<Cam*>(static_cast<char*>(mem) + rad_bytes);
+    uint32_t* counter = reinterpret_cast<uint32_t*>(static_cast<char*>(mem) + rad_bytes + cam_bytes);
+    if (h_cams)
+    {
+        if (scratch.capturing()) { return fail(RT_E_INVALID, "a render of several scenes cannot be captured"); }
+        // (an upload from pageable memory has left the host array when cudaMemcpyAsync returns)
+        RT_CUDA(cudaMemcpyAsync(cams, h_cams, J.S * sizeof(Cam), cudaMemcpyHostToDevice, st));
+        J.cams = cams;
+    }
+    const TraceCtx T = make_trace_ctx(B);
+    const PathFn fn = W.stack_depth < 64 ? k_paths<32> : k_paths<STACK>;
+    const uint64_t channels = npix * J.S * 3;
+    for (uint64_t s0 = 0; s0 < J.P.spp; s0 += group)
+    {
+        const uint64_t ns = std::min<uint64_t>(group, J.P.spp - s0), all = ns * per_sample;
+        const uint64_t piece = std::min<uint64_t>(std::max<uint64_t>(W.chunk_paths, 1), 1ull << 30);
+        J.sample0 = (uint32_t)s0;
+        for (uint64_t g = 0; g < all; g += piece)
+        {
+            J.first = (uint32_t)g;
+            J.n = (uint32_t)std::min<uint64_t>(piece, all - g);
+            if (int e = launch_paths(fn, T, J, counter, W.trace_block, st)) { return e; }
+        }
+        const uint64_t blocks = (channels + W.shade_block - 1) / W.shade_block;
+        k_sum<<<(uint32_t)std::min<uint64_t>(blocks, 1u << 20), W.shade_block, 0, st>>>(J.rad, channels, (uint32_t)ns, s0 == 0,
+                                                                                  s0 + ns == J.P.spp, (float)J.P.spp, rgb, rgb2);
+        count_launch();
+        if (int e = check_launch("sample sums")) { return e; }
+    }
     return RT_OK;
 }
 
@@ -611,32 +643,22 @@ rt_wavefront_params pick_params(const rt_bvh* B, const rt_wavefront_params* W)
 int render(const rt_bvh* B, const rt_render_cfg& cfg, const rt_shading& sh, int mode, float* rgb, float* rgb2,
            cudaStream_t st)
 {
-    const TraceCtx T = make_trace_ctx(B);
-    const RP P = make_rp(cfg, sh);
-    const Shade S{ sh.mats, sh.mat_of_tri, sh.tri_albedo, sh.n_mats };
-    if (mode == RT_RENDER_PLAIN)
-    {
-        const dim3 grid((cfg.width + 15) / 16, (cfg.height + 7) / 8);
-        k_render_plain<<<grid, 128, 0, st>>>(T, P, S, rgb, rgb2);
-        count_launch();
-        return check_launch("render plain");
-    }
-    if (mode != RT_RENDER_WAVEFRONT) { return fail(RT_E_INVALID, "unknown render mode"); }
-    if (cfg.max_bounce + 2 > kMaxBounceQueues) { return fail(RT_E_INVALID, "max_bounce must be below 62 for the wavefront"); }
-    rt_bvh* Bm = const_cast<rt_bvh*>(B);
-    WfJob J;
-    std::memset(&J, 0, sizeof(J));
-    J.P = P; J.cams = nullptr; J.S = 1; J.sh = S; J.roots = nullptr; J.rgb = rgb; J.rgb2 = rgb2;
-    rt_wavefront_params W = pick_params(B, nullptr);
-    if (W.stack_depth < 64) { W.stack_depth = 64; }  // tuned for a batch; a plain handle keeps the full stack
-    return wf_run_graph(Bm, J, W, st);
+    if (mode != RT_RENDER_PLAIN && mode != RT_RENDER_WAVEFRONT) { return fail(RT_E_INVALID, "unknown render mode"); }
+    if (mode == RT_RENDER_WAVEFRONT && cfg.max_bounce > MAX_WAVEFRONT_BOUNCE) { return fail(RT_E_INVALID, "max_bounce must be below 63 for the wavefront"); }
+    PathJob J{};
+    J.P = make_rp(cfg, sh);
+    J.S = 1;
+    J.sh = Shade{ sh.mats, sh.mat_of_tri, sh.tri_albedo, sh.n_mats };
+    rt_wavefront_params W = mode == RT_RENDER_WAVEFRONT ? pick_params(B, nullptr) : default_params();
+    W.stack_depth = 64;  // tuned for a batch; a plain handle keeps the full stack
+    return run_paths(B, J, nullptr, W, rgb, rgb2, st);
 }
 
 int render_batch(rt_bvh* B, const rt_render_cfg* cfgs, uint32_t S, const rt_shading& sh, const rt_wavefront_params* params,
                  float* rgb, float* rgb2, cudaStream_t st)
 {
     const rt_render_cfg& c0 = cfgs[0];
-    if (c0.max_bounce + 2 > kMaxBounceQueues) { return fail(RT_E_INVALID, "max_bounce must be below 62 for the wavefront"); }
+    if (c0.max_bounce > MAX_WAVEFRONT_BOUNCE) { return fail(RT_E_INVALID, "max_bounce must be below 63 for the wavefront"); }
     const rt_wavefront_params W = pick_params(B, params);
     if (int e = check_params(W)) { return e; }
     if (W.stack_depth < 64)
@@ -647,19 +669,12 @@ int render_batch(rt_bvh* B, const rt_render_cfg* cfgs, uint32_t S, const rt_shad
     }
     std::vector<Cam> cams(S);
     for (uint32_t s = 0; s < S; s++) { cams[s] = make_cam(cfgs[s]); }
-    if (B->wf_cams.ensure((size_t)S * sizeof(Cam))) { return RT_E_CUDA; }
-    RT_CUDA(cudaMemcpyAsync(B->wf_cams.p, cams.data(), (size_t)S * sizeof(Cam), cudaMemcpyHostToDevice, st));
-    WfJob J;
-    std::memset(&J, 0, sizeof(J));
+    PathJob J{};
     J.P = make_rp(c0, sh);
-    J.cams = B->wf_cams.as<Cam>();
     J.S = S;
     J.sh = Shade{ sh.mats, sh.mat_of_tri, sh.tri_albedo, sh.n_mats };
     J.roots = S > 1 ? B->scene_roots.as<TraceRoot>() : nullptr;  // one scene: the whole tree
-    J.rgb = rgb; J.rgb2 = rgb2;
-    if (S == 1) { J.cams = nullptr; J.P.cam = cams[0]; }
-    // (an upload from pageable memory has left the host vector when cudaMemcpyAsync returns)
-    return wf_run_graph(B, J, W, st);
+    return run_paths(B, J, S > 1 ? cams.data() : nullptr, W, rgb, rgb2, st);
 }
 
 int autotune_wavefront(rt_bvh* B, const rt_render_cfg* cfgs, uint32_t S, const rt_shading& sh, rt_wavefront_params* best,
@@ -697,7 +712,7 @@ int autotune_wavefront(rt_bvh* B, const rt_render_cfg* cfgs, uint32_t S, const r
                 rt_wavefront_params W = default_params();
                 W.trace_block = blk; W.chunk_paths = ch; W.stack_depth = stack;
                 float ms = 0.f;
-                for (int rep = 0; rep < 2 && !err; rep++)  // the first run captures the graph
+                for (int rep = 0; rep < 2 && !err; rep++)  // the first run warms up
                 {
                     if (cudaEventRecord(a, st) != cudaSuccess) { err = fail(RT_E_CUDA, "event"); break; }
                     err = render_batch(B, c1.data(), S, sh, &W, scratch_rgb, nullptr, st);

@@ -4,6 +4,7 @@
 #include <atomic>
 #include <cstddef>
 #include <cstdint>
+#include <mutex>
 #include <string>
 #include <vector>
 
@@ -206,17 +207,17 @@ struct rt_bvh
     rtb::DevBuf  scene_info, scene_roots;
     std::vector<uint32_t> scene_info_host;
     uint32_t     depth = 0;                 // tree depth (computed on demand; 0 = unknown)
-    bool         trace_ww = true;           // traversal loop form: while-while for large leaves
+    bool         trace_ww = true;           // loop form of the adjoint's traversal
     bool         trace_wide = false;        // traverse the 8-wide layout (rebuilt after every rebuild)
     rtb::DevBuf  wnodes, wid;               // wide layout and the wide index of each binary node
     uint32_t     n_wide = 0;
     uint32_t     stats[8] = {0, 0, 0, 0, 0, 0, 0, 0};
     BuildScratch s;
     rtb::DevBuf  trace_status, trace_rays, trace_hits;
-    rtb::DevBuf  wf_rays[2], wf_state[2], wf_hits, wf_acc, wf_ctr;  // wavefront path tracer
-    rtb::DevBuf  wf_scene[2], wf_cams;      // scene of each queued ray; per-scene cameras
-    cudaStream_t wf_stream = nullptr;       // the graph replays here, fenced by wf_ev
-    cudaEvent_t  wf_ev[2] = { nullptr, nullptr };
+    // the path tracer's scratch, handed from call to call through wf_ev (render.cu)
+    std::mutex   wf_mu;
+    rtb::DevBuf  wf_buf;
+    cudaEvent_t  wf_ev = nullptr;
     // an LBVH bake's launch sequence, captured on the second call with the same key (sizes,
     // settings, inputs, buffer addresses) and replayed on bake_stream (fenced with the caller's
     // stream by bake_ev); its key, and the key the last plain bake left
@@ -227,9 +228,6 @@ struct rt_bvh
     uint32_t*    bake_perm = nullptr;
     cudaStream_t bake_stream = nullptr;
     cudaEvent_t  bake_ev[2] = { nullptr, nullptr };
-    cudaGraphExec_t wf_exec = nullptr;      // the captured launch sequence and its key
-    std::vector<unsigned char> wf_key;
-    uint32_t     wf_kernels = 0;
     rt_wavefront_params wf_tuned = { 0, 0, 0, 0 };
     bool         wf_tuned_valid = false;
     // stage timing (rt_bvh_profile): events at the stage boundaries of a build
@@ -240,7 +238,7 @@ struct rt_bvh
 
 namespace rtb
 {
-// The traversal loop form for a tree with n_tris triangles in n_leaves leaves: the
+// The loop form of the adjoint's traversal for a tree with n_tris triangles in n_leaves leaves: the
 // while-while loop pays off when leaves hold 6 or more triangles on average.
 inline bool prefer_while_while(uint64_t n_tris, uint64_t n_leaves) { return n_tris >= 6 * n_leaves; }
 
@@ -291,6 +289,8 @@ struct TraceLaunch
 // d_counter must be zero on entry.
 int trace_launch(const rt_bvh* b, const void* d_rays, void* d_hits, uint64_t n, const uint32_t* n_dev, uint32_t flags,
                  cudaStream_t st, uint32_t* d_status, unsigned long long* d_counter, const TraceLaunch& opt);
+// traverse.cu: resident blocks per SM of a kernel (cached)
+int blocks_per_sm(const void* fn, int block, size_t smem);
 // render.cu
 int render(const rt_bvh* b, const rt_render_cfg& cfg, const rt_shading& sh, int mode, float* rgb, float* rgb2,
            cudaStream_t st);

@@ -1,5 +1,6 @@
-// trace_core.cuh -- the traversal loop shared by the trace kernels and the path tracers:
-// bvh::trace (src/bvh/bvh_traverse.cpp:91-178) over the 64-byte two-child node layout.
+// trace_core.cuh -- box and triangle tests, the traversal context, and per-lane traversal loops: bvh::trace
+// (src/bvh/bvh_traverse.cpp:91-178) over the 64-byte two-child node layout for the adjoint, and
+// over the 8-wide layout. (Traces and images: trace_warp.cuh.)
 #pragma once
 
 #include "device_math.cuh"

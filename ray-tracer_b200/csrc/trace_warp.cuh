@@ -305,11 +305,11 @@ __device__ __forceinline__ void warp_leaves(LaneTrace<MODE, STK>& L, uint2 (&stk
     }
 }
 
-// Walks inner nodes until every live lane stands at a leaf, or enough lanes wait (more: finished
-// lanes can get new rays; idle: how many lanes those are when they may).
+// Walks inner nodes until every live lane stands at a leaf, or few lanes walk and others wait at a
+// leaf or, `serve` or more of `takers`, to be served by the caller (a new ray).
 template <int MODE, int STK>
 __device__ __forceinline__ void warp_walk(LaneTrace<MODE, STK>& L, uint2 (&stk)[STK], const TraceCtx& T, const WarpShare& S,
-                                          unsigned lanes, bool more, int refill)
+                                          unsigned takers, int serve)
 {
     constexpr unsigned FULL = 0xffffffffu;
     uint32_t it = 0;
@@ -321,7 +321,7 @@ __device__ __forceinline__ void warp_walk(LaneTrace<MODE, STK>& L, uint2 (&stk)[
         if (it > 0 && __popc(walking) < WALK_MIN)
         {
             const unsigned live = __ballot_sync(FULL, L.live);
-            if (live != walking || (more && __popc(lanes & ~live) >= refill)) { break; }
+            if (live != walking || __popc(takers & ~live) >= serve) { break; }
         }
         if (walk) { L.step(stk, T.gn, S); }
         __syncwarp();

@@ -2,7 +2,7 @@
 // for batches of rays on the GPU.
 //
 // Layout: the .bvh node array is re-laid as 64-byte two-child nodes (rt_gnode: both children's
-// boxes and references, four 128-bit loads per visited inner node) and a 48-byte triangle
+// boxes and references, two 256-bit loads per visited inner node) and a 48-byte triangle
 // position record per baked triangle (three 128-bit loads per triangle test). Node indices are
 // those of the .bvh array, so the traversal visits exactly the reference's nodes.
 //
@@ -14,7 +14,7 @@
 // do not depend on bestT). Children are tested and pushed in the reference's order (far child
 // first, the left child first on ties, :143-174) and triangles are tested in leaf order with the
 // strict "t < bestT" update (:112-142), so the first triangle at the minimal distance wins as
-// in the reference and hits carry identical triangle indices (trace_core.cuh).
+// in the reference and hits carry identical triangle indices (trace_warp.cuh).
 //
 // The kernel is persistent: warps claim rays from a global counter as their lanes finish, and
 // test leaves together (trace_warp.cuh).
@@ -205,7 +205,7 @@ k_trace(TraceCtx T, const float4* __restrict__ rays, float4* __restrict__ hits, 
             __syncwarp();
             continue;
         }
-        warp_walk<MODE, STK>(L, stk, T, S, lanes, more, refill);
+        warp_walk<MODE, STK>(L, stk, T, S, more ? lanes : 0u, refill);
         warp_leaves<MODE, STK>(L, stk, T, S);
     }
 }
@@ -267,26 +267,28 @@ TraceFn trace_fn(uint32_t flags, int stack, bool roots, bool wide)
     }
 }
 
-// Resident blocks per SM, per kernel variant and block size.
+// Resident blocks per SM, per device, kernel variant and block size.
 std::mutex g_occ_mu;
-struct OccKey { TraceFn fn; int block; int v; };
+struct OccKey { const void* fn; int device, block, v; };
 std::vector<OccKey> g_occ;
 
-int blocks_per_sm(TraceFn fn, int block, size_t smem)
+} // namespace
+
+int blocks_per_sm(const void* fn, int block, size_t smem)
 {
+    int device = 0;
+    cudaGetDevice(&device);
     std::lock_guard<std::mutex> lk(g_occ_mu);
     for (const OccKey& k : g_occ)
     {
-        if (k.fn == fn && k.block == block) { return k.v; }
+        if (k.fn == fn && k.device == device && k.block == block) { return k.v; }
     }
     int v = 0;
     if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&v, fn, block, smem) != cudaSuccess) { cudaGetLastError(); v = 1; }
     if (v < 1) { v = 1; }
-    g_occ.push_back(OccKey{ fn, block, v });
+    g_occ.push_back(OccKey{ fn, device, block, v });
     return v;
 }
-
-} // namespace
 
 TraceCtx make_trace_ctx(const rt_bvh* B)
 {
@@ -350,7 +352,7 @@ int trace_launch(const rt_bvh* B, const void* d_rays, void* d_hits, uint64_t n, 
     const int block = opt.block > 0 ? opt.block : TBLK;
     if (block % 32 || block > 256) { return fail(RT_E_INVALID, "trace block must be a multiple of 32, at most 256"); }
     const size_t smem = B->trace_wide ? 0 : (size_t)(block / 32) * sizeof(WarpShare);
-    uint64_t grid = (uint64_t)device_sm_count() * (uint64_t)blocks_per_sm(fn, block, smem);
+    uint64_t grid = (uint64_t)device_sm_count() * (uint64_t)blocks_per_sm(reinterpret_cast<const void*>(fn), block, smem);
     int per_warp = 32;
     if (!n_dev)
     {

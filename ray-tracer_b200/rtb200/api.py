@@ -351,9 +351,9 @@ class Bvh:
         _check(lib().rt_write_bvh(self.h, path.encode()))
 
     def trace_loop(self, form: int = -1):
-        """Traversal form: 0 one-loop, 1 while-while, -1 the default choice by leaf size (all three
-        the reference's visiting order); 2 the 8-wide layout (same closest distance, ties may
-        report another triangle; kept up to date across rebuilds)."""
+        """Traversal form: -1, 0 and 1 the reference's visiting order over the binary tree; 2 the
+        8-wide layout for trace() (same closest distance, ties may report another triangle; kept up
+        to date across rebuilds)."""
         _check(lib().rt_bvh_trace_loop(self.h, int(form)))
 
     def wide_nodes(self):
@@ -394,7 +394,7 @@ class Bvh:
         import torch
         rgb = torch.empty((rcfg.height, rcfg.width, 3), dtype=torch.float32, device="cuda")
         rgb2 = torch.empty_like(rgb) if want_sq else None
-        sh, keep = _shading(mats, mat_of_tri, tri_albedo, env_map)
+        sh, keep = _shading(mats, mat_of_tri, tri_albedo, env_map, self.counts()[1])
         _check(lib().rt_render_ex(self.h, C.byref(rcfg), C.byref(sh), mode, _ptr(rgb), _ptr(rgb2),
                                   _stream_ptr(stream, True)))
         del keep
@@ -410,7 +410,7 @@ class Bvh:
         assert d_rgb.is_cuda and d_rgb.numel() == rcfg.width * rcfg.height * 3
         g_alb = torch.zeros((nt, 3), dtype=torch.float32, device="cuda")
         g_em = torch.zeros((len(mats), 3), dtype=torch.float32, device="cuda") if mats is not None else None
-        sh, keep = _shading(mats, mat_of_tri, tri_albedo)
+        sh, keep = _shading(mats, mat_of_tri, tri_albedo, n_tris=nt)
         _check(lib().rt_adjoint(self.h, C.byref(rcfg), C.byref(sh), _ptr(d_rgb), _ptr(g_alb), _ptr(g_em),
                                 _stream_ptr(stream, True)))
         del keep
@@ -419,7 +419,7 @@ class Bvh:
 
     def render_batch(self, rcfgs, mats=None, mat_of_tri=None, params: WavefrontParams | None = None, want_sq=False,
                      stream=None, tri_albedo=None):
-        """All scenes of a batched handle in one wavefront render: rcfgs = one RenderCfg per scene
+        """All scenes of a batched handle in one render: rcfgs = one RenderCfg per scene
         (camera and seed; the rest from rcfgs[0]). Returns (rgb, rgb2) (n_scenes, H, W, 3)."""
         import torch
         n = len(rcfgs)
@@ -427,7 +427,7 @@ class Bvh:
         c0 = rcfgs[0]
         rgb = torch.empty((n, c0.height, c0.width, 3), dtype=torch.float32, device="cuda")
         rgb2 = torch.empty_like(rgb) if want_sq else None
-        sh, keep = _shading(mats, mat_of_tri, tri_albedo)
+        sh, keep = _shading(mats, mat_of_tri, tri_albedo, n_tris=self.counts()[1])
         _check(lib().rt_render_batch(self.h, arr, n, C.byref(sh), C.byref(params) if params is not None else None,
                                      _ptr(rgb), _ptr(rgb2), _stream_ptr(stream, True)))
         del keep
@@ -498,8 +498,10 @@ def _device_u32(x):
     return torch.from_numpy(np.ascontiguousarray(x, np.uint32).view(np.int32)).cuda()
 
 
-def _shading(mats, mat_of_tri, tri_albedo, env_map=None):
-    """An rt_shading record over device copies of the inputs (kept alive by the caller)."""
+def _shading(mats, mat_of_tri, tri_albedo, env_map=None, n_tris=0):
+    """An rt_shading record over device copies of the inputs (kept alive by the caller). An albedo
+    table with fewer than n_tris rows (baked triangles: spatial splits add some) is continued in
+    black, so that no kernel reads past it."""
     import torch
     sh = Shading()
     keep = []
@@ -519,6 +521,8 @@ def _shading(mats, mat_of_tri, tri_albedo, env_map=None):
     if tri_albedo is not None:
         ta = tri_albedo.detach() if _is_torch(tri_albedo) else torch.from_numpy(np.ascontiguousarray(tri_albedo, np.float32))
         ta = ta.to(device="cuda", dtype=torch.float32).contiguous()
+        if ta.numel() < 3 * n_tris:
+            ta = torch.cat([ta.reshape(-1), ta.new_zeros(3 * n_tris - ta.numel())])
         keep.append(ta)
         sh.tri_albedo = ta.data_ptr()
     return sh, keep

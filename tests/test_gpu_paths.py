@@ -1,0 +1,104 @@
+"""The persistent path kernel where it can go wrong: images that are not whole tiles, fewer paths than
+lanes, sample groups and launch pieces of every kind, calls on several streams, graph capture."""
+import numpy as np
+import pytest
+
+import rtb200
+from oracle import Baked
+from render_checks import orc_cfg_from
+from test_gpu_batch import batch_setup, cfgs_for
+from test_gpu_render import compare, cornell_scene
+
+pytestmark = pytest.mark.gpu
+VIEW = ((0.0, 0.0, -2.9), (0.0, 0.0, 0.0), 45.0)
+
+
+def scene(preset="lbvh30"):
+    v, t, obj, mats = cornell_scene()
+    b = rtb200.Bvh.build(v, t, preset)
+    return b, mats, obj[b.prim_ids()]
+
+
+@pytest.mark.parametrize("w,h,spp", [(1, 1, 300), (7, 5, 40), (8, 4, 33), (9, 33, 16), (61, 43, 9)])
+def test_image_sizes_match_oracle(orc, w, h, spp):
+    b, mats, mot = scene()
+    nodes, tris, verts = b.download()
+    rc = rtb200.render_cfg(w, h, spp, max_bounce=4, rr_after=1, env_kind=1, env_color=(0.1, 0.2, 0.3), seed=w, lookat=VIEW)
+    rgb, rgb2 = b.render(rc, mats, mot, want_sq=True)
+    ref, ref2 = orc.render(Baked(nodes, tris, verts), orc_cfg_from(rc), mats, mot, threads=8, want_sq=True)
+    # a pixel sums spp samples; a sample differs where host and device cosf / sinf round apart
+    compare(rgb, rgb2, ref, ref2, spp, f"{w}x{h}x{spp}", min_equal=0.0)
+
+
+@pytest.mark.parametrize("chunk,stack,blk", [(1024, 64, 32), (4096, 64, 256), (16384, 64, 96), (1 << 26, 64, 128)])
+def test_groups_and_pieces_give_the_same_image(chunk, stack, blk):
+    """Samples are summed in order whatever the launches are: bit-equal images."""
+    scs, bb, mats, mot = batch_setup(n=3)
+    rcs = cfgs_for(scs, 50, 37, 7, max_bounce=4, rr_after=2)
+    a, a2 = bb.render_batch(rcs, mats, mot, want_sq=True)
+    c, c2 = bb.render_batch(rcs, mats, mot, params=rtb200.WavefrontParams(blk, chunk, stack, 256), want_sq=True)
+    assert np.array_equal(a.cpu().numpy(), c.cpu().numpy()) and np.array_equal(a2.cpu().numpy(), c2.cpu().numpy())
+
+
+def test_calls_on_two_streams():
+    import torch
+    b, mats, mot = scene("hybrid")
+    rc = [rtb200.render_cfg(128, 96, 16, max_bounce=4, rr_after=-1, env_kind=1, seed=s, lookat=VIEW) for s in (1, 2)]
+    want = [b.render(r, mats, mot)[0].cpu().numpy() for r in rc]
+    streams = [torch.cuda.Stream() for _ in rc]
+    dm, dmot = torch.from_numpy(rtb200.materials_array(mats)).cuda(), torch.from_numpy(mot.astype(np.int32)).cuda()
+    torch.cuda.synchronize()
+    got = []
+    for k in range(6):
+        with torch.cuda.stream(streams[k % 2]):
+            got.append(b.render(rc[k % 2], dm, dmot)[0])
+    torch.cuda.synchronize()
+    for k, g in enumerate(got):
+        assert np.array_equal(g.cpu().numpy(), want[k % 2]), k
+
+
+def test_capture_and_replay():
+    import torch
+    b, mats, mot = scene("hybrid")
+    rc = rtb200.render_cfg(40, 30, 8, max_bounce=4, rr_after=-1, env_kind=1, seed=3, lookat=VIEW)
+    dm, dmot = torch.from_numpy(rtb200.materials_array(mats)).cuda(), torch.from_numpy(mot.astype(np.int32)).cuda()
+    alb = torch.rand(mot.shape[0], 3, device="cuda")
+    want = b.render(rc, dm, dmot, tri_albedo=alb)[0].cpu().numpy()
+    graph = torch.cuda.CUDAGraph()
+    with torch.cuda.graph(graph):
+        img = b.render(rc, dm, dmot, tri_albedo=alb)[0]
+    graph.replay()
+    assert np.array_equal(img.cpu().numpy(), want)
+    alb.mul_(0.5)
+    graph.replay()
+    torch.cuda.synchronize()
+    assert np.array_equal(img.cpu().numpy(), b.render(rc, dm, dmot, tri_albedo=alb)[0].cpu().numpy())
+
+
+def test_adjoint_does_not_depend_on_zero_pixels():
+    """Pixels with dLoss/dI = 0 are skipped: the gradients of the others are those of their paths alone."""
+    import torch
+    b, mats, mot = scene()
+    rc = rtb200.render_cfg(33, 21, 12, max_bounce=4, rr_after=2, env_kind=1, seed=5, lookat=VIEW)
+    d = torch.zeros(21, 33, 3, device="cuda")
+    d[:, ::3] = 1.0
+    rest = torch.ones_like(d) - d
+    one, two, full = (b.adjoint(rc, x, mats, mot) for x in (d, rest, torch.ones_like(d)))
+    for k in range(2):
+        total = (one[k].double() + two[k].double()).cpu().numpy()
+        ref = full[k].double().cpu().numpy()
+        # float sums of the same terms in other orders
+        assert np.linalg.norm(total - ref) <= 1e-4 * np.linalg.norm(ref)
+
+
+def test_short_albedo_table():
+    """A table with fewer rows than baked triangles: the missing rows are black."""
+    import torch
+    b, mats, mot = scene()
+    rc = rtb200.render_cfg(24, 16, 4, max_bounce=3, rr_after=-1, env_kind=1, seed=2, lookat=VIEW)
+    n = mot.shape[0]
+    full = torch.full((n, 3), 0.5)
+    full[n // 2:] = 0.0
+    a = b.render(rc, mats, mot, tri_albedo=full)[0]
+    c = b.render(rc, mats, mot, tri_albedo=full[:n // 2])[0]
+    assert torch.equal(a, c)
