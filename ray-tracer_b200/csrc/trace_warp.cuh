@@ -13,15 +13,16 @@
 // Every ray still sees the reference's nodes, leaves and triangles in the reference's order with the
 // same best distance at each test, so hits are the reference's bit for bit: a leaf's accepted
 // triangles reach their ray's lane in leaf order and pass the strict "t < best" there.
-// 2,097,152 incoherent rays, 1M-triangle soup: LBVH (leaf 16) 15.7 -> 6.8 ms, SAH (leaf 4)
-// 11.4 -> 6.2 ms; 1080p primary plus shadow rays, 1M triangles, hybrid tree: 3.07 -> 2.05 ms.
+// 2,097,152 incoherent rays, 1M-triangle soup: LBVH (leaf 16) 15.7 -> 6.5 ms, SAH (leaf 4)
+// 11.4 -> 6.0 ms; 1080p primary plus shadow rays, 1M triangles, hybrid tree: 3.07 -> 1.96 ms.
 //
-// The rest of the time goes to L1 (node and triangle fetches and the stacks, 58 % of its
-// wavefronts) at half of the issue slots. Hence the 8-byte stack entries (16 bytes: 8.2 ms on the
+// The rest of the time goes to L1 (node and triangle fetches, stacks: 55-73 % of its wavefronts)
+// and issue slots (50-70 %) with 17-21 lanes busy. Hence the 8-byte stack entries (16 bytes: 8.2 ms on the
 // SAH tree -- the stacks of an SM alone filled its L1), the top entry kept in registers, nodes
 // fetched with two 256-bit loads, and rays and hits kept in shared memory rather than in
-// registers (64 registers, four blocks of 256 threads per SM; 72 registers 5 % slower, 56 and
-// less spill inside the loop).
+// registers (64 registers, four blocks of 256 threads per SM; 80 registers 5-10 % slower). Slower too:
+// both planes of an axis in Blackwell's packed f32x2 arithmetic (2-5 %: six more registers), triangles
+// in pair records tested with it (3-8 %, and 30 % with a filter before the exact test).
 #pragma once
 
 #include "trace_core.cuh"
@@ -29,29 +30,10 @@
 namespace rtb
 {
 
-// two floats in one register pair (Blackwell's packed f32x2 arithmetic, rounded as the scalar one)
-using pair32 = unsigned long long;
-__device__ __forceinline__ pair32 pack2(float a, float b)
-{
-    pair32 r;
-    asm("mov.b64 %0, {%1, %2};" : "=l"(r) : "f"(a), "f"(b));
-    return r;
-}
-__device__ __forceinline__ void unpack2(pair32 r, float& a, float& b)
+// the halves of a 64-bit register pair
+__device__ __forceinline__ void unpack2(unsigned long long r, float& a, float& b)
 {
     asm("mov.b64 {%0, %1}, %2;" : "=f"(a), "=f"(b) : "l"(r));
-}
-__device__ __forceinline__ pair32 add2(pair32 a, pair32 b)
-{
-    pair32 r;
-    asm("add.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b));
-    return r;
-}
-__device__ __forceinline__ pair32 mul2(pair32 a, pair32 b)
-{
-    pair32 r;
-    asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b));
-    return r;
 }
 
 // 256-bit read-only load (p: 32-byte aligned)
@@ -79,8 +61,8 @@ struct WarpShare
 constexpr int WALK_MIN = 12;
 constexpr int REFILL = 16;
 // Leaves are tested lane by lane instead of pair by pair when the longest one would leave the warp
-// at least DIRECT_NUM / 32 busy (a pair costs about 1.3 times a lane's own test: its ray comes
-// from shared memory, its accepted hits go to another lane).
+// at least DIRECT_NUM / 32 busy: the ray is at hand and hits stay in the lane. (Rare: with it off,
+// nothing measured changes by more than 1 %.)
 constexpr uint32_t DIRECT_NUM = 24;
 constexpr uint32_t SHARE_MAX = 1u << 20;  // leaves above this are always tested lane by lane
 
@@ -90,7 +72,7 @@ constexpr uint32_t SHARE_MAX = 1u << 20;  // leaves above this are always tested
 template <int MODE, int STK>
 struct LaneTrace
 {
-    pair32   nx, ny, nz, ix, iy, iz;  // (-o, -o) and (1 / d, 1 / d) per axis
+    float    ox, oy, oz, ix, iy, iz;  // o and 1 / d
     float    tmin, best;
     uint32_t ref, cnt;                // the node or leaf the lane stands at
     uint32_t tref;                    // the top stack entry (stk[1 .. top - 1] holds those below)
@@ -117,8 +99,7 @@ struct LaneTrace
               tmin != tmin || best != best;
         ref = R.ref; cnt = R.cnt;
         live = ray_box(o, inv, tmin, best, R.box[0], R.box[1], R.box[2], R.box[3], R.box[4], R.box[5]) < best;
-        nx = pack2(-o.x, -o.x); ny = pack2(-o.y, -o.y); nz = pack2(-o.z, -o.z);
-        ix = pack2(inv.x, inv.x); iy = pack2(inv.y, inv.y); iz = pack2(inv.z, inv.z);
+        ox = o.x; oy = o.y; oz = o.z; ix = inv.x; iy = inv.y; iz = inv.z;
     }
 
     // The next stack entry whose entry distance is below best, or none. (All entries pass unless
@@ -167,20 +148,19 @@ struct LaneTrace
         }
         else
         {
-            // rayAABB (bvh_traverse.cpp:22-41) with both planes of an axis in one packed operation
-            float x0, x1, y0, y1, z0, z1;
-            unpack2(mul2(add2(A.x, nx), ix), x0, x1);
-            unpack2(mul2(add2(A.y, ny), iy), y0, y1);
-            unpack2(mul2(add2(A.z, nz), iz), z0, z1);
-            float tn = fmaxf(fmaxf(fmaxf(fminf(x0, x1), fminf(y0, y1)), fminf(z0, z1)), tmin);
-            float tf = fminf(fminf(fminf(fmaxf(x0, x1), fmaxf(y0, y1)), fmaxf(z0, z1)), best);
-            tl = tn <= tf ? tn : inf;
-            unpack2(mul2(add2(A.w, nx), ix), x0, x1);
-            unpack2(mul2(add2(B.x, ny), iy), y0, y1);
-            unpack2(mul2(add2(B.y, nz), iz), z0, z1);
-            tn = fmaxf(fmaxf(fmaxf(fminf(x0, x1), fminf(y0, y1)), fminf(z0, z1)), tmin);
-            tf = fminf(fminf(fminf(fmaxf(x0, x1), fmaxf(y0, y1)), fmaxf(z0, z1)), best);
-            tr = tn <= tf ? tn : inf;
+            // rayAABB (bvh_traverse.cpp:22-41)
+            auto slab = [&](unsigned long long bx, unsigned long long by, unsigned long long bz) {
+                float x0, x1, y0, y1, z0, z1;
+                unpack2(bx, x0, x1); unpack2(by, y0, y1); unpack2(bz, z0, z1);
+                x0 = (x0 - ox) * ix; x1 = (x1 - ox) * ix;
+                y0 = (y0 - oy) * iy; y1 = (y1 - oy) * iy;
+                z0 = (z0 - oz) * iz; z1 = (z1 - oz) * iz;
+                const float tn = fmaxf(fmaxf(fmaxf(fminf(x0, x1), fminf(y0, y1)), fminf(z0, z1)), tmin);
+                const float tf = fminf(fminf(fminf(fmaxf(x0, x1), fmaxf(y0, y1)), fmaxf(z0, z1)), best);
+                return tn <= tf ? tn : inf;
+            };
+            tl = slab(A.x, A.y, A.z);
+            tr = slab(A.w, B.x, B.y);
         }
         const bool left = tl <= tr;  // left first on ties
         const float nt = left ? tl : tr, ft = left ? tr : tl;
