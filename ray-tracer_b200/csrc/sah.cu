@@ -170,6 +170,11 @@ struct GlobalRefs
         b = mk3(verts[tr.v[1]].x, verts[tr.v[1]].y, verts[tr.v[1]].z);
         c = mk3(verts[tr.v[2]].x, verts[tr.v[2]].y, verts[tr.v[2]].z);
     }
+    __device__ __forceinline__ f3 vert(uint32_t i, int k) const
+    {
+        const rt_vertex& q = verts[tris[R[i]].v[k]];
+        return mk3(q.x, q.y, q.z);
+    }
 };
 
 // A warp's shared copy of at most EVAL_STAGE references: bounds with the x / y centroids in
@@ -213,6 +218,11 @@ struct StagedRefs
         a = mk3(v[0], v[1], v[2]);
         b = mk3(v[3], v[4], v[5]);
         c = mk3(v[6], v[7], v[8]);
+    }
+    __device__ __forceinline__ f3 vert(uint32_t i, int k) const
+    {
+        const float* v = S->v + 9 * i + 3 * k;
+        return mk3(v[0], v[1], v[2]);
     }
 };
 
@@ -277,6 +287,76 @@ __device__ __forceinline__ box3 sbox_result(const SBox& s)
     box3 b = box_empty();
     if (s.m[0] != 0xffffffffu) { b = sbox_get(s); }
     return b;
+}
+
+// ---- clipping by eight lanes ----
+// clip_triangle_general for up to four triangles of a warp at once, a vertex per lane: the clips that
+// clip_triangle_bin does not take (triangles that a spatial split above already cut on another axis).
+// Their polygons in a thread's indexed arrays cost 10-20 us a warp round, which set the time of the
+// deep levels of a mesh's subtrees: few nodes, all of whose references straddle.
+struct ClipSlots
+{
+    float v[4][8][3];
+};
+
+__device__ __noinline__ box3 clip_slow(f3 v0, f3 v1, f3 v2, box3 region) { return clip_triangle_general(v0, v1, v2, region); }
+
+// Lane 8 g + j holds vertex j of triangle g's polygon (n of them; n = 0: no triangle) and the triangle's
+// region; on return the clipped polygon's. False, in all lanes of a group, where it has more than eight
+// vertices or one that is not finite. All 32 lanes call it.
+__device__ __forceinline__ bool clip_group(f3& p, int& n, const box3& region, ClipSlots& S)
+{
+    constexpr unsigned FULL = 0xffffffffu;
+    const int lane = (int)(threadIdx.x & 31u), j = lane & 7, g8 = lane & 24;
+    const unsigned below = (1u << j) - 1u;
+    bool ok = true;
+#pragma unroll 1
+    for (int pl = 0; pl < 6; pl++)
+    {
+        const int axis = pl >> 1, side = pl & 1;
+        const float plane = side == 0 ? sel3(region.mn[0], region.mn[1], region.mn[2], axis)
+                                      : sel3(region.mx[0], region.mx[1], region.mx[2], axis);
+        const float c = get3(p, axis);
+        const bool valid = j < n, in = valid && (side == 0 ? c >= plane : c <= plane);
+        const unsigned ins = __ballot_sync(FULL, in);
+        if (ins == __ballot_sync(FULL, valid)) { continue; }  // the plane cuts nothing
+        const int nl = g8 | (j + 1 < n ? j + 1 : 0);
+        const f3 q = mk3(__shfl_sync(FULL, p.x, nl), __shfl_sync(FULL, p.y, nl), __shfl_sync(FULL, p.z, nl));
+        const bool cross = valid && in != (((ins >> nl) & 1u) != 0u);
+        const unsigned gi = (ins >> g8) & 255u, gx = (__ballot_sync(FULL, cross) >> g8) & 255u;
+        // a vertex inside goes out, then the crossing of its edge, in the polygon's order
+        int at = __popc(gi & below) + __popc(gx & below);
+        if (in && at < 8) { S.v[g8 >> 3][at][0] = p.x; S.v[g8 >> 3][at][1] = p.y; S.v[g8 >> 3][at][2] = p.z; }
+        at += in ? 1 : 0;
+        if (cross && at < 8)
+        {
+            const float t = (plane - c) / (get3(q, axis) - c);
+            const f3 r = add3(p, muls(sub3(q, p), t));
+            S.v[g8 >> 3][at][0] = r.x; S.v[g8 >> 3][at][1] = r.y; S.v[g8 >> 3][at][2] = r.z;
+        }
+        __syncwarp();
+        n = __popc(gi) + __popc(gx);
+        if (n > 8) { ok = false; n = 0; }
+        if (j < n) { p = mk3(S.v[g8 >> 3][j][0], S.v[g8 >> 3][j][1], S.v[g8 >> 3][j][2]); }
+        __syncwarp();
+    }
+    const float all = p.x + p.y + p.z;
+    const unsigned odd = __ballot_sync(FULL, j < n && !(all - all == 0.f));
+    return ok && ((odd >> g8) & 255u) == 0u;
+}
+
+// The lane of the (lane / 8)-th set bit of m, -1 if there are fewer; drops the four lowest bits of m.
+__device__ __forceinline__ int take_four(unsigned& m)
+{
+    const int g = (int)(threadIdx.x & 31u) >> 3;
+    unsigned q = m;
+#pragma unroll
+    for (int k = 0; k < 3; k++)
+    {
+        if (k < g) { q &= q - 1u; }
+    }
+    for (int k = 0; k < 4; k++) { m &= m - 1u; }
+    return q ? __ffs((int)q) - 1 : -1;
 }
 
 // Hoare-scheme partition of in[0, n) by pred into out[0, n) (in == out allowed). Returns the
@@ -464,6 +544,48 @@ __device__ __forceinline__ void bin_bounds(float* bnd, float node_min, float ssc
     for (int b = t; b <= nb; b += count) { bnd[b] = node_min + (float)b / sscale; }
 }
 
+// Whether a triangle with box tb lies inside the region, so that its clipped box is tb. cs: the sum of its
+// centroid's coordinates, not finite when a vertex is not (a box can miss a NaN vertex).
+__device__ __forceinline__ bool inside_region(const box3& tb, const box3& region, float cs)
+{
+    return cs - cs == 0.f && tb.mn[0] >= region.mn[0] && tb.mx[0] <= region.mx[0] && tb.mn[1] >= region.mn[1] &&
+           tb.mx[1] <= region.mx[1] && tb.mn[2] >= region.mn[2] && tb.mx[2] <= region.mx[2];
+}
+
+// Adds each lane's box to bins[b] and 1 to cnt[b] (b < 0: nothing; either array may be nullptr). The references
+// of a large node are in Morton order, so a warp's lanes mostly share a few bins: up to AGG_GROUPS
+// bins are reduced over their lanes first, since a shared atomic serialises over equal addresses (with
+// direct atomics alone the wide binning of 1M references takes 190-240 us a level). All 32 lanes call it.
+constexpr int AGG_GROUPS = 3;
+__device__ __forceinline__ void warp_bin_add(SBox* bins, uint32_t* cnt, int b, const box3& x)
+{
+    const int lane = (int)(threadIdx.x & 31u);
+    const unsigned peers = __match_any_sync(0xffffffffu, b);
+    const bool leader = __ffs((int)peers) - 1 == lane && b >= 0;
+    if (__popc(__ballot_sync(0xffffffffu, leader)) <= AGG_GROUPS)
+    {
+        if (b >= 0)
+        {
+            if (bins)
+            {
+#pragma unroll
+                for (int k = 0; k < 3; k++)
+                {
+                    const uint32_t m = __reduce_min_sync(peers, f2ord(x.mn[k])), M = __reduce_max_sync(peers, f2ord(x.mx[k]));
+                    if (leader) { atomicMin(&bins[b].m[k], m); atomicMax(&bins[b].M[k], M); }
+                }
+            }
+            if (cnt && leader) { atomicAdd(&cnt[b], (uint32_t)__popc(peers)); }
+        }
+    }
+    else if (b >= 0)
+    {
+        if (bins) { sbox_add(bins[b], x); }
+        if (cnt) { atomicAdd(&cnt[b], 1u); }
+    }
+    __syncwarp();
+}
+
 // Spatial binning of references R[i0 + lane] (i0 + lane < n) along `axis` by one whole warp:
 // entry / exit counts, then every (triangle, bin) pair of the 32 references clipped and added to
 // its bin -- the pairs spread evenly over the lanes (a warp-wide scan of each reference's bin
@@ -474,7 +596,7 @@ __device__ __forceinline__ void bin_bounds(float* bnd, float node_min, float ssc
 template <class Src>
 __device__ __forceinline__ void spatial_bin_warp(const Src& src, uint32_t i0, uint32_t n, int axis, const box3& nbox,
                                                  float node_min, float sscale, int nb, const float* bnd, uint32_t* cin,
-                                                 uint32_t* cout, SBox* bins, bool count = true)
+                                                 uint32_t* cout, SBox* bins, ClipSlots& slots, bool count = true)
 {
     const int lane = threadIdx.x & 31;
     const uint32_t i = i0 + (uint32_t)lane;
@@ -490,7 +612,19 @@ __device__ __forceinline__ void spatial_bin_warp(const Src& src, uint32_t i0, ui
             atomicAdd(&cout[bmax], 1u);
         }
     }
-    const uint32_t c = bmin <= bmax ? (uint32_t)(bmax - bmin + 1) : 0u;
+    uint32_t c = bmin <= bmax ? (uint32_t)(bmax - bmin + 1) : 0u;
+    if (c == 1u)
+    {
+        // a triangle inside its one bin: its own box
+        const box3 tb = src.box(i);
+        box3 region = nbox;
+#pragma unroll
+        for (int k = 0; k < 3; k++)
+        {
+            if (k == axis) { region.mn[k] = bnd[bmin]; region.mx[k] = bnd[bmin + 1]; }
+        }
+        if (inside_region(tb, region, src.cen(i, 0) + src.cen(i, 1) + src.cen(i, 2))) { sbox_add(bins[bmin], tb); c = 0u; }
+    }
     const uint32_t incl = warp_incl_scan(c);
     const uint32_t total = __shfl_sync(0xffffffffu, incl, 31);
     for (uint32_t j0 = 0; j0 < total; j0 += 32)
@@ -505,21 +639,50 @@ __device__ __forceinline__ void spatial_bin_warp(const Src& src, uint32_t i0, ui
         const uint32_t to = i0 + (uint32_t)o;
         const int bo = __shfl_sync(0xffffffffu, bmin, o);
         const uint32_t eo = __shfl_sync(0xffffffffu, incl - c, o);
+        const int b = bo + (int)(j - eo);
+        box3 region = nbox;
+        bool rest = false;  // clip_triangle_bin does not take this pair
         if (j < total)
         {
-            const int b = bo + (int)(j - eo);
             f3 v0, v1, v2;
             src.tri_verts(to, v0, v1, v2);
-            const float lo_b = bnd[b], hi_b = bnd[b + 1];
-            box3 region;
 #pragma unroll
             for (int k = 0; k < 3; k++)
             {
-                region.mn[k] = k == axis ? lo_b : nbox.mn[k];
-                region.mx[k] = k == axis ? hi_b : nbox.mx[k];
+                region.mn[k] = k == axis ? bnd[b] : nbox.mn[k];
+                region.mx[k] = k == axis ? bnd[b + 1] : nbox.mx[k];
             }
-            const box3 cl = clip_triangle(v0, v1, v2, region);
-            if (box_valid(cl)) { sbox_add(bins[b], cl); }
+            box3 cl;
+            rest = !clip_triangle_bin(v0, v1, v2, axis, region, cl);
+            if (!rest && box_valid(cl)) { sbox_add(bins[b], cl); }
+        }
+        for (unsigned m = __ballot_sync(0xffffffffu, rest); m;)
+        {
+            const int sl = take_four(m);
+            const uint32_t tg = __shfl_sync(0xffffffffu, to, sl & 31);
+            const int bg = __shfl_sync(0xffffffffu, b, sl & 31);
+            f3 p = mk3(0.f, 0.f, 0.f);
+            int n = 0;
+            box3 rg = nbox;
+            if (sl >= 0)
+            {
+                n = 3;
+                if ((lane & 7) < 3) { p = src.vert(tg, lane & 7); }
+#pragma unroll
+                for (int k = 0; k < 3; k++)
+                {
+                    if (k == axis) { rg.mn[k] = bnd[bg]; rg.mx[k] = bnd[bg + 1]; }
+                }
+            }
+            const bool ok = clip_group(p, n, rg, slots);
+            if (ok) { if ((lane & 7) < n) { box3 c; for (int k = 0; k < 3; k++) { c.mn[k] = c.mx[k] = get3(p, k); } sbox_add(bins[bg], c); } }
+            else if ((lane & 7) == 0)
+            {
+                f3 v0, v1, v2;
+                src.tri_verts(tg, v0, v1, v2);
+                const box3 cl = clip_slow(v0, v1, v2, rg);
+                if (box_valid(cl)) { sbox_add(bins[bg], cl); }
+            }
         }
     }
 }
@@ -599,16 +762,23 @@ __device__ __forceinline__ bool warp_spatial_can_win(const uint32_t* cin, const 
 
 // Nodes with more references than this are evaluated and partitioned by many blocks (the
 // wide kernels below); nodes with at most WARP_MAX references are evaluated by one warp each
-// (k_sah_eval_warp); the rest by one block each.
-constexpr uint32_t WIDE_MIN = 16384;
+// (k_sah_eval_warp); the rest by one block each. A level of the 1M soup has 64 nodes of 16,384 references:
+// one block each left half of the chip idle. SAH leaf 4 bake with this / WIDE_CH = 16384 / 4096 15.1 ms,
+// 4096 / 4096 13.1, 2048 / 2048 12.4, 2048 / 1024 12.2, 1024 / 1024 12.3.
+constexpr uint32_t WIDE_MIN = 2048;
 constexpr uint32_t WARP_MAX = 512;
-constexpr int      EVAL_WPB = 8;  // warps (nodes) per block of k_sah_eval_warp
+constexpr int      EVAL_WPB = 7;  // warps (nodes) per block of k_sah_eval_warp (shared memory: 6.1 KB each)
 
 // The evaluation of k_sah_eval below for one small node per warp: the same candidates, bins
 // and serial sweeps (lane 0), with warp reductions in place of block ones.
 struct EvalWS
 {
-    uint32_t cnt[SAH_MAX_BINS], cin[SAH_MAX_BINS], cout[SAH_MAX_BINS];
+    union
+    {
+        uint32_t  cnt[SAH_MAX_BINS];  // object splits
+        ClipSlots slots;              // spatial splits
+    };
+    uint32_t cin[SAH_MAX_BINS], cout[SAH_MAX_BINS];
     SBox     bins[SAH_MAX_BINS];
     float    bnd[SAH_MAX_BINS + 1];
 };
@@ -679,7 +849,7 @@ __device__ __forceinline__ void eval_node_warp(const Src& src, const LvlNode& nd
         }
         for (uint32_t i0 = 0; i0 < n; i0 += 32)
         {
-            spatial_bin_warp(src, i0, n, axis, nbox, node_min, sscale, nb, S.bnd, S.cin, S.cout, S.bins, !prune);
+            spatial_bin_warp(src, i0, n, axis, nbox, node_min, sscale, nb, S.bnd, S.cin, S.cout, S.bins, S.slots, !prune);
         }
         __syncwarp();
         warp_eval_spatial_axis(S.cin, S.cout, S.bins, nb, axis, node_min, sscale, parent_inv_area, C, Bw);
@@ -789,6 +959,7 @@ k_sah_eval(const LvlNode* __restrict__ lv, const uint32_t* __restrict__ refs, Ct
     __shared__ uint32_t cnt[SAH_MAX_BINS], cin[SAH_MAX_BINS], cout[SAH_MAX_BINS];
     __shared__ SBox bins[SAH_MAX_BINS];
     __shared__ float bnd[SAH_MAX_BINS + 1];
+    __shared__ ClipSlots slots[SBLK / 32];
     __shared__ uint32_t s_red[SBLK / 32 + 1];
     __shared__ uint32_t s_cm, s_cM;
     __shared__ Best sB;
@@ -888,7 +1059,7 @@ k_sah_eval(const LvlNode* __restrict__ lv, const uint32_t* __restrict__ refs, Ct
         }
         for (uint32_t i0 = (uint32_t)(tid & ~31); i0 < n; i0 += SBLK)
         {
-            spatial_bin_warp(GlobalRefs(C, R), i0, n, axis, nbox, node_min, sscale, nb, bnd, cin, cout, bins, !prune);
+            spatial_bin_warp(GlobalRefs(C, R), i0, n, axis, nbox, node_min, sscale, nb, bnd, cin, cout, bins, slots[threadIdx.x >> 5], !prune);
         }
         __syncthreads();
         if (tid < 32)
@@ -962,7 +1133,7 @@ k_sah_eval(const LvlNode* __restrict__ lv, const uint32_t* __restrict__ refs, Ct
 // encoding, which are the same values the one-block path accumulates in shared memory -- and
 // then evaluated by one thread per node with the same serial code, so the decisions are the
 // ones the one-block path makes.
-constexpr uint32_t WIDE_CH = 4096;
+constexpr uint32_t WIDE_CH = 1024;
 
 struct WideAcc
 {
@@ -1137,39 +1308,49 @@ k_wide_bins(const LvlNode* __restrict__ lv, const uint32_t* __restrict__ refs, C
         if (sscale[a] != 0.f) { bin_bounds(bnd[a], node_min[a], sscale[a], nb, threadIdx.x, SBLK); }
     }
     __syncthreads();
-    for (uint32_t i = b0 + threadIdx.x; i < e0; i += SBLK)
+    for (uint32_t i0 = b0 + (threadIdx.x & ~31u); i0 < e0; i0 += SBLK)
     {
-        const uint32_t t = R[i];
-        const box3 tb = tri_box(C, t);
-        for (int a = 0; a < 3; a++)
-        {
-            if (scale[a] == 0.f) { continue; }
-            const int b = obj_bin(centroid(C, t, a), cmin[a], scale[a], nb);
-            atomicAdd(&ocnt[a][b], 1u);
-            sbox_add(obox[a][b], tb);
-        }
+        const uint32_t i = i0 + (threadIdx.x & 31u);
+        const bool have = i < e0;
+        const uint32_t t = have ? R[i] : 0u;
+        const float4 lo4 = have ? C.lo[t] : make_float4(0.f, 0.f, 0.f, 0.f), hi4 = have ? C.hi[t] : lo4;
+        const float cen[3] = { lo4.w, hi4.w, have ? C.cz[t] : 0.f };
+        box3 tb;
+        tb.mn[0] = lo4.x; tb.mn[1] = lo4.y; tb.mn[2] = lo4.z; tb.mx[0] = hi4.x; tb.mx[1] = hi4.y; tb.mx[2] = hi4.z;
+        const float top = (float)(nb - 1), cs = cen[0] + cen[1] + cen[2];
         f3 v0, v1, v2;
         bool have_v = false;
-        const float top = (float)(nb - 1);
+#pragma unroll
         for (int a = 0; a < 3; a++)
         {
+            if (scale[a] != 0.f) { warp_bin_add(obox[a], ocnt[a], have ? obj_bin(cen[a], cmin[a], scale[a], nb) : -1, tb); }
             if (sscale[a] == 0.f) { continue; }
-            const int bmin = bin_clamp((tri_lo(C, t, a) - node_min[a]) * sscale[a], top);
-            const int bmax = bin_clamp((tri_hi(C, t, a) - node_min[a]) * sscale[a], top);
-            atomicAdd(&cin[a][bmin], 1u);
-            atomicAdd(&cout[a][bmax], 1u);
-            if (bmin <= bmax)
+            const int bmin = have ? bin_clamp((tb.mn[a] - node_min[a]) * sscale[a], top) : -1;
+            const int bmax = have ? bin_clamp((tb.mx[a] - node_min[a]) * sscale[a], top) : -1;
+            box3 region = nbox;
+            bool own = have && bmin == bmax;  // a triangle inside its one bin: its own box
+            if (own)
+            {
+                region.mn[a] = bnd[a][bmin];
+                region.mx[a] = bnd[a][bmin + 1];
+                own = inside_region(tb, region, cs);
+            }
+            warp_bin_add(nullptr, cin[a], bmin, tb);
+            warp_bin_add(nullptr, cout[a], bmax, tb);
+            warp_bin_add(sbx[a], nullptr, own ? bmin : -1, tb);
+            if (have && !own && bmin <= bmax)
             {
                 if (!have_v) { tri_verts(C, t, v0, v1, v2); have_v = true; }
-                box3 region = nbox;
                 for (int b = bmin; b <= bmax; b++)
                 {
                     region.mn[a] = bnd[a][b];
                     region.mx[a] = bnd[a][b + 1];
-                    const box3 cl = clip_triangle(v0, v1, v2, region);
+                    box3 cl;
+                    if (!clip_triangle_bin(v0, v1, v2, a, region, cl)) { cl = clip_triangle(v0, v1, v2, region); }
                     if (box_valid(cl)) { sbox_add(sbx[a][b], cl); }
                 }
             }
+            __syncwarp();
         }
     }
     __syncthreads();
@@ -1785,6 +1966,7 @@ k_sah_split_warp(const LvlNode* __restrict__ lv, const uint32_t* __restrict__ re
                  uint32_t* __restrict__ refs_next, OutNode* __restrict__ out, uint32_t out_base, uint32_t leaf_base,
                  uint32_t* __restrict__ leaf_refs, uint32_t n_lvl)
 {
+    __shared__ ClipSlots s_slots[SPLIT_WPB];
     const int lane = threadIdx.x & 31;
     const uint32_t ni = blockIdx.x * SPLIT_WPB + (threadIdx.x >> 5);
     if (ni >= n_lvl) { return; }
@@ -1877,8 +2059,12 @@ k_sah_split_warp(const LvlNode* __restrict__ lv, const uint32_t* __restrict__ re
         const int ax = d.axis;
         box3 lclip, rclip;
         for (int k = 0; k < 3; k++) { lclip.mn[k] = rclip.mn[k] = nd.box[k]; lclip.mx[k] = rclip.mx[k] = nd.box[3 + k]; }
-        lclip.mx[ax] = d.plane;
-        rclip.mn[ax] = d.plane;
+#pragma unroll
+        for (int k = 0; k < 3; k++)
+        {
+            if (k == ax) { lclip.mx[k] = d.plane; rclip.mn[k] = d.plane; }
+        }
+        unsigned rest[2] = { 0u, 0u };  // bit 0 / 1: the left / right clip of w[h] is left
 #pragma unroll
         for (int h = 0; h < 2; h++)
         {
@@ -1890,15 +2076,57 @@ k_sah_split_warp(const LvlNode* __restrict__ lv, const uint32_t* __restrict__ re
                 if (straddles) { Q[n + p - left_end] = w[h]; }
                 f3 v0, v1, v2;
                 tri_verts(C, w[h], v0, v1, v2);
+                box3 cl;
                 if (p < straddle_end)
                 {
-                    const box3 cl = clip_triangle(v0, v1, v2, lclip);
-                    if (box_valid(cl)) { obox_add(ob[0], cl); }
+                    if (!clip_triangle_bin(v0, v1, v2, ax, lclip, cl)) { rest[h] |= 1u; }
+                    else if (box_valid(cl)) { obox_add(ob[0], cl); }
                 }
                 if (p >= straddle_end || straddles)
                 {
-                    const box3 cl = clip_triangle(v0, v1, v2, rclip);
-                    if (box_valid(cl)) { obox_add(ob[1], cl); }
+                    if (!clip_triangle_bin(v0, v1, v2, ax, rclip, cl)) { rest[h] |= 2u; }
+                    else if (box_valid(cl)) { obox_add(ob[1], cl); }
+                }
+            }
+        }
+        // the clips that are left, four at a time (clip_group)
+        ClipSlots& slots = s_slots[threadIdx.x >> 5];
+        for (int q = 0; q < 4; q++)
+        {
+            const int side = q & 1;
+            const unsigned left = q >> 1 ? rest[1] : rest[0];
+            const uint32_t wq = q >> 1 ? w[1] : w[0];
+            for (unsigned m = __ballot_sync(0xffffffffu, ((left >> side) & 1u) != 0u); m;)
+            {
+                const int sl = take_four(m);
+                const uint32_t t = __shfl_sync(0xffffffffu, wq, sl & 31);
+                f3 v = mk3(0.f, 0.f, 0.f);
+                int nv = 0;
+                const box3 region = side ? rclip : lclip;
+                if (sl >= 0)
+                {
+                    nv = 3;
+                    if ((lane & 7) < 3)
+                    {
+                        const rt_vertex& a = C.verts[C.tris[t].v[lane & 7]];
+                        v = mk3(a.x, a.y, a.z);
+                    }
+                }
+                if (clip_group(v, nv, region, slots))
+                {
+                    if ((lane & 7) < nv)
+                    {
+                        box3 c;
+                        for (int k = 0; k < 3; k++) { c.mn[k] = c.mx[k] = get3(v, k); }
+                        if (side) { obox_add(ob[1], c); } else { obox_add(ob[0], c); }
+                    }
+                }
+                else if ((lane & 7) == 0)
+                {
+                    f3 v0, v1, v2;
+                    tri_verts(C, t, v0, v1, v2);
+                    const box3 cl = clip_slow(v0, v1, v2, region);
+                    if (box_valid(cl)) { if (side) { obox_add(ob[1], cl); } else { obox_add(ob[0], cl); } }
                 }
             }
         }
@@ -1924,7 +2152,8 @@ k_sah_split_warp(const LvlNode* __restrict__ lv, const uint32_t* __restrict__ re
 // flags and satisfied counts; per chunk the failing elements left of the split point and the
 // satisfying ones right of it; their ranks from the chunk prefixes; the scatter, where the
 // k-th failing element from the left and the k-th satisfying one from the right trade places.
-// Each block owns WIDE_CH consecutive references, 16 per thread.
+// Each block owns WIDE_CH consecutive references, WP_ITEMS per thread.
+constexpr uint32_t WP_ITEMS = WIDE_CH / SBLK;
 struct WideSplit
 {
     const LvlNode*  lv;
@@ -1982,8 +2211,8 @@ __device__ __forceinline__ WpItem wp_item(const WideSplit& W)
     it.n = W.lv[it.node].count;
     it.c0 = c * WIDE_CH;
     it.c1 = min(it.n, it.c0 + WIDE_CH);
-    it.t0 = min(it.c1, it.c0 + threadIdx.x * 16u);
-    it.t1 = min(it.c1, it.t0 + 16u);
+    it.t0 = min(it.c1, it.c0 + threadIdx.x * WP_ITEMS);
+    it.t1 = min(it.c1, it.t0 + WP_ITEMS);
     return it;
 }
 
