@@ -226,10 +226,10 @@ struct StagedRefs
     }
 };
 
-// Copies references [0, n) of R (n <= EVAL_STAGE) into S, one warp.
-__device__ __forceinline__ void stage_refs(const Ctx& C, const uint32_t* R, uint32_t n, StageBuf& S)
+// Copies references [0, n) of R (n <= EVAL_STAGE) into S, by threads t of `count`.
+__device__ __forceinline__ void stage_refs(const Ctx& C, const uint32_t* R, uint32_t n, StageBuf& S, int t0, int count)
 {
-    for (uint32_t i = threadIdx.x & 31; i < n; i += 32)
+    for (uint32_t i = (uint32_t)t0; i < n; i += (uint32_t)count)
     {
         const uint32_t t = R[i];
         S.lo[i] = C.lo[t];
@@ -244,7 +244,6 @@ __device__ __forceinline__ void stage_refs(const Ctx& C, const uint32_t* R, uint
             v[3 * k] = q.x; v[3 * k + 1] = q.y; v[3 * k + 2] = q.z;
         }
     }
-    __syncwarp();
 }
 
 // Shared box accumulator in the order-preserving uint encoding.
@@ -769,8 +768,6 @@ constexpr uint32_t WIDE_MIN = 2048;
 constexpr uint32_t WARP_MAX = 512;
 constexpr int      EVAL_WPB = 7;  // warps (nodes) per block of k_sah_eval_warp (shared memory: 6.1 KB each)
 
-// The evaluation of k_sah_eval below for one small node per warp: the same candidates, bins
-// and serial sweeps (lane 0), with warp reductions in place of block ones.
 struct EvalWS
 {
     union
@@ -783,19 +780,17 @@ struct EvalWS
     float    bnd[SAH_MAX_BINS + 1];
 };
 
+// Evaluation of one small node by a warp: the candidates, bins and serial sweeps of k_sah_eval below,
+// with warp reductions in place of block ones, in three parts.
+
+// Phase 1: the best centroid-binned object split (bvh_sah.cpp:52-126), identical in every lane.
 template <class Src>
-__device__ __forceinline__ void eval_node_warp(const Src& src, const LvlNode& nd, uint32_t n, const Ctx& C, EvalWS& S,
-                                               Dec& d)
+__device__ __forceinline__ Best eval_object_warp(const Src& src, uint32_t n, int nb, float parent_inv_area, const Ctx& C, EvalWS& S)
 {
     const int lane = threadIdx.x & 31;
-    const int nb = std_clampi((int)n / 4, (int)C.bins_min, (int)C.bins_max);
-    box3 nbox;
-    for (int k = 0; k < 3; k++) { nbox.mn[k] = nd.box[k]; nbox.mx[k] = nd.box[3 + k]; }
-    const float parent_inv_area = 1.0f / box_half_area(nbox);
-    Best Bw;  // identical in every lane
+    Best Bw;
     Bw.cost = C.c_isect * (float)n;  // leaf cost, bvh_sah.cpp:32
     Bw.axis = -1; Bw.bin = -1; Bw.cmin = 0.f; Bw.scale = 0.f; Bw.spatial = 0; Bw.node_min = 0.f; Bw.sscale = 0.f;
-    // phase 1: centroid-binned object split (bvh_sah.cpp:52-126)
     for (int axis = 0; axis < 3; axis++)
     {
         uint32_t m = 0xffffffffu, M = 0u;
@@ -822,14 +817,24 @@ __device__ __forceinline__ void eval_node_warp(const Src& src, const LvlNode& nd
         warp_eval_object_axis(S.cnt, S.bins, nb, axis, cmin, scale, parent_inv_area, C, Bw);
         __syncwarp();
     }
-    const int oa = Bw.axis, ob = Bw.bin;
-    const float oc = Bw.cmin, os = Bw.scale;
-    // phase 2: spatial bins over the node box, triangles clipped per bin (bvh_sah.cpp:135-243)
+    return Bw;
+}
+
+// Phase 2: spatial bins over the node box, triangles clipped per bin (bvh_sah.cpp:135-243), on the axes
+// whose bound can beat the best so far. DEFER: only finds those axes (their mask is returned), with the
+// object split as the best.
+template <bool DEFER, class Src>
+__device__ __forceinline__ uint32_t eval_spatial_warp(const Src& src, uint32_t n, int nb, const box3& nbox, float parent_inv_area,
+                                                      const Ctx& C, EvalWS& S, Best& Bw)
+{
+    const int lane = threadIdx.x & 31;
     const bool prune = C.c_isect >= 0.f;  // (the bound needs a cost monotone in the areas)
+    uint32_t mask = 0;
     for (int axis = 0; axis < 3; axis++)
     {
         const float node_min = nbox.mn[axis], node_max = nbox.mx[axis];
         if (node_max - node_min < C.spatial_eps) { continue; }
+        if (DEFER && !prune) { mask |= 1u << axis; continue; }
         const float sscale = (float)nb / (node_max - node_min);
         for (int b = lane; b < nb; b += 32) { S.cin[b] = 0u; S.cout[b] = 0u; sbox_clear(S.bins[b]); }
         bin_bounds(S.bnd, node_min, sscale, nb, lane, 32);
@@ -844,19 +849,31 @@ __device__ __forceinline__ void eval_node_warp(const Src& src, const LvlNode& nd
             const bool can = warp_spatial_can_win(S.cin, S.cout, S.bins, nb, parent_inv_area, C, Bw.cost);
             __syncwarp();
             if (!can) { continue; }
+            if (DEFER) { mask |= 1u << axis; continue; }
             for (int b = lane; b < nb; b += 32) { sbox_clear(S.bins[b]); }  // the exact boxes; the counts stay
             __syncwarp();
         }
-        for (uint32_t i0 = 0; i0 < n; i0 += 32)
+        if constexpr (!DEFER)
         {
-            spatial_bin_warp(src, i0, n, axis, nbox, node_min, sscale, nb, S.bnd, S.cin, S.cout, S.bins, S.slots, !prune);
+            for (uint32_t i0 = 0; i0 < n; i0 += 32)
+            {
+                spatial_bin_warp(src, i0, n, axis, nbox, node_min, sscale, nb, S.bnd, S.cin, S.cout, S.bins, S.slots, !prune);
+            }
+            __syncwarp();
+            warp_eval_spatial_axis(S.cin, S.cout, S.bins, nb, axis, node_min, sscale, parent_inv_area, C, Bw);
+            __syncwarp();
         }
-        __syncwarp();
-        warp_eval_spatial_axis(S.cin, S.cout, S.bins, nb, axis, node_min, sscale, parent_inv_area, C, Bw);
-        __syncwarp();
     }
-    // decision and partition side counts (bvh_sah.cpp:249-394)
-    const Best B = Bw;
+    return mask;
+}
+
+// Decision and partition side counts (bvh_sah.cpp:249-394): B the best candidate, O the best object split.
+template <class Src>
+__device__ __forceinline__ void decide_warp(const Src& src, uint32_t n, int nb, const Best& B, const Best& O, Dec& d)
+{
+    const int lane = threadIdx.x & 31;
+    const int oa = O.axis, ob = O.bin;
+    const float oc = O.cmin, os = O.scale;
     d.nb = nb;
     d.oaxis = oa; d.obin = ob; d.ocmin = oc; d.oscale = os;
     if (B.axis == -1)
@@ -906,15 +923,24 @@ __device__ __forceinline__ void eval_node_warp(const Src& src, const LvlNode& nd
     }
 }
 
+// What k_sah_eval_warp<true> leaves for k_sah_eval_clip: a node with axes to clip.
+struct ClipJob
+{
+    uint32_t node, mask;  // bit a: axis a
+    Best     object;      // its best object split
+};
+
 // STAGED: the nodes of at most EVAL_STAGE references (leaves included), read from a shared
 // copy; else the nodes of EVAL_STAGE + 1 .. WARP_MAX references, read from global memory.
-// Each warp takes the level's nodes one at a time from a counter (*ctr, zero at launch), so a
+// Each warp takes the level's nodes one at a time from a counter (io[13 / 14], zero at launch), so a
 // warp that meets leaves or another kernel's nodes moves on at once and the grid need only
-// fill the GPU.
+// fill the GPU. STAGED leaves nodes with axes to clip (one in ten of a mesh's) to k_sah_eval_clip
+// (jobs, their count in io[16]): a warp took up to 280 us for such a node, which was the time of the
+// level, and without the clip its code fits the instruction cache.
 template <bool STAGED>
 __global__ void __launch_bounds__(EVAL_WPB * 32, 4)  // (64 registers: occupancy over spills)
 k_sah_eval_warp(const LvlNode* __restrict__ lv, const uint32_t* __restrict__ refs, Ctx C, Dec* __restrict__ dec,
-                uint32_t n_lvl, uint32_t* __restrict__ ctr)
+                uint32_t n_lvl, uint32_t* __restrict__ io, ClipJob* __restrict__ jobs)
 {
     __shared__ EvalWS ws[EVAL_WPB];
     __shared__ StageBuf stage[STAGED ? EVAL_WPB : 1];
@@ -922,7 +948,7 @@ k_sah_eval_warp(const LvlNode* __restrict__ lv, const uint32_t* __restrict__ ref
     for (;;)
     {
         uint32_t node = 0;
-        if (lane == 0) { node = atomicAdd(ctr, 1u); }
+        if (lane == 0) { node = atomicAdd(&io[STAGED ? 13 : 14], 1u); }
         node = __shfl_sync(0xffffffffu, node, 0);
         if (node >= n_lvl) { return; }
         const LvlNode nd = lv[node];
@@ -937,17 +963,178 @@ k_sah_eval_warp(const LvlNode* __restrict__ lv, const uint32_t* __restrict__ ref
             if (lane == 0) { d.kind = K_LEAF; dec[node] = d; }
             continue;
         }
+        const int nb = std_clampi((int)n / 4, (int)C.bins_min, (int)C.bins_max);
+        box3 nbox;
+        for (int k = 0; k < 3; k++) { nbox.mn[k] = nd.box[k]; nbox.mx[k] = nd.box[3 + k]; }
+        const float parent_inv_area = 1.0f / box_half_area(nbox);
         if constexpr (STAGED)
         {
-            stage_refs(C, R, n, stage[w]);
-            eval_node_warp(StagedRefs{ &stage[w], R }, nd, n, C, ws[w], d);
+            stage_refs(C, R, n, stage[w], (int)(threadIdx.x & 31), 32);
+            __syncwarp();
+            const StagedRefs src{ &stage[w], R };
+            Best B = eval_object_warp(src, n, nb, parent_inv_area, C, ws[w]);
+            const uint32_t mask = eval_spatial_warp<true>(src, n, nb, nbox, parent_inv_area, C, ws[w], B);
+            if (mask)
+            {
+                if (lane == 0)
+                {
+                    ClipJob j;
+                    j.node = node; j.mask = mask; j.object = B;
+                    jobs[atomicAdd(&io[16], 1u)] = j;
+                }
+                __syncwarp();
+                continue;
+            }
+            decide_warp(src, n, nb, B, B, d);
         }
         else
         {
-            eval_node_warp(GlobalRefs(C, R), nd, n, C, ws[w], d);
+            const GlobalRefs src(C, R);
+            const Best O = eval_object_warp(src, n, nb, parent_inv_area, C, ws[w]);
+            Best B = O;
+            eval_spatial_warp<false>(src, n, nb, nbox, parent_inv_area, C, ws[w], B);
+            decide_warp(src, n, nb, B, O, d);
         }
         if (lane == 0) { dec[node] = d; }
         __syncwarp();  // every lane done with the shared copy and bins before the next node
+    }
+}
+
+// The spatial splits of one deferred node per block of G warps: the (axis, reference, bin) triples spread
+// over the block, what clip_triangle_bin does not take queued and clipped by eight lanes each, then a
+// warp per axis sweeps its candidates. The axes' best candidates are compared in the reference's order
+// with the strict comparison, so the decision is the serial one's. G = 12 for levels of few nodes, where
+// a node's own time counts; G = 4 where nodes fill the chip.
+struct AxisWS
+{
+    uint32_t cin[SAH_MAX_BINS], cout[SAH_MAX_BINS];
+    SBox     bins[SAH_MAX_BINS];
+    float    bnd[SAH_MAX_BINS + 1];
+    float    node_min, sscale;
+    Best     best;
+};
+template <int G>
+__global__ void __launch_bounds__(G * 32)
+k_sah_eval_clip(const LvlNode* __restrict__ lv, const uint32_t* __restrict__ refs, Ctx C, Dec* __restrict__ dec,
+                uint32_t* __restrict__ io, const ClipJob* __restrict__ jobs)
+{
+    __shared__ StageBuf stage;
+    __shared__ AxisWS ax[3];
+    __shared__ ClipSlots slots[G];
+    __shared__ uint16_t queue[3 * EVAL_STAGE * SAH_MAX_BINS];
+    __shared__ uint32_t s_job, s_queued;
+    const int tid = threadIdx.x, w = tid >> 5, lane = tid & 31;
+    for (;;)
+    {
+        __syncthreads();
+        if (tid == 0) { s_job = atomicAdd(&io[17], 1u); s_queued = 0u; }
+        __syncthreads();
+        if (s_job >= io[16]) { return; }
+        const ClipJob job = jobs[s_job];
+        const LvlNode nd = lv[job.node];
+        const uint32_t n = nd.count;
+        const uint32_t* R = refs + nd.ref_off;
+        const int nb = std_clampi((int)n / 4, (int)C.bins_min, (int)C.bins_max);
+        box3 nbox;
+        for (int k = 0; k < 3; k++) { nbox.mn[k] = nd.box[k]; nbox.mx[k] = nd.box[3 + k]; }
+        const float parent_inv_area = 1.0f / box_half_area(nbox);
+        stage_refs(C, R, n, stage, tid, G * 32);
+        const StagedRefs src{ &stage, R };
+        for (int a = 0; a < 3; a++)
+        {
+            if (!((job.mask >> a) & 1u)) { continue; }
+            AxisWS& A = ax[a];
+            const float sscale = (float)nb / (nbox.mx[a] - nbox.mn[a]);
+            for (int b = tid; b < nb; b += G * 32) { A.cin[b] = 0u; A.cout[b] = 0u; sbox_clear(A.bins[b]); }
+            bin_bounds(A.bnd, nbox.mn[a], sscale, nb, tid, G * 32);
+            if (tid == 0) { A.node_min = nbox.mn[a]; A.sscale = sscale; }
+        }
+        __syncthreads();
+        const float top = (float)(nb - 1);
+        const uint32_t per_axis = n * (uint32_t)nb;
+        for (uint32_t item = (uint32_t)tid; item < 3u * per_axis; item += G * 32)
+        {
+            const uint32_t a = item / per_axis, q = item - a * per_axis, i = q / (uint32_t)nb;
+            const int b = (int)(q - i * (uint32_t)nb), axis = (int)a;
+            if (!((job.mask >> a) & 1u)) { continue; }
+            AxisWS& A = ax[a];
+            const int bmin = bin_clamp((src.lo_of(i, axis) - A.node_min) * A.sscale, top);
+            const int bmax = bin_clamp((src.hi_of(i, axis) - A.node_min) * A.sscale, top);
+            if (b == bmin) { atomicAdd(&A.cin[b], 1u); }
+            if (b == bmax) { atomicAdd(&A.cout[b], 1u); }
+            if (b < bmin || b > bmax) { continue; }
+            box3 region = nbox;
+#pragma unroll
+            for (int k = 0; k < 3; k++)
+            {
+                if (k == axis) { region.mn[k] = A.bnd[b]; region.mx[k] = A.bnd[b + 1]; }
+            }
+            f3 v0, v1, v2;
+            src.tri_verts(i, v0, v1, v2);
+            box3 cl;
+            if (!clip_triangle_bin(v0, v1, v2, axis, region, cl)) { queue[atomicAdd(&s_queued, 1u)] = (uint16_t)((a * EVAL_STAGE + i) * SAH_MAX_BINS + b); }
+            else if (box_valid(cl)) { sbox_add(A.bins[b], cl); }
+        }
+        __syncthreads();
+        const uint32_t queued = s_queued;
+        for (uint32_t q0 = (uint32_t)w * 4u; q0 < queued; q0 += G * 4u)
+        {
+            const uint32_t q = q0 + (uint32_t)(lane >> 3);
+            const bool have = q < queued;
+            const uint32_t id = have ? queue[q] : 0u;
+            const int b = (int)(id % SAH_MAX_BINS), axis = (int)(id / (SAH_MAX_BINS * EVAL_STAGE));
+            const uint32_t i = id / SAH_MAX_BINS % EVAL_STAGE;
+            box3 region = nbox;
+            f3 p = mk3(0.f, 0.f, 0.f);
+            int nv = 0;
+            if (have)
+            {
+#pragma unroll
+                for (int k = 0; k < 3; k++)
+                {
+                    if (k == axis) { region.mn[k] = ax[axis].bnd[b]; region.mx[k] = ax[axis].bnd[b + 1]; }
+                }
+                nv = 3;
+                if ((lane & 7) < 3) { p = src.vert(i, lane & 7); }
+            }
+            if (clip_group(p, nv, region, slots[w]))
+            {
+                if ((lane & 7) < nv)
+                {
+                    box3 c;
+                    for (int k = 0; k < 3; k++) { c.mn[k] = c.mx[k] = get3(p, k); }
+                    sbox_add(ax[axis].bins[b], c);
+                }
+            }
+            else if ((lane & 7) == 0)
+            {
+                f3 v0, v1, v2;
+                src.tri_verts(i, v0, v1, v2);
+                const box3 cl = clip_slow(v0, v1, v2, region);
+                if (box_valid(cl)) { sbox_add(ax[axis].bins[b], cl); }
+            }
+        }
+        __syncthreads();
+        if (w < 3 && ((job.mask >> w) & 1u))
+        {
+            Best B = job.object;
+            warp_eval_spatial_axis(ax[w].cin, ax[w].cout, ax[w].bins, nb, w, ax[w].node_min, ax[w].sscale, parent_inv_area, C, B);
+            if (lane == 0) { ax[w].best = B; }
+        }
+        __syncthreads();
+        if (w == 0)
+        {
+            Best B = job.object;
+            for (int a = 0; a < 3; a++)
+            {
+                if (((job.mask >> a) & 1u) && ax[a].best.cost < B.cost) { B = ax[a].best; }
+            }
+            Dec d;
+            memset(&d, 0, sizeof(d));
+            d.n = n;
+            decide_warp(src, n, nb, B, job.object, d);
+            if (lane == 0) { dec[job.node] = d; }
+        }
     }
 }
 
@@ -1643,7 +1830,7 @@ k_sah_grant(Dec* __restrict__ dec, const LvlNode* __restrict__ lv, const SahRoot
     __syncthreads();
     for (uint32_t k = tid; k < n_scenes; k += 1024) { need[k] = 0ull; }
     for (uint32_t k = tid; k <= 3 * n_tiles; k += 1024) { desc[k] = 0ull; }
-    if (tid == 0) { io[10] = 0u; io[11] = 0u; io[13] = 0u; io[14] = 0u; io[15] = 0xffffffffu; }
+    if (tid == 0) { io[10] = 0u; io[11] = 0u; io[13] = 0u; io[14] = 0u; io[15] = 0xffffffffu; io[16] = 0u; io[17] = 0u; }
 }
 
 // Child slots, reference offsets and leaf offsets of a level: three exclusive scans in one pass
@@ -2632,6 +2819,9 @@ k_sah_emit(const OutNode* __restrict__ out, uint32_t n_out, const SahRoot* __res
     }
 }
 
+// Levels of at most this many nodes per SM clip with 12 warps a node.
+constexpr uint32_t CLIP_FEW = 32;
+
 inline uint32_t nblk(uint64_t n) { return (uint32_t)((n + SBLK - 1) / SBLK); }
 
 } // namespace
@@ -2647,7 +2837,7 @@ int sah_build(rt_bvh* B, const rt_build_cfg& cfg, const SahInput& in, cudaStream
         S.sah_refs_a.ensure((size_t)cap * 4) || S.sah_refs_b.ensure((size_t)cap * 4) || S.sah_tmp.ensure((size_t)cap * 4) ||
         S.sah_pos.ensure((size_t)cap * 4) || S.sah_scan_in.ensure((size_t)cap) || S.sah_dec.ensure((size_t)cap * sizeof(Dec)) ||
         S.sah_out.ensure((size_t)2 * cap * sizeof(OutNode)) || S.sah_leaf_refs.ensure((size_t)cap * 4) ||
-        S.sah_scan_out.ensure((size_t)3 * cap * 4 + (size_t)2 * nr * 4 + 64))
+        S.sah_scan_out.ensure((size_t)3 * cap * 4 + (size_t)2 * nr * 4 + 80) || S.sah_jobs.ensure((size_t)cap * sizeof(ClipJob)))
     {
         return RT_E_CUDA;
     }
@@ -2714,8 +2904,8 @@ int sah_build(rt_bvh* B, const rt_build_cfg& cfg, const SahInput& in, cudaStream
     uint32_t* root_out = leaf_offs + cap;
     uint32_t* new_off = root_out + nr;
     uint32_t* io = new_off + nr;
-    uint32_t io_h[16] = { in.n, 0, 0, 0, 0, 0, 0, 0, 0, 0, 0, 0, 0, 0, 0, 0xffffffffu };
-    RT_CUDA(cudaMemcpyAsync(io, io_h, 64, cudaMemcpyHostToDevice, st));
+    uint32_t io_h[20] = { in.n, 0, 0, 0, 0, 0, 0, 0, 0, 0, 0, 0, 0, 0, 0, 0xffffffffu };
+    RT_CUDA(cudaMemcpyAsync(io, io_h, 80, cudaMemcpyHostToDevice, st));
     // wide-node scratch: at most cap / WIDE_MIN nodes of a level have more than WIDE_MIN references
     const uint32_t max_wide = cap / WIDE_MIN + 2;
     const uint32_t max_chunks = cap / WIDE_CH + max_wide + 1;
@@ -2817,12 +3007,18 @@ int sah_build(rt_bvh* B, const rt_build_cfg& cfg, const SahInput& in, cudaStream
             if (nw > max_wide) { return fail(RT_E_CAPACITY, "SAH builder: too many wide nodes"); }
         }
         const uint32_t eval_blocks = std::min<uint32_t>((n_cur + EVAL_WPB - 1) / EVAL_WPB, 8u * (uint32_t)device_sm_count());
-        k_sah_eval_warp<true><<<eval_blocks, EVAL_WPB * 32, 0, st>>>(lv_cur, refs_cur, C, S.sah_dec.as<Dec>(), n_cur, io + 13);
-        count_launch();
+        const uint32_t sms = (uint32_t)device_sm_count();
+        ClipJob* jobs = S.sah_jobs.as<ClipJob>();
+        k_sah_eval_warp<true><<<eval_blocks, EVAL_WPB * 32, 0, st>>>(lv_cur, refs_cur, C, S.sah_dec.as<Dec>(), n_cur, io, jobs);
+        if (n_cur <= CLIP_FEW * sms)
+        {
+            k_sah_eval_clip<12><<<std::min(n_cur, 2u * sms), 12 * 32, 0, st>>>(lv_cur, refs_cur, C, S.sah_dec.as<Dec>(), io, jobs);
+        }
+        else { k_sah_eval_clip<4><<<std::min(n_cur, 8u * sms), 4 * 32, 0, st>>>(lv_cur, refs_cur, C, S.sah_dec.as<Dec>(), io, jobs); }
+        count_launch(2);
         if (next_bound > EVAL_STAGE)
         {
-            k_sah_eval_warp<false><<<eval_blocks, EVAL_WPB * 32, 0, st>>>(lv_cur, refs_cur, C, S.sah_dec.as<Dec>(), n_cur,
-                                                                           io + 14);
+            k_sah_eval_warp<false><<<eval_blocks, EVAL_WPB * 32, 0, st>>>(lv_cur, refs_cur, C, S.sah_dec.as<Dec>(), n_cur, io, jobs);
             count_launch();
         }
         if (next_bound > WARP_MAX)
