@@ -7,6 +7,7 @@
 // This replaces the reference's serial 8-pass LSD sort (src/bvh/bvh_morton.cpp:109-159);
 // stability keeps equal Morton codes in ascending triangle order, as there.
 #include <atomic>
+#include "cta_utils.cuh"
 #include "rt_internal.h"
 
 namespace rtb
@@ -14,58 +15,30 @@ namespace rtb
 namespace
 {
 
-constexpr int      RS_BLOCK   = 256;
-constexpr int      RS_WARPS   = RS_BLOCK / 32;
-// Two tile shapes: up to 2^21 keys, tiles of 16 keys per thread (4096) with 2 resident blocks
-// per SM; above, 8 keys per thread (2048) with 5 resident blocks per SM (48 registers), whose
-// extra occupancy hides the memory latency of the long passes.
+// Two tile shapes (threads, keys per thread, blocks per SM): up to 2^21 keys 4,096 keys on 512
+// threads (100,000 keys: 50 us a sort, 54 on 256 threads of 16 keys); above, 4,608 keys on 384
+// threads. A pass is bound by issue slots (65 % used; ranking, not memory, takes most of them), so
+// the long passes want both many warps and few instructions per key for the tile's own work: at
+// 16.8M keys a sort takes 0.75 ms with 384 x 12, 0.77 with 384 x 13, 0.81 with 384 x 10, 0.83 with
+// 256 x 13 or 512 x 12 and 0.86 with 256 x 8.
 constexpr uint32_t RS_SMALL_MAX = RS_SMALL_MAX_KEYS;
+constexpr int      RS_SB = 512, RS_SI = 8, RS_SM = 2;
+constexpr int      RS_LB = 384, RS_LI = 12, RS_LM = 3;
 constexpr uint32_t LB_AGG     = 1u << 30;           // tile aggregate published
 constexpr uint32_t LB_PRE     = 2u << 30;           // inclusive prefix published
 constexpr uint32_t LB_VAL     = (1u << 30) - 1u;
 constexpr uint32_t SPIN_LIMIT = 1u << 22;           // bounded wait per look-back step
-constexpr int      LB_WIN     = 32;                 // predecessors read per look-back step
+// which path sorts a large input (a word on the device; k_crowded, k_runs)
+constexpr uint32_t SORT_RUNS = 0u, SORT_CROWDED = 1u, SORT_UNDONE = 2u;
+constexpr int      LB_WIN     = 8;                 // predecessors read per look-back step
 
 __device__ __forceinline__ uint32_t ld_volatile(const uint32_t* p) { return *(const volatile uint32_t*)p; }
 __device__ __forceinline__ void     st_volatile(uint32_t* p, uint32_t v) { *(volatile uint32_t*)p = v; }
 
-// Exclusive scan of one value per thread over a 256-thread block; also returns the total.
-__device__ __forceinline__ uint32_t block_excl_scan_256(uint32_t v, uint32_t* warp_sums, uint32_t* total)
-{
-    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-    uint32_t x = v;
-#pragma unroll
-    for (int o = 1; o < 32; o <<= 1)
-    {
-        uint32_t y = __shfl_up_sync(0xffffffffu, x, o);
-        if (lane >= o) { x += y; }
-    }
-    if (lane == 31) { warp_sums[warp] = x; }
-    __syncthreads();
-    if (warp == 0)
-    {
-        uint32_t w = lane < RS_WARPS ? warp_sums[lane] : 0u;
-#pragma unroll
-        for (int o = 1; o < 32; o <<= 1)
-        {
-            uint32_t y = __shfl_up_sync(0xffffffffu, w, o);
-            if (lane >= o) { w += y; }
-        }
-        if (lane < RS_WARPS) { warp_sums[lane] = w; }
-    }
-    __syncthreads();
-    uint32_t base = warp > 0 ? warp_sums[warp - 1] : 0u;
-    if (total) { *total = warp_sums[RS_WARPS - 1]; }
-    uint32_t r = base + x - v;
-    __syncthreads();
-    return r;
-}
-
 // Lanes of the warp holding the same 8-bit digit as this one (d = 0xffffffff: no key; such
 // lanes match only each other): the set __match_any_sync returns, built from one ballot per
-// digit bit plus one for the key's presence. The per-bucket sort below ranks with it (faster
-// there than the match instruction; the onesweep passes keep the instruction, which is faster
-// for them at 16M keys).
+// digit bit plus one for the key's presence. The sorts rank with it: 8 passes over
+// 16.8M keys take 1.43 ms, with the match instruction, whose latency they then wait for, 1.58.
 __device__ __forceinline__ uint32_t match_digit8(uint32_t d)
 {
     const bool valid = d != 0xffffffffu;
@@ -81,182 +54,207 @@ __device__ __forceinline__ uint32_t match_digit8(uint32_t d)
     return m;
 }
 
-template <typename K, int RS_IPT, int MINB>
-__global__ void __launch_bounds__(RS_BLOCK, MINB)
+// Blocks of BLOCK threads, as many as are resident, take tiles of BLOCK * RS_IPT keys in input order
+// (a ticket) until none is left; a launch that is skipped then costs 4 us at any size.
+template <typename K, int BLOCK, int RS_IPT, int MINB>
+__global__ void __launch_bounds__(BLOCK, MINB)
 k_onesweep(const K* __restrict__ kin, const uint32_t* __restrict__ vin, int vals_identity, K* __restrict__ kout,
            uint32_t* __restrict__ vout, uint32_t n, uint32_t tiles, int shift, const uint32_t* __restrict__ hist,
            uint32_t* __restrict__ tile_counter, uint32_t* __restrict__ lookback, uint32_t* __restrict__ status,
            const uint32_t* __restrict__ skip, uint32_t skip_if)
 {
-    if (skip && *skip == skip_if) { return; }  // the other sort path runs (radix_sort_pairs)
-    constexpr int RS_TILE = RS_BLOCK * RS_IPT;
+    const uint32_t skip_word = skip ? *skip : ~skip_if;
+    if (skip_word == skip_if) { return; }  // the other sort path runs (radix_sort_pairs)
+    const bool identity = vals_identity == 1 || (vals_identity == 2 && skip_word == SORT_CROWDED);
+    constexpr int RS_TILE = BLOCK * RS_IPT, WARPS = BLOCK / 32;
+    static_assert(BLOCK >= 256 && RS_TILE < 65536, "one thread per digit, 16-bit offsets in a tile");
     extern __shared__ __align__(16) unsigned char smem[];
     K*        sk     = reinterpret_cast<K*>(smem);
     uint32_t* sv     = reinterpret_cast<uint32_t*>(sk + RS_TILE);
     uint32_t* whist  = sv + RS_TILE;            // [warp][digit]
-    uint32_t* tstart = whist + RS_WARPS * 256;  // tile-local digit start
-    uint32_t* gbase  = tstart + 256;            // global position of digit d minus tstart[d]
+    uint32_t* gbase  = whist + WARPS * 256;     // global position of digit d minus its tile-local start
     __shared__ uint32_t s_tile;
-    __shared__ uint32_t s_warp_sums[RS_WARPS];
+    __shared__ uint32_t s_ts[8], s_hs[8];
 
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-    if (threadIdx.x == 0) { s_tile = atomicAdd(tile_counter, 1u); }
-    for (int i = threadIdx.x; i < RS_WARPS * 256; i += RS_BLOCK) { whist[i] = 0u; }
-    __syncthreads();
-    const uint32_t tile = s_tile;
-    const uint32_t tile_base = tile * (uint32_t)RS_TILE;
-    const uint32_t tile_n = min((uint32_t)RS_TILE, n - tile_base);
-
-    // load: warp w owns the contiguous run [w*32*IPT, (w+1)*32*IPT) of the tile, item j of
-    // lane l is element w*32*IPT + j*32 + l, so (warp, j, lane) order is input order.
-    K        key[RS_IPT];
-    uint32_t val[RS_IPT];
-    uint32_t dig[RS_IPT];
-    uint32_t off[RS_IPT];
-#pragma unroll
-    for (int j = 0; j < RS_IPT; j++)
+    for (;;)
     {
-        const uint32_t li = (uint32_t)warp * (32u * RS_IPT) + (uint32_t)j * 32u + (uint32_t)lane;
-        if (li < tile_n)
+        if (threadIdx.x == 0) { s_tile = atomicAdd(tile_counter, 1u); }
+        for (int i = threadIdx.x; i < WARPS * 256; i += BLOCK) { whist[i] = 0u; }
+        __syncthreads();
+        const uint32_t tile = s_tile;
+        if (tile >= tiles) { return; }
+        const uint32_t tile_base = tile * (uint32_t)RS_TILE;
+        const uint32_t tile_n = min((uint32_t)RS_TILE, n - tile_base);
+
+        // load: warp w owns the contiguous run [w*32*IPT, (w+1)*32*IPT) of the tile, item j of
+        // lane l is element w*32*IPT + j*32 + l, so (warp, j, lane) order is input order.
+        const uint32_t l0 = (uint32_t)warp * (32u * RS_IPT) + (uint32_t)lane;
+        K key[RS_IPT];
+    #pragma unroll
+        for (int j = 0; j < RS_IPT; j++) { key[j] = l0 + 32u * j < tile_n ? kin[tile_base + l0 + 32u * j] : (K)0; }
+        // stable rank inside the warp: peers with the same digit, counted in lane order
+        const uint32_t lt = (1u << lane) - 1u;
+        uint32_t* wh = whist + warp * 256;
+        uint16_t off[RS_IPT];
+    #pragma unroll
+        for (int j = 0; j < RS_IPT; j++)
         {
-            key[j] = kin[tile_base + li];
-            val[j] = vals_identity ? tile_base + li : vin[tile_base + li];
-            dig[j] = (uint32_t)(key[j] >> shift) & 255u;
+            const bool valid = l0 + 32u * j < tile_n;
+            const uint32_t d = (uint32_t)(key[j] >> shift) & 255u;
+            const uint32_t peers = match_digit8(valid ? d : 0xffffffffu);
+            const uint32_t before = __popc(peers & lt);
+            const uint32_t cnt = valid ? wh[d] : 0u;
+            __syncwarp();
+            if (valid && before == 0u) { wh[d] = cnt + __popc(peers); }
+            __syncwarp();
+            off[j] = (uint16_t)(cnt + before);
         }
-        else
+        uint32_t val[RS_IPT];
+    #pragma unroll
+        for (int j = 0; j < RS_IPT; j++)
         {
-            key[j] = 0; val[j] = 0; dig[j] = 0xffffffffu;
+            const uint32_t li = l0 + 32u * j;
+            val[j] = li < tile_n ? (identity ? tile_base + li : vin[tile_base + li]) : 0u;
         }
-    }
-    // stable rank inside the warp: peers with the same digit, counted in lane order
-    const uint32_t lt = (1u << lane) - 1u;
-    uint32_t* wh = whist + warp * 256;
-#pragma unroll
-    for (int j = 0; j < RS_IPT; j++)
-    {
-        const uint32_t d = dig[j];
-        const uint32_t peers = __match_any_sync(0xffffffffu, d);
-        const uint32_t before = __popc(peers & lt);
-        const bool valid = d != 0xffffffffu;
-        uint32_t cnt = valid ? wh[d] : 0u;
-        __syncwarp();
-        if (valid && before == 0u) { wh[d] = cnt + __popc(peers); }
-        __syncwarp();
-        off[j] = cnt + before;
-    }
-    __syncthreads();
+        __syncthreads();
 
-    // per digit: tile count, and exclusive offsets of each warp
-    const uint32_t d = threadIdx.x;  // RS_BLOCK == 256 digits
-    uint32_t run = 0u;
-#pragma unroll
-    for (int w = 0; w < RS_WARPS; w++)
-    {
-        uint32_t c = whist[w * 256 + d];
-        whist[w * 256 + d] = run;
-        run += c;
-    }
-    const uint32_t my = run;
-    // publish this tile's count at once so later tiles can proceed. Status words are
-    // [tile][digit], so a block reads one predecessor's 256 words as one coalesced row.
-    uint32_t* lb = lookback + d;
-    st_volatile(&lb[(size_t)tile * 256u], (tile == 0 ? LB_PRE : LB_AGG) | (my & LB_VAL));
-
-    // scatter into shared memory in digit order; it needs only tile-local offsets, so it runs
-    // before the look-back and frees the item registers
-    const uint32_t ts = block_excl_scan_256(my, s_warp_sums, nullptr);
-    const uint32_t hs = block_excl_scan_256(hist[d], s_warp_sums, nullptr);
-    tstart[d] = ts;
-    __syncthreads();
-#pragma unroll
-    for (int j = 0; j < RS_IPT; j++)
-    {
-        if (dig[j] != 0xffffffffu)
+        // per digit (threads 0 .. 255): tile count, and exclusive offsets of each warp
+        const uint32_t d = threadIdx.x;
+        uint32_t my = 0u, ts = 0u, hs = 0u;
+        uint32_t* lb = lookback + d;
+        if (d < 256u)
         {
-            const uint32_t pos = tstart[dig[j]] + whist[warp * 256 + dig[j]] + off[j];
-            sk[pos] = key[j];
-            sv[pos] = val[j];
-        }
-    }
-
-    // decoupled look-back over earlier tiles: each step reads the status words of up to
-    // LB_WIN predecessors with independent loads and folds them newest first until an
-    // inclusive prefix is met. A word not yet published is waited on alone (bounded, with a
-    // short sleep), then the walk resumes there.
-    uint32_t excl = 0u;
-    if (tile > 0)
-    {
-        int p = (int)tile - 1;
-        uint32_t spins = 0u;
-        bool done = false;
-        while (!done && p >= 0)
-        {
-            uint32_t w[LB_WIN];
-#pragma unroll
-            for (int k = 0; k < LB_WIN; k++) { w[k] = (p - k >= 0) ? ld_volatile(&lb[(size_t)(p - k) * 256u]) : LB_PRE; }
-            int used = 0;
-#pragma unroll
-            for (int k = 0; k < LB_WIN; k++)
+    #pragma unroll
+            for (int w = 0; w < WARPS; w++)
             {
-                if (done || used != k) { continue; }
-                if ((w[k] & ~LB_VAL) == 0u) { continue; }  // not published yet: resume here
-                excl += w[k] & LB_VAL;
-                used = k + 1;
-                if (w[k] & LB_PRE) { done = true; }
+                const uint32_t c = whist[w * 256 + d];
+                whist[w * 256 + d] = my;
+                my += c;
             }
-            p -= used;
-            if (!done && used == 0)
+            // publish this tile's count at once so later tiles can proceed. Status words are
+            // [tile][digit], so a block reads one predecessor's 256 words as one coalesced row.
+            st_volatile(&lb[(size_t)tile * 256u], (tile == 0 ? LB_PRE : LB_AGG) | (my & LB_VAL));
+            // exclusive scans over the digits: of the tile's counts and of the whole input's
+            ts = my;
+            hs = hist[d];
+            const uint32_t h = hs;
+    #pragma unroll
+            for (int o = 1; o < 32; o <<= 1)
             {
-                // wait for tile p alone
-                while ((ld_volatile(&lb[(size_t)p * 256u]) & ~LB_VAL) == 0u)
+                const uint32_t x = __shfl_up_sync(0xffffffffu, ts, o), y = __shfl_up_sync(0xffffffffu, hs, o);
+                if (lane >= o) { ts += x; hs += y; }
+            }
+            if (lane == 31) { s_ts[warp] = ts; s_hs[warp] = hs; }
+            ts -= my;
+            hs -= h;
+        }
+        __syncthreads();
+        if (d < 256u)
+        {
+            for (int w = 0; w < warp; w++) { ts += s_ts[w]; hs += s_hs[w]; }
+    #pragma unroll
+            for (int w = 0; w < WARPS; w++) { whist[w * 256 + d] += ts; }
+        }
+        __syncthreads();
+        // scatter into shared memory in digit order; it needs only tile-local offsets, so it runs
+        // before the look-back and frees the item registers
+    #pragma unroll
+        for (int j = 0; j < RS_IPT; j++)
+        {
+            if (l0 + 32u * j < tile_n)
+            {
+                const uint32_t pos = wh[(uint32_t)(key[j] >> shift) & 255u] + off[j];
+                sk[pos] = key[j];
+                sv[pos] = val[j];
+            }
+        }
+
+        // decoupled look-back over earlier tiles: each step reads the status words of up to
+        // LB_WIN predecessors with independent loads and folds them newest first until an
+        // inclusive prefix is met. A word not yet published is waited on alone (bounded, with a
+        // short sleep), then the walk resumes there.
+        if (d < 256u)
+        {
+            uint32_t excl = 0u;
+            if (tile > 0)
+            {
+                int p = (int)tile - 1;
+                uint32_t spins = 0u;
+                bool done = false;
+                while (!done && p >= 0)
                 {
-                    if (++spins > SPIN_LIMIT) { break; }
-                    __nanosleep(32);
+                    uint32_t w[LB_WIN];
+    #pragma unroll
+                    for (int k = 0; k < LB_WIN; k++) { w[k] = (p - k >= 0) ? ld_volatile(&lb[(size_t)(p - k) * 256u]) : LB_PRE; }
+                    int used = 0;
+    #pragma unroll
+                    for (int k = 0; k < LB_WIN; k++)
+                    {
+                        if (done || used != k) { continue; }
+                        if ((w[k] & ~LB_VAL) == 0u) { continue; }  // not published yet: resume here
+                        excl += w[k] & LB_VAL;
+                        used = k + 1;
+                        if (w[k] & LB_PRE) { done = true; }
+                    }
+                    p -= used;
+                    if (!done && used == 0)
+                    {
+                        // wait for tile p alone
+                        while ((ld_volatile(&lb[(size_t)p * 256u]) & ~LB_VAL) == 0u)
+                        {
+                            if (++spins > SPIN_LIMIT) { break; }
+                            __nanosleep(32);
+                        }
+                        if (spins > SPIN_LIMIT) { atomicOr(status, ST_TIMEOUT); break; }
+                    }
                 }
-                if (spins > SPIN_LIMIT) { atomicOr(status, ST_TIMEOUT); break; }
+                st_volatile(&lb[(size_t)tile * 256u], LB_PRE | ((excl + my) & LB_VAL));
             }
+            gbase[d] = hs + excl - ts;
         }
-        st_volatile(&lb[(size_t)tile * 256u], LB_PRE | ((excl + my) & LB_VAL));
-    }
-    gbase[d] = hs + excl - ts;
-    __syncthreads();
+        __syncthreads();
 
-    // write out with contiguous runs per digit
-    for (uint32_t i = threadIdx.x; i < tile_n; i += RS_BLOCK)
-    {
-        const K k = sk[i];
-        const uint32_t g = gbase[(uint32_t)(k >> shift) & 255u] + i;
-        if (g >= n) { atomicOr(status, ST_CAPACITY); continue; }
-        kout[g] = k;
-        vout[g] = sv[i];
+        // write out with contiguous runs per digit
+        for (uint32_t i = threadIdx.x; i < tile_n; i += BLOCK)
+        {
+            const K k = sk[i];
+            const uint32_t g = gbase[(uint32_t)(k >> shift) & 255u] + i;
+            if (g >= n) { atomicOr(status, ST_CAPACITY); continue; }
+            kout[g] = k;
+            vout[g] = sv[i];
+        }
+        __syncthreads();  // the next tile reuses the shared memory
     }
 }
 
-template <typename K, int IPT>
+template <typename K, int BLOCK, int IPT>
 constexpr size_t onesweep_smem()
 {
-    return (size_t)RS_BLOCK * IPT * sizeof(K) + (size_t)RS_BLOCK * IPT * 4 + (size_t)RS_WARPS * 256 * 4 + 2 * 256 * 4;
+    return (size_t)BLOCK * IPT * (sizeof(K) + 4) + (size_t)(BLOCK / 32) * 256 * 4 + 256 * 4;
 }
 
-// All passes of one tile shape on the given scratch. skip (device, optional): the passes do
-// nothing when *skip == skip_if (the MSD path of radix_sort_pairs sorted the keys instead).
-template <typename K, int IPT, int MINB>
-int onesweep_passes(K* keys, uint32_t* vals, bool vals_identity, uint32_t n, int passes, const uint32_t* hist, K* keys_alt,
+// Passes first .. last - 1 of one tile shape on the given scratch. skip (device, optional): the
+// passes do nothing when *skip == skip_if (another path of radix_sort_pairs sorts the keys).
+// identity: 1 = pass `first` takes the positions as values, 2 = only while *skip == SORT_CROWDED.
+template <typename K, int BLOCK, int IPT, int MINB>
+int onesweep_passes(K* keys, uint32_t* vals, int identity, uint32_t n, int first, int last, const uint32_t* hist, K* keys_alt,
                     uint32_t* vals_alt, uint32_t* lookback, uint32_t* tile_counters, uint32_t* status, cudaStream_t st,
                     K** keys_out, uint32_t** vals_out, const uint32_t* skip = nullptr, uint32_t skip_if = 0,
                     bool zeroed = false)
 {
-    constexpr uint32_t tile = RS_BLOCK * IPT;
+    constexpr uint32_t tile = BLOCK * IPT;
     const uint32_t tiles = (n + tile - 1) / tile;
     if (!zeroed)
     {
-        RT_CUDA(cudaMemsetAsync(lookback, 0, (size_t)passes * tiles * 256 * 4, st));
+        RT_CUDA(cudaMemsetAsync(lookback, 0, (size_t)last * tiles * 256 * 4, st));
         RT_CUDA(cudaMemsetAsync(tile_counters, 0, 64 * 4, st));
     }
-    constexpr size_t smem = onesweep_smem<K, IPT>();
+    constexpr size_t smem = onesweep_smem<K, BLOCK, IPT>();
     static PerDeviceOnce attr;  // per instantiation and device (bakes may run on several host threads and GPUs)
     if (int e = attr.once([] {
-            RT_CUDA(cudaFuncSetAttribute(k_onesweep<K, IPT, MINB>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+            RT_CUDA(cudaFuncSetAttribute(k_onesweep<K, BLOCK, IPT, MINB>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                         (int)smem));
             return (int)RT_OK;
         }))
     {
@@ -266,11 +264,12 @@ int onesweep_passes(K* keys, uint32_t* vals, bool vals_identity, uint32_t n, int
     K* kalt = keys_alt;
     uint32_t* vin = vals;
     uint32_t* valt = vals_alt;
-    for (int p = 0; p < passes; p++)
+    const uint32_t grid = std::min(tiles, (uint32_t)(MINB * device_sm_count()));
+    for (int p = first; p < last; p++)
     {
-        k_onesweep<K, IPT, MINB><<<tiles, RS_BLOCK, smem, st>>>(kin, vin, (vals_identity && p == 0) ? 1 : 0, kalt, valt, n,
-                                                                tiles, 8 * p, hist + 256 * p, tile_counters + p,
-                                                                lookback + (size_t)p * tiles * 256, status, skip, skip_if);
+        k_onesweep<K, BLOCK, IPT, MINB><<<grid, BLOCK, smem, st>>>(kin, vin, p == first ? identity : 0, kalt, valt, n, tiles,
+                                                                   8 * p, hist + 256 * p, tile_counters + p,
+                                                                   lookback + (size_t)p * tiles * 256, status, skip, skip_if);
         count_launch();
         if (int e = check_launch("onesweep")) { return e; }
         K* tk = kin; kin = kalt; kalt = tk;
@@ -279,6 +278,132 @@ int onesweep_passes(K* keys, uint32_t* vals, bool vals_identity, uint32_t n, int
     *keys_out = kin;
     *vals_out = vin;
     return RT_OK;
+}
+
+// ---- Large sorts of 7 or 8 digits: the four top digits by onesweep passes, then every run of
+// keys equal in them ordered by the rest where it stands (k_runs). A cell of the four top digits
+// of a 63-bit Morton code is a 1,290th of the scene on a side, so runs are short (1 to 10 keys
+// for soups and surfaces) unless triangles crowd together. Whether they do is estimated first
+// from a sample of the keys (k_crowded); a run of more than n / RUN_DIV keys that the sample
+// missed undoes the choice. The LSD passes then sort the keys, on the device's word, without the
+// host. The order is the LSD passes' own: the top passes are stable and equal keys of a run keep
+// theirs. 16.8M keys: 0.75 ms, against 1.57 by 8 passes (a crowded
+// input) and 2.15 where a run was missed; 8 passes on 2,048-key tiles that ranked with the match
+// instruction took 1.79.
+constexpr uint32_t RUN_DIV = 512;
+constexpr int TOP_PASSES = 4;
+constexpr uint32_t CR_SAMPLES = 8192, CR_TABLE = 2 * CR_SAMPLES;
+
+// One block: *path = SORT_CROWDED when too many of CR_SAMPLES evenly spaced keys share their top
+// digits. Runs of L keys make CR_SAMPLES^2 / 2 * L / n such pairs; the line is at L = 64, where
+// k_runs costs about as much as the passes it saves. One run of L keys holds CR_SAMPLES * L / n
+// samples; 8 of them in one run mark one of about n / 1024 keys or more, half of what k_runs takes
+// (one thread's walk over it, some 25 cycles a key, stays below the time of the passes saved).
+template <typename K>
+__global__ void __launch_bounds__(1024) k_crowded(const K* __restrict__ keys, uint32_t n, int low_bits,
+                                                  uint32_t* __restrict__ path)
+{
+    extern __shared__ uint32_t tab[];
+    uint32_t* cnt = tab + CR_TABLE;
+    __shared__ uint32_t s_dup, s_max;
+    for (uint32_t i = threadIdx.x; i < CR_TABLE; i += 1024) { tab[i] = 0xffffffffu; cnt[i] = 0u; }
+    if (threadIdx.x == 0) { s_dup = 0u; s_max = 0u; }
+    __syncthreads();
+    uint32_t dup = 0, most = 0;
+    for (uint32_t i = threadIdx.x; i < CR_SAMPLES; i += 1024)
+    {
+        // 31 bits: a table word is never all ones
+        const uint32_t top = (uint32_t)(keys[(uint64_t)i * n / CR_SAMPLES] >> low_bits) & 0x7fffffffu;
+        uint32_t h = (top * 2654435769u) >> 18;  // 14 bits (Knuth's multiplicative hash)
+        for (uint32_t probe = 0; probe < CR_TABLE; probe++)
+        {
+            const uint32_t was = atomicCAS(&tab[h], 0xffffffffu, top);
+            if (was == 0xffffffffu) { break; }
+            if (was == top)
+            {
+                dup++;
+                most = max(most, atomicAdd(&cnt[h], 1u) + 2u);
+                break;
+            }
+            h = (h + 1u) & (CR_TABLE - 1u);
+        }
+    }
+    if (dup) { atomicAdd(&s_dup, dup); atomicMax(&s_max, most); }
+    __syncthreads();
+    if (threadIdx.x == 0)
+    {
+        const uint32_t line = 8u + (uint32_t)(64ull * CR_SAMPLES * CR_SAMPLES / 2 / n);
+        *path = s_dup > line || s_max >= 8u ? SORT_CROWDED : SORT_RUNS;
+    }
+}
+
+// The rank of every key in its run (by the low bits, then by position), counted by walking to
+// both ends of the run, four keys at a time: neighbouring lanes read neighbouring keys, so the
+// walk hits L1.
+template <typename K>
+__global__ void __launch_bounds__(256) k_runs(const K* __restrict__ kin, const uint32_t* __restrict__ vin, uint32_t n,
+                                              int low_bits, uint32_t run_max, K* __restrict__ kout,
+                                              uint32_t* __restrict__ vout, uint32_t* __restrict__ path)
+{
+    if (*path != SORT_RUNS) { return; }
+    const uint32_t i = blockIdx.x * 256u + threadIdx.x;
+    if (i >= n) { return; }
+    const K k = kin[i];
+    const uint32_t v = vin[i];
+    const K top = k >> low_bits;
+    uint32_t back = 0, fwd = 0, before = 0;
+    if (i > 0 && (kin[i - 1u] >> low_bits) == top)
+    {
+        for (bool in = true; in && back < run_max;)
+        {
+            K o[4];
+#pragma unroll
+            for (uint32_t j = 0; j < 4; j++) { o[j] = back + j < i ? kin[i - 1u - back - j] : ~k; }
+#pragma unroll
+            for (int j = 0; j < 4; j++)
+            {
+                in = in && (o[j] >> low_bits) == top;
+                if (in) { back++; before += o[j] <= k; }
+            }
+        }
+    }
+    if (i + 1u < n && (kin[i + 1u] >> low_bits) == top)
+    {
+        for (bool in = true; in && fwd < run_max;)
+        {
+            K o[4];
+#pragma unroll
+            for (uint32_t j = 0; j < 4; j++) { o[j] = fwd + j < n - 1u - i ? kin[i + 1u + fwd + j] : ~k; }
+#pragma unroll
+            for (int j = 0; j < 4; j++)
+            {
+                in = in && (o[j] >> low_bits) == top;
+                if (in) { fwd++; before += o[j] < k; }
+            }
+        }
+    }
+    if (back + fwd >= run_max) { *path = SORT_UNDONE; return; }
+    kout[i - back + before] = k;
+    vout[i - back + before] = v;
+}
+
+// The LSD passes after an undone choice start from cleared look-back words and tickets.
+__global__ void __launch_bounds__(256) k_undone(uint32_t* __restrict__ lookback, size_t words, uint32_t* __restrict__ tickets,
+                                                const uint32_t* __restrict__ path)
+{
+    if (*path != SORT_UNDONE) { return; }
+    for (size_t i = blockIdx.x * 256u + threadIdx.x; i < words; i += gridDim.x * 256u) { lookback[i] = 0u; }
+    if (blockIdx.x == 0 && threadIdx.x < 64) { tickets[threadIdx.x] = 0u; }
+}
+
+// The sorted keys to the buffers where the other path leaves them.
+template <typename K>
+__global__ void __launch_bounds__(256) k_settle(const K* __restrict__ kin, const uint32_t* __restrict__ vin, uint32_t n,
+                                                K* __restrict__ kout, uint32_t* __restrict__ vout,
+                                                const uint32_t* __restrict__ path)
+{
+    if (*path == SORT_RUNS) { return; }
+    for (uint32_t i = blockIdx.x * 256u + threadIdx.x; i < n; i += gridDim.x * 256u) { kout[i] = kin[i]; vout[i] = vin[i]; }
 }
 
 // ---- MSD path: one onesweep pass on the most significant digit, then every bucket of that
@@ -296,13 +421,13 @@ __global__ void __launch_bounds__(256)
 k_msd_check(const uint32_t* __restrict__ hist_top, uint32_t n, uint32_t cap, uint32_t* __restrict__ bstart,
             uint32_t* __restrict__ flag, uint32_t* __restrict__ flag_copy)
 {
-    __shared__ uint32_t ws[RS_WARPS];
+    __shared__ uint32_t ws[256 / 32 + 1];
     __shared__ uint32_t s_big;
     const uint32_t h = hist_top[threadIdx.x];
     if (threadIdx.x == 0) { s_big = 0u; }
     __syncthreads();
     if (h > cap) { atomicOr(&s_big, 1u); }
-    const uint32_t ex = block_excl_scan_256(h, ws, nullptr);
+    const uint32_t ex = block_excl_scan<256>(h, ws, nullptr);
     bstart[threadIdx.x] = ex;
     if (threadIdx.x == 0)
     {
@@ -622,7 +747,7 @@ k_local_sort(const K* kin, const uint32_t* vin, K* kout, uint32_t* vout, const u
 // Look-back words the sort of n keys needs (passes x tiles x 256).
 size_t sort_lookback_words(uint32_t n, int passes)
 {
-    const uint32_t tile = n <= RS_SMALL_MAX ? RS_BLOCK * 16 : RS_BLOCK * 8;
+    const uint32_t tile = n <= RS_SMALL_MAX ? RS_SB * RS_SI : RS_LB * RS_LI;
     return (size_t)passes * ((n + tile - 1) / tile) * 256;
 }
 
@@ -657,14 +782,15 @@ int radix_sort_pairs(K* keys, uint32_t* vals, bool vals_identity, uint32_t n, in
         {
             // top digit (bits key_bits-8 .. key_bits-1) by one onesweep pass keys -> alt, then the
             // buckets by the lower digits in shared memory, alt -> the buffer the LSD passes end in
-            constexpr uint32_t tile = RS_BLOCK * 16;
+            constexpr uint32_t tile = RS_SB * RS_SI;
             const uint32_t tiles = (n + tile - 1) / tile;
-            constexpr size_t smem = onesweep_smem<K, 16>();
+            constexpr size_t smem = onesweep_smem<K, RS_SB, RS_SI>();
             constexpr size_t sm_small = local_sort_smem<K, LS_SMALL_B, LS_SMALL_I>();
             constexpr size_t sm_large = local_sort_smem<K, LS_LARGE_B, LS_LARGE_I>();
             static PerDeviceOnce attr;  // per key type and device
             if (int e = attr.once([] {
-                    RT_CUDA(cudaFuncSetAttribute(k_onesweep<K, 16, 2>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+                    RT_CUDA(cudaFuncSetAttribute(k_onesweep<K, RS_SB, RS_SI, RS_SM>,
+                                                 cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
                     RT_CUDA(cudaFuncSetAttribute(k_local_sort<K, LS_SMALL_B, LS_SMALL_I, 2>,
                                                  cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm_small));
                     RT_CUDA(cudaFuncSetAttribute(k_local_sort<K, LS_LARGE_B, LS_LARGE_I, 1>,
@@ -692,9 +818,9 @@ int radix_sort_pairs(K* keys, uint32_t* vals, bool vals_identity, uint32_t n, in
                 RT_CUDA(cudaMemsetAsync(s.tile_counters.as<uint32_t>() + 63, 0, 4, st));
             }
             k_msd_check<<<1, 256, 0, st>>>(msd_hist, n, small ? cap_small : cap_large, bstart, flag, msd_only_flag);
-            k_onesweep<K, 16, 2><<<tiles, RS_BLOCK, smem, st>>>(keys, vals, vals_identity ? 1 : 0, kalt, valt, n, tiles,
-                                                                key_bits - 8, msd_hist, s.tile_counters.as<uint32_t>() + 63,
-                                                                s.lookback.as<uint32_t>(), status, flag, 1u);
+            k_onesweep<K, RS_SB, RS_SI, RS_SM><<<std::min(tiles, (uint32_t)(RS_SM * device_sm_count())), RS_SB, smem, st>>>(
+                keys, vals, vals_identity ? 1 : 0, kalt, valt, n, tiles, key_bits - 8, msd_hist,
+                s.tile_counters.as<uint32_t>() + 63, s.lookback.as<uint32_t>(), status, flag, 1u);
             if (small)
             {
                 k_local_sort<K, LS_SMALL_B, LS_SMALL_I, 2><<<256, LS_SMALL_B, sm_small, st>>>(kalt, valt, kfin, vfin, bstart,
@@ -714,13 +840,60 @@ int radix_sort_pairs(K* keys, uint32_t* vals, bool vals_identity, uint32_t n, in
                 return RT_OK;
             }
         }
-        return onesweep_passes<K, 16, 2>(keys, vals, vals_identity, n, passes, hist, s.keys_alt.as<K>(), s.vals_alt.as<uint32_t>(),
-                                         s.lookback.as<uint32_t>(), s.tile_counters.as<uint32_t>(), status, st, keys_out,
-                                         vals_out, msd ? flag : nullptr, 0u, scratch_zeroed);
+        return onesweep_passes<K, RS_SB, RS_SI, RS_SM>(keys, vals, vals_identity ? 1 : 0, n, 0, passes, hist,
+                                                       s.keys_alt.as<K>(), s.vals_alt.as<uint32_t>(),
+                                                       s.lookback.as<uint32_t>(), s.tile_counters.as<uint32_t>(), status, st,
+                                                       keys_out, vals_out, msd ? flag : nullptr, 0u, scratch_zeroed);
     }
-    return onesweep_passes<K, 8, 5>(keys, vals, vals_identity, n, passes, hist, s.keys_alt.as<K>(), s.vals_alt.as<uint32_t>(),
-                                    s.lookback.as<uint32_t>(), s.tile_counters.as<uint32_t>(), status, st, keys_out, vals_out,
-                                    nullptr, 0u, scratch_zeroed);
+    uint32_t* lookback = s.lookback.as<uint32_t>();
+    uint32_t* tickets = s.tile_counters.as<uint32_t>();
+    K* kalt = s.keys_alt.as<K>();
+    uint32_t* valt = s.vals_alt.as<uint32_t>();
+    const int identity = vals_identity ? 1 : 0;
+    if (passes < TOP_PASSES + 3)
+    {
+        return onesweep_passes<K, RS_LB, RS_LI, RS_LM>(keys, vals, identity, n, 0, passes, hist, kalt, valt, lookback, tickets,
+                                                       status, st, keys_out, vals_out, nullptr, 0u, scratch_zeroed);
+    }
+    const int low_bits = 8 * (passes - TOP_PASSES);
+    uint32_t* path = tickets + 64;
+    static PerDeviceOnce attr;  // per key type and device
+    if (int e = attr.once([] {
+            RT_CUDA(cudaFuncSetAttribute(k_crowded<K>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)(CR_TABLE * 8)));
+            return (int)RT_OK;
+        }))
+    {
+        return e;
+    }
+    k_crowded<K><<<1, 1024, CR_TABLE * 8, st>>>(keys, n, low_bits, path);
+    K* ktop = nullptr;
+    uint32_t* vtop = nullptr;
+    if (int e = onesweep_passes<K, RS_LB, RS_LI, RS_LM>(keys, vals, identity, n, passes - TOP_PASSES, passes, hist, kalt, valt,
+                                                        lookback, tickets, status, st, &ktop, &vtop, path, SORT_CROWDED,
+                                                        scratch_zeroed))
+    {
+        return e;
+    }
+    // an even number of passes: the keys are back in their own buffers
+    k_runs<K><<<(n + 255) / 256, 256, 0, st>>>(ktop, vtop, n, low_bits, n / RUN_DIV, kalt, valt, path);
+    const uint32_t blocks = 8u * (uint32_t)device_sm_count();
+    k_undone<<<blocks, 256, 0, st>>>(lookback, lbw, tickets, path);
+    count_launch(3);
+    K* klsd = nullptr;
+    uint32_t* vlsd = nullptr;
+    if (int e = onesweep_passes<K, RS_LB, RS_LI, RS_LM>(keys, vals, identity ? 2 : 0, n, 0, passes, hist, kalt, valt, lookback,
+                                                        tickets, status, st, &klsd, &vlsd, path, SORT_RUNS, true))
+    {
+        return e;
+    }
+    if (klsd != kalt)
+    {
+        k_settle<K><<<blocks, 256, 0, st>>>(klsd, vlsd, n, kalt, valt, path);
+        count_launch();
+    }
+    *keys_out = kalt;
+    *vals_out = valt;
+    return check_launch("radix sort");
 }
 
 template int radix_sort_pairs<uint64_t>(uint64_t*, uint32_t*, bool, uint32_t, int, const uint32_t*, const uint32_t*,
@@ -748,9 +921,9 @@ int radix_sort_pairs_raw(K* keys, uint32_t* vals, uint32_t n, int key_bits, cons
     if (n == 0) { return RT_OK; }
     const int passes = sort_passes(key_bits);
     if (n > RS_SMALL_MAX) { return fail(RT_E_CAPACITY, "radix sort on fixed scratch: at most 2^21 keys"); }
-    static_assert(RS_BLOCK * 16 == RS_SMALL_TILE_KEYS, "fixed-scratch callers size the look-back words by this tile");
-    return onesweep_passes<K, 16, 2>(keys, vals, true, n, passes, hist, keys_alt, vals_alt, lookback, tile_counters, status, st,
-                                     keys_out, vals_out);
+    static_assert(RS_SB * RS_SI == RS_SMALL_TILE_KEYS, "fixed-scratch callers size the look-back words by this tile");
+    return onesweep_passes<K, RS_SB, RS_SI, RS_SM>(keys, vals, 1, n, 0, passes, hist, keys_alt, vals_alt, lookback,
+                                                   tile_counters, status, st, keys_out, vals_out);
 }
 
 template int radix_sort_pairs_raw<uint64_t>(uint64_t*, uint32_t*, uint32_t, int, const uint32_t*, uint64_t*, uint32_t*,

@@ -85,8 +85,9 @@ int          device_sm_count();
 
 // ---- radix sort (radix_sort.cu) ---------------------------------------------------------
 // Stable sort of `n` keys with uint32 values by their low `key_bits` bits: onesweep LSD
-// passes, or up to 2^21 keys an MSD pass on the top digit and a per-bucket sort in shared
-// memory (radix_sort_pairs). Histograms of all digit passes must already be in `hist` (256
+// passes, up to 2^21 keys an MSD pass on the top digit and a per-bucket sort in shared memory,
+// above that (7 or 8 digits) passes on the top four digits and a sort of the runs they leave
+// (radix_sort_pairs). Histograms of all digit passes must already be in `hist` (256
 // counters per pass, built by the producer of the keys). keys/vals are ping-ponged: the
 // sorted result ends in the buffer returned through *keys_out / *vals_out.
 struct SortScratch
@@ -119,8 +120,8 @@ int radix_sort_pairs_raw(K* keys, uint32_t* vals, uint32_t n, int key_bits, cons
 inline int sort_passes(int key_bits) { return (key_bits + 7) / 8; }
 // Look-back words (passes x tiles x 256) a sort of n keys uses.
 size_t sort_lookback_words(uint32_t n, int passes);
-// Keys per tile of the onesweep passes up to RS_SMALL_MAX_KEYS keys (256 threads x 16 keys),
-// the shape radix_sort_pairs_raw always uses; above that size the tile is half as large.
+// Keys per tile of the onesweep passes up to RS_SMALL_MAX_KEYS keys,
+// the shape radix_sort_pairs_raw always uses.
 constexpr uint32_t RS_SMALL_TILE_KEYS = 4096;
 constexpr uint32_t RS_SMALL_MAX_KEYS = 1u << 21;
 // Look-back words of a radix_sort_pairs_raw sort of n keys (n <= RS_SMALL_MAX_KEYS).
