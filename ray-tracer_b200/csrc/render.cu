@@ -24,10 +24,10 @@
 // Adjoint (no counterpart in the reference): gradients of sum(dL/dI * I) with respect to the
 // albedo used at each triangle and each material's emission, by path-replay backpropagation
 // (Vicini, Speierer, Jakob: "Path Replay Backpropagation", SIGGRAPH 2021). Per sample, a first
-// pass computes the path's radiance L; a second pass re-traces the same path from the same
-// counter-based random numbers, and at vertex k the radiance still to come,
-// L - sum_{i<=k} T_i E_i, divided by the albedo there is dL/dalbedo_k. The RNG is recomputed,
-// not stored, so memory stays O(pixels). Russian-roulette probabilities are held constant.
+// pass computes the path's radiance L and keeps its triangles; a second pass follows them (or
+// re-traces a long path from the same counter-based random numbers), and at vertex k the radiance still to
+// come, L - sum_{i<=k} T_i E_i, divided by the albedo there is dL/dalbedo_k. One path per thread
+// is kept at a time, so memory stays O(pixels). Russian-roulette probabilities are held constant.
 #include "trace_warp.cuh"
 
 #include <algorithm>
@@ -329,9 +329,14 @@ k_paths(const TraceCtx T, const __grid_constant__ PathJob J, uint32_t* __restric
     }
 }
 
-// The radiance of one sample of one pixel (primaryRay + pathTrace).
+constexpr uint32_t NO_TRI = 0xFFFFFFFFu;
+constexpr uint32_t REC_BOUNCES = 64;  // triangles of a path that are kept
+
+// The radiance of one sample of one pixel (primaryRay + pathTrace). REC: rec[] gets the triangles
+// of the path, and NO_TRI after its last where it ends before max_bounce.
+template <bool REC>
 __device__ __forceinline__ f3 path_sample(const TraceCtx& T, const RP& P, const Shade& S, uint32_t x, uint32_t y,
-                                          uint32_t pix, uint32_t sidx)
+                                          uint32_t pix, uint32_t sidx, uint32_t (&rec)[REC_BOUNCES])
 {
     f3 o, d;
     primary(P, P.cam, x, y, pix, sidx, o, d);
@@ -340,6 +345,7 @@ __device__ __forceinline__ f3 path_sample(const TraceCtx& T, const RP& P, const 
     for (uint32_t bounce = 0; bounce <= P.max_bounce; bounce++)
     {
         const THit H = trace_ray<0>(T, o, d, tmin, bits2f(0x7f800000u));
+        if (REC) { rec[bounce] = H.hit ? H.tri : NO_TRI; }
         if (!H.hit)
         {
             L = add3(L, mul3(tp, environment(P, d)));
@@ -347,9 +353,14 @@ __device__ __forceinline__ f3 path_sample(const TraceCtx& T, const RP& P, const 
         }
         const Surf sf = surface(S, H.tri);
         L = add3(L, mul3(tp, sf.emission));
+        if (REC && bounce == P.max_bounce) { break; }
         const f3 n = hit_normal(T, H.tri, H.u, H.v);
         f3 nd;
-        if (!scatter(P, P.cam.seed, sf, n, d, pix, sidx, bounce, tp, nd)) { break; }
+        if (!scatter(P, P.cam.seed, sf, n, d, pix, sidx, bounce, tp, nd))
+        {
+            if (REC) { rec[bounce + 1] = NO_TRI; }
+            break;
+        }
         o = add3(o, muls(d, H.t));
         d = nd;
         tmin = 1e-4f;
@@ -392,14 +403,22 @@ __device__ __forceinline__ void warp_add3(float* __restrict__ dst, uint32_t key,
     }
 }
 
-// Why a thread per pixel and per-lane traversal stay here: a material's emission gradient is one
-// 32-bit sum of millions of terms, off by 1.5e-4 from the exact one at 512 x 512 x 32, and where it
-// ends up depends on which tiles are at work together; schedules that trace 3-5 times faster move
-// it by up to 3e-5.
-// Path-replay adjoint, one thread per pixel (the plain schedule). Lanes run the replay's
-// bounce loop in step so the gradient adds can be combined per warp; pixels whose dL/dI is
-// zero are skipped.
-__global__ void __launch_bounds__(128)
+// Path-replay adjoint, one thread per pixel. Lanes run the replay's bounce loop in step so the
+// gradient adds can be combined per warp; pixels whose dL/dI is zero are skipped.
+//
+// REC: the forward pass keeps the triangles of its path, and the replay needs no more: throughput and
+// gradients follow from them (roulette's survivors are the paths with a next triangle). Without it
+// the replay traces the path again, which half of the time went to: 512 x 512 x 32, 50,000
+// triangles, 4 bounces 106 -> 57 ms, 200,000 triangles, 5 bounces 201 -> 105 ms. Paths of more than
+// REC_BOUNCES bounces are traced twice.
+//
+// Why a thread per pixel, per-lane traversal and five blocks per SM: a material's emission gradient
+// is one 32-bit sum of millions of terms, off by 1.5e-4 from the exact one at 512 x 512 x 32, and
+// where it ends up depends on which tiles are at work together. With this schedule it stays within 1.2e-5
+// of the path traced twice; warps that trace together as the renderer's do (31 ms) move it by 0.5-4e-5,
+// paths traced by k_paths and replayed by a kernel of their own (35 ms) or other numbers of blocks by up to 3e-4.
+template <bool REC>
+__global__ void __launch_bounds__(128, 5)
 k_adjoint(TraceCtx T, RP P, Shade S, const float* __restrict__ dimg, float* __restrict__ g_alb, float* __restrict__ g_em)
 {
     const uint32_t x = blockIdx.x * 16 + (threadIdx.x & 15);
@@ -411,14 +430,15 @@ k_adjoint(TraceCtx T, RP P, Shade S, const float* __restrict__ dimg, float* __re
     if (in_img) { dl = mk3(dimg[3 * pix] / fs, dimg[3 * pix + 1] / fs, dimg[3 * pix + 2] / fs); }
     const bool act = in_img && (dl.x != 0.f || dl.y != 0.f || dl.z != 0.f);
     if (!__any_sync(0xFFFFFFFFu, act)) { return; }
+    uint32_t rec[REC_BOUNCES];
     for (uint32_t s = 0; s < P.spp; s++)
     {
         const uint32_t sidx = P.sample_offset + s;
         f3 Ltot = mk3(0.f, 0.f, 0.f);
-        if (act) { Ltot = path_sample(T, P, S, x, y, pix, sidx); }
+        if (act) { Ltot = path_sample<REC>(T, P, S, x, y, pix, sidx, rec); }
         // replay
         f3 o = mk3(0.f, 0.f, 0.f), d = mk3(0.f, 0.f, 1.f);
-        if (act) { primary(P, P.cam, x, y, pix, sidx, o, d); }
+        if (!REC && act) { primary(P, P.cam, x, y, pix, sidx, o, d); }
         float tmin = 1e-3f;
         f3 tp = mk3(1.f, 1.f, 1.f), Ssum = mk3(0.f, 0.f, 0.f);
         bool alive = act;
@@ -430,27 +450,41 @@ k_adjoint(TraceCtx T, RP P, Shade S, const float* __restrict__ dimg, float* __re
             f3 ga = mk3(0.f, 0.f, 0.f), ge = mk3(0.f, 0.f, 0.f);
             if (alive)
             {
-                const THit H = trace_ray<0>(T, o, d, tmin, bits2f(0x7f800000u));
-                if (!H.hit) { alive = false; }
+                THit H;
+                if (REC) { tri = rec[bounce]; }
                 else
                 {
-                    const Surf sf = surface(S, H.tri);
-                    hv = true; tri = H.tri; mat = sf.mat;
+                    H = trace_ray<0>(T, o, d, tmin, bits2f(0x7f800000u));
+                    tri = H.hit ? H.tri : NO_TRI;
+                }
+                if (tri == NO_TRI) { alive = false; }
+                else
+                {
+                    const Surf sf = surface(S, tri);
+                    hv = true; mat = sf.mat;
                     ge = mul3(dl, tp);
                     Ssum = add3(Ssum, mul3(tp, sf.emission));
                     const f3 rest = sub3(Ltot, Ssum);
                     ga = mk3(sf.albedo.x != 0.f ? dl.x * rest.x / sf.albedo.x : 0.f,
                              sf.albedo.y != 0.f ? dl.y * rest.y / sf.albedo.y : 0.f,
                              sf.albedo.z != 0.f ? dl.z * rest.z / sf.albedo.z : 0.f);
-                    const f3 n = hit_normal(T, H.tri, H.u, H.v);
-                    f3 nd;
-                    if (!scatter(P, P.cam.seed, sf, n, d, pix, sidx, bounce, tp, nd) || bounce >= P.max_bounce)
+                    if (REC)
                     {
-                        alive = false;
+                        tp = mul3(tp, sf.albedo);
+                        if (P.rr_after >= 0 && (int32_t)bounce > P.rr_after) { tp = divs(tp, std_max(std_max(tp.x, tp.y), tp.z)); }
                     }
-                    o = add3(o, muls(d, H.t));
-                    d = nd;
-                    tmin = 1e-4f;
+                    else
+                    {
+                        const f3 n = hit_normal(T, tri, H.u, H.v);
+                        f3 nd;
+                        if (!scatter(P, P.cam.seed, sf, n, d, pix, sidx, bounce, tp, nd) || bounce >= P.max_bounce)
+                        {
+                            alive = false;
+                        }
+                        o = add3(o, muls(d, H.t));
+                        d = nd;
+                        tmin = 1e-4f;
+                    }
                 }
             }
             if (g_alb) { warp_add3(g_alb, tri, hv, ga); }
@@ -746,7 +780,8 @@ int adjoint(const rt_bvh* B, const rt_render_cfg& cfg, const rt_shading& sh, con
     const RP P = make_rp(cfg, sh);
     const Shade S{ sh.mats, sh.mat_of_tri, sh.tri_albedo, sh.n_mats };
     const dim3 grid((cfg.width + 15) / 16, (cfg.height + 7) / 8);
-    k_adjoint<<<grid, 128, 0, st>>>(T, P, S, d_rgb, g_alb, sh.mats ? g_em : nullptr);
+    const auto fn = cfg.max_bounce < REC_BOUNCES ? k_adjoint<true> : k_adjoint<false>;
+    fn<<<grid, 128, 0, st>>>(T, P, S, d_rgb, g_alb, sh.mats ? g_em : nullptr);
     count_launch();
     return check_launch("adjoint");
 }

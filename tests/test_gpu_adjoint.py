@@ -167,6 +167,23 @@ def test_autograd_harness_descends():
     assert losses[-1] < 0.9 * losses[0], losses
 
 
+@pytest.mark.parametrize("rr_after", [-1, 2])
+@pytest.mark.parametrize("size", [(24, 16), (33, 9)])
+def test_adjoint_with_kept_and_with_retraced_paths(rr_after, size):
+    """Up to 63 bounces the forward pass keeps a path's triangles, above that the replay traces it again.
+    What a 65th vertex adds is below 0.75^64 of its path, so the gradients at 63 and 64 bounces are
+    float sums of the same terms in other orders: at most 2e4 terms into one sum, rounding by about
+    sqrt(2e4) 2^-24 = 8e-6 of it; held to ten times that."""
+    sc = small_scene()
+    b = rtb200.Bvh.build(sc.verts, sc.tris, "hybrid")
+    mot = sc.baked_materials(b.prim_ids())
+    d = torch.ones(size[1], size[0], 3, device="cuda")
+    kept, again = (b.adjoint(rcfg(*size, 8, max_bounce=m, rr_after=rr_after), d, sc.mats, mot) for m in (63, 64))
+    for x, y in zip(kept, again):
+        x, y = x.double(), y.double()
+        assert float(y.norm()) > 0 and float((x - y).norm()) <= 8e-5 * float(y.norm())
+
+
 def test_adjoint_skips_zero_weight_pixels_and_validates():
     sc = small_scene(1)
     b = rtb200.Bvh.build(sc.verts, sc.tris, "lbvh30")
