@@ -1959,6 +1959,154 @@ k_sah_offsets(Dec* __restrict__ dec, uint32_t n_lvl, unsigned long long* __restr
     }
 }
 
+// The three kernels above as one, for a level of one scene that a block holds: the launches and the
+// passes over memory between them took longer than their work (three launches and a look-back, 15 us a level
+// under ncu; one launch here). Decisions and results are the same: the requests all fit, not even the
+// smallest does, or one thread walks the candidates in queue order until the smallest no longer fits.
+constexpr int LB_THREADS = 1024, LB_ITEMS = 4;
+constexpr uint32_t LB_MAX = LB_THREADS * LB_ITEMS;
+
+__global__ void __launch_bounds__(LB_THREADS)
+k_sah_level(Dec* __restrict__ dec, uint32_t n_lvl, uint32_t* __restrict__ used, const uint32_t* __restrict__ cap,
+            uint32_t* __restrict__ io, uint32_t* __restrict__ child_slot, uint32_t* __restrict__ ref_off,
+            uint32_t* __restrict__ leaf_off)
+{
+    __shared__ uint32_t sh[LB_THREADS / 32 + 1];
+    __shared__ uint32_t s_need[LB_MAX];  // the candidates' requests, REFUSED where the walk refuses
+    __shared__ uint32_t s_min, s_max, s_stop;
+    constexpr uint32_t REFUSED = 0xffffffffu;
+    const uint32_t tid = threadIdx.x, i0 = tid * LB_ITEMS;
+    if (tid == 0) { s_min = 0xffffffffu; s_max = 0u; }
+    int kind[LB_ITEMS];
+    uint32_t nd[LB_ITEMS], sp = 0, sum = 0, mn = 0xffffffffu;
+#pragma unroll
+    for (int r = 0; r < LB_ITEMS; r++)
+    {
+        kind[r] = K_LEAF;
+        nd[r] = 0;
+        if (i0 + r < n_lvl)
+        {
+            kind[r] = dec[i0 + r].kind;
+            if (kind[r] == K_SPATIAL)
+            {
+                nd[r] = dec[i0 + r].right + dec[i0 + r].straddle;
+                mn = min(mn, nd[r]);
+                sum += nd[r];
+                sp++;
+            }
+        }
+    }
+    uint32_t n_sp;
+    const uint32_t first = block_excl_scan<LB_THREADS>(sp, sh, &n_sp);
+    if (n_sp > 0)  // (the same for all threads)
+    {
+        const uint32_t all = block_sum<LB_THREADS>(sum, sh);  // (a level's references fit 32 bits)
+        mn = __reduce_min_sync(0xffffffffu, mn);
+        if ((tid & 31u) == 0 && mn != 0xffffffffu) { atomicMin(&s_min, mn); }
+        __syncthreads();
+        const uint32_t used0 = used[0];
+        const uint64_t cap0 = cap[0];
+        uint32_t stop = n_sp;  // candidates from here on are refused
+        if ((uint64_t)used0 + all <= cap0)
+        {
+            __syncthreads();
+            if (tid == 0) { used[0] = used0 + all; io[1] += n_sp; }
+        }
+        else if ((uint64_t)used0 + s_min > cap0)
+        {
+            stop = 0;
+            if (tid == 0) { io[2] += n_sp; }
+        }
+        else
+        {
+            uint32_t j = first;
+#pragma unroll
+            for (int r = 0; r < LB_ITEMS; r++)
+            {
+                if (kind[r] == K_SPATIAL) { s_need[j++] = nd[r]; }
+            }
+            __syncthreads();
+            if (tid == 0)
+            {
+                uint64_t u = used0;
+                uint32_t granted = 0;
+                for (j = 0; j < n_sp && u + s_min <= cap0; j++)
+                {
+                    if (u + s_need[j] > cap0) { s_need[j] = REFUSED; }
+                    else { u += s_need[j]; granted++; }
+                }
+                used[0] = (uint32_t)u;
+                io[1] += granted;
+                io[2] += n_sp - granted;
+                s_stop = j;
+            }
+            __syncthreads();
+            stop = s_stop;
+        }
+        const bool walked = stop > 0 && (uint64_t)used0 + all > cap0;
+        uint32_t j = first;
+#pragma unroll
+        for (int r = 0; r < LB_ITEMS; r++)
+        {
+            if (kind[r] != K_SPATIAL) { continue; }
+            if (j >= stop || (walked && s_need[j] == REFUSED))
+            {
+                // the saved object split (or a leaf) in place of the refused spatial split
+                Dec& d = dec[i0 + r];
+                kind[r] = d.fb_kind;
+                d.kind = kind[r]; d.pre_spatial = 1;
+                d.axis = d.oaxis; d.bin = d.obin; d.cmin = d.ocmin; d.scale = d.oscale;
+            }
+            j++;
+        }
+    }
+    uint32_t v[3][LB_ITEMS], tot3[3] = { 0, 0, 0 }, nleaf = 0, bmax = 0;
+#pragma unroll
+    for (int r = 0; r < LB_ITEMS; r++)
+    {
+        v[0][r] = v[1][r] = v[2][r] = 0;
+        if (i0 + r < n_lvl)
+        {
+            const Dec& d = dec[i0 + r];
+            const uint32_t n = d.n;
+            if (kind[r] == K_LEAF) { v[2][r] = n; nleaf++; }
+            else if (kind[r] == K_OBJECT)
+            {
+                v[0][r] = 2;
+                v[1][r] = n;
+                bmax = max(bmax, max(d.oleft, n - d.oleft));
+            }
+            else
+            {
+                v[0][r] = 2;
+                v[1][r] = n + d.straddle;
+                bmax = max(bmax, max(n - d.right, d.right + d.straddle));
+            }
+        }
+        for (int a = 0; a < 3; a++) { tot3[a] += v[a][r]; }
+    }
+    uint32_t run[3], tot[3];
+#pragma unroll
+    for (int a = 0; a < 3; a++) { run[a] = block_excl_scan<LB_THREADS>(tot3[a], sh, &tot[a]); }
+    nleaf = block_sum<LB_THREADS>(nleaf, sh);
+    bmax = __reduce_max_sync(0xffffffffu, bmax);
+    if ((tid & 31u) == 0 && bmax) { atomicMax(&s_max, bmax); }
+#pragma unroll
+    for (int r = 0; r < LB_ITEMS; r++)
+    {
+        if (i0 + r < n_lvl) { child_slot[i0 + r] = run[0]; ref_off[i0 + r] = run[1]; leaf_off[i0 + r] = run[2]; }
+        for (int a = 0; a < 3; a++) { run[a] += v[a][r]; }
+    }
+    __syncthreads();
+    if (tid == 0)
+    {
+        for (int a = 0; a < 3; a++) { io[3 + a] = tot[a]; }
+        io[6] += nleaf;
+        io[7] = 0u; io[10] = s_max;
+        io[11] = 0u; io[13] = 0u; io[14] = 0u; io[15] = 0xffffffffu; io[16] = 0u; io[17] = 0u;
+    }
+}
+
 __device__ __forceinline__ void set_node(LvlNode& L, uint32_t off, uint32_t cnt, uint32_t out, uint32_t root,
                                          uint32_t root_first, const box3& b)
 {
@@ -2749,10 +2897,16 @@ k_sah_merge(const LvlNode* __restrict__ cont, uint32_t n_cont, const SahRoot* __
     }
 }
 
-__global__ void __launch_bounds__(SBLK) k_sah_up(OutNode* __restrict__ out, uint32_t b, uint32_t e)
+// Consecutive levels of the output nodes: level l is nodes at[l] .. at[l + 1] - 1.
+constexpr uint32_t SPAN_LEVELS = 32, SPAN_NODES = 1024;
+struct LevelSpan
 {
-    const uint32_t i = b + blockIdx.x * SBLK + threadIdx.x;
-    if (i >= e) { return; }
+    uint32_t n;
+    uint32_t at[SPAN_LEVELS + 1];
+};
+
+__device__ __forceinline__ void out_up(OutNode* out, uint32_t i)
+{
     OutNode& o = out[i];
     if (o.is_leaf) { o.size = 1; o.refs = o.b; }
     else
@@ -2762,10 +2916,8 @@ __global__ void __launch_bounds__(SBLK) k_sah_up(OutNode* __restrict__ out, uint
     }
 }
 
-__global__ void __launch_bounds__(SBLK) k_sah_down(OutNode* __restrict__ out, uint32_t b, uint32_t e)
+__device__ __forceinline__ void out_down(OutNode* out, uint32_t i)
 {
-    const uint32_t i = b + blockIdx.x * SBLK + threadIdx.x;
-    if (i >= e) { return; }
     const OutNode o = out[i];
     if (o.is_leaf) { return; }
     OutNode& l = out[o.a];
@@ -2774,6 +2926,23 @@ __global__ void __launch_bounds__(SBLK) k_sah_down(OutNode* __restrict__ out, ui
     l.toff = o.toff;
     r.pre = o.pre + 1 + l.size;
     r.toff = o.toff + l.refs;
+}
+
+// Subtree sizes (UP: the deepest level first) or pre-order slots and triangle offsets. A level of many
+// nodes takes a launch of its own; levels of at most SPAN_NODES nodes, where a launch takes longer than its
+// work, are walked by one block.
+template <bool UP>
+__global__ void __launch_bounds__(SPAN_NODES) k_sah_walk(OutNode* out, const __grid_constant__ LevelSpan S)
+{
+    for (uint32_t k = 0; k < S.n; k++)
+    {
+        const uint32_t l = UP ? S.n - 1 - k : k;
+        for (uint32_t i = S.at[l] + blockIdx.x * blockDim.x + threadIdx.x; i < S.at[l + 1]; i += gridDim.x * blockDim.x)
+        {
+            if (UP) { out_up(out, i); } else { out_down(out, i); }
+        }
+        __syncthreads();
+    }
 }
 
 __global__ void __launch_bounds__(SBLK)
@@ -3037,14 +3206,22 @@ int sah_build(rt_bvh* B, const rt_build_cfg& cfg, const SahInput& in, cudaStream
             count_launch(6);
         }
         const uint32_t n_tiles = (n_cur + SO_TILE - 1) / SO_TILE;
-        k_sah_need<<<(n_cur + NEED_THREADS - 1) / NEED_THREADS, NEED_THREADS, 0, st>>>(S.sah_dec.as<Dec>(), lv_cur, d_roots,
-                                                                                        n_cur, n_budget, d_need, io);
-        k_sah_grant<<<1, 1024, 0, st>>>(S.sah_dec.as<Dec>(), lv_cur, d_roots, n_cur, n_budget, d_used, d_used + n_budget,
-                                        d_need, io, leaf_offs, d_desc, n_tiles);
-        k_sah_offsets<<<n_tiles, SO_THREADS, 0, st>>>(S.sah_dec.as<Dec>(), n_cur, d_desc,
-                                                      reinterpret_cast<uint32_t*>(d_desc + 3 * (size_t)n_tiles), io,
-                                                      child_slot, ref_offs, leaf_offs);
-        count_launch(3);
+        if (n_budget == 1 && n_cur <= LB_MAX)
+        {
+            k_sah_level<<<1, LB_THREADS, 0, st>>>(S.sah_dec.as<Dec>(), n_cur, d_used, d_used + 1, io, child_slot, ref_offs, leaf_offs);
+            count_launch();
+        }
+        else
+        {
+            k_sah_need<<<(n_cur + NEED_THREADS - 1) / NEED_THREADS, NEED_THREADS, 0, st>>>(S.sah_dec.as<Dec>(), lv_cur, d_roots,
+                                                                                            n_cur, n_budget, d_need, io);
+            k_sah_grant<<<1, 1024, 0, st>>>(S.sah_dec.as<Dec>(), lv_cur, d_roots, n_cur, n_budget, d_used, d_used + n_budget,
+                                            d_need, io, leaf_offs, d_desc, n_tiles);
+            k_sah_offsets<<<n_tiles, SO_THREADS, 0, st>>>(S.sah_dec.as<Dec>(), n_cur, d_desc,
+                                                          reinterpret_cast<uint32_t*>(d_desc + 3 * (size_t)n_tiles), io,
+                                                          child_slot, ref_offs, leaf_offs);
+            count_launch(3);
+        }
         if (int e = check_launch("sah eval")) { return e; }
         RT_CUDA(cudaMemcpyAsync(io_h, io, 64, cudaMemcpyDeviceToHost, st));
         RT_CUDA(cudaStreamSynchronize(st));
@@ -3104,15 +3281,25 @@ int sah_build(rt_bvh* B, const rt_build_cfg& cfg, const SahInput& in, cudaStream
         depth++;
     }
     // subtree sizes bottom-up, then pre-order slots and triangle offsets top-down
-    for (size_t l = levels.size(); l-- > 0;)
-    {
-        const auto& L = levels[l];
-        if (L.second > L.first) { k_sah_up<<<nblk(L.second - L.first), SBLK, 0, st>>>(out, L.first, L.second); count_launch(); }
-    }
+    std::vector<LevelSpan> spans;
     for (const auto& L : levels)
     {
-        if (L.second > L.first) { k_sah_down<<<nblk(L.second - L.first), SBLK, 0, st>>>(out, L.first, L.second); count_launch(); }
+        const bool few = L.second - L.first <= SPAN_NODES;
+        if (few && !spans.empty() && spans.back().n < SPAN_LEVELS && spans.back().at[spans.back().n] == L.first &&
+            spans.back().at[1] - spans.back().at[0] <= SPAN_NODES)
+        {
+            spans.back().at[++spans.back().n] = L.second;
+        }
+        else { spans.push_back({ 1, { L.first, L.second } }); }
     }
+    const auto walk = [&](auto kernel, const LevelSpan& L) {
+        const uint32_t nodes = L.at[1] - L.at[0];
+        if (nodes > SPAN_NODES) { kernel<<<nblk(nodes), SBLK, 0, st>>>(out, L); }
+        else { kernel<<<1, SPAN_NODES, 0, st>>>(out, L); }
+        count_launch();
+    };
+    for (size_t l = spans.size(); l-- > 0;) { walk(k_sah_walk<true>, spans[l]); }
+    for (const LevelSpan& L : spans) { walk(k_sah_walk<false>, L); }
     k_sah_root_weights<<<nblk(nr), SBLK, 0, st>>>(d_roots, nr, root_out, out, in.wnode, in.wtri);
     count_launch();
     if (int e = check_launch("sah finish")) { return e; }

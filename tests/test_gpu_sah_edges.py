@@ -6,6 +6,7 @@ import pytest
 
 import rtb200
 from rtb200 import scenes
+from oracle import make_cfg as orc_make_cfg
 from test_gpu_build import assert_same_tree, orc_cfg
 
 pytestmark = pytest.mark.gpu
@@ -50,3 +51,16 @@ def test_fans(orc, preset, count, blades):
     ref = orc.build(v, t, orc_cfg(preset))
     assert_same_tree(b.download(), ref, f"{preset}/{count}x{blades}")
     assert b.stats()["spatial_taken"] == int(ref.stats[0])
+
+
+@pytest.mark.parametrize("mult", [1.0, 1.01, 1.1, 1.5])
+@pytest.mark.parametrize("count,blades", [(12, 24), (300, 33), (900, 40)])
+def test_budgets(orc, count, blades, mult):
+    """Reference budgets that no, some, or all spatial splits of a level fit, on levels within one block's reach
+    (4,096 nodes) and beyond it."""
+    v, t = fans(count, blades, 5)
+    b = rtb200.Bvh.build(v, t, rtb200.make_cfg("sah4", spatial_mult=mult))
+    ref = orc.build(v, t, orc_make_cfg(**{**rtb200.PRESETS["sah4"], "spatial_mult": mult}))
+    assert_same_tree(b.download(), ref, f"{count}x{blades}/{mult}")
+    st = b.stats()
+    assert st["spatial_taken"] == int(ref.stats[0]) and st["spatial_refused"] == int(ref.stats[1])
