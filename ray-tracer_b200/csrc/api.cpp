@@ -7,6 +7,7 @@
 #include <algorithm>
 #include <atomic>
 #include <cmath>
+#include <condition_variable>
 #include <cstdio>
 #include <cstring>
 #include <fstream>
@@ -113,6 +114,42 @@ using namespace rtb;
 
 static cudaStream_t pick(void* s) { return s ? static_cast<cudaStream_t>(s) : default_stream(); }
 
+// Words of page-locked host memory that trace kernels report an overflow in: a call takes one and gives
+// it back when its stream is done; with all taken it waits for one.
+class TraceStatus
+{
+    static constexpr int N = 64;
+    inline static std::mutex              mu_;
+    inline static std::condition_variable back_;
+    inline static volatile uint32_t*      words_ = nullptr;
+    inline static uint64_t                free_ = ~0ull;
+    int                                   slot_ = -1;
+
+public:
+    uint32_t* take()
+    {
+        std::unique_lock<std::mutex> lk(mu_);
+        if (!words_)
+        {
+            void* p = nullptr;
+            if (cudaHostAlloc(&p, N * 4, cudaHostAllocPortable | cudaHostAllocMapped) != cudaSuccess) { cudaGetLastError(); return nullptr; }
+            words_ = static_cast<volatile uint32_t*>(p);
+        }
+        back_.wait(lk, [] { return free_ != 0; });
+        slot_ = __builtin_ctzll(free_);
+        free_ &= free_ - 1;
+        words_[slot_] = 0;
+        return const_cast<uint32_t*>(words_ + slot_);
+    }
+    uint32_t read() const { return words_[slot_]; }
+    ~TraceStatus()
+    {
+        if (slot_ < 0) { return; }
+        std::lock_guard<std::mutex> lk(mu_);
+        free_ |= 1ull << slot_;
+        back_.notify_one();
+    }
+};
 static void free_bvh(rt_bvh* b)
 {
     if (!b) { return; }
@@ -560,16 +597,13 @@ int rt_trace(const rt_bvh* b, const rt_ray* rays, rt_hit* hits, uint64_t n, uint
 {
     if (!b) { return fail(RT_E_NOT_LOADED, "BVH not loaded on trace()"); }
     if (n && (!rays || !hits)) { return fail(RT_E_INVALID, "null rays/hits"); }
-    rt_bvh* bm = const_cast<rt_bvh*>(b);
-    if (bm->s.status.ensure(64)) { return RT_E_CUDA; }
     cudaStream_t st = pick(stream);
-    uint32_t* status = bm->s.status.as<uint32_t>() + 8;
-    RT_CUDA(cudaMemsetAsync(status, 0, 4, st));
-    if (int e = rtb::trace(b, rays, hits, n, flags, st, status)) { return e; }
-    uint32_t hs = 0;
-    RT_CUDA(cudaMemcpyAsync(&hs, status, 4, cudaMemcpyDeviceToHost, st));
+    TraceStatus status;
+    uint32_t* word = status.take();
+    if (!word) { return fail(RT_E_CUDA, "no page-locked memory for a trace's status"); }
+    if (int e = rtb::trace(b, rays, hits, n, flags, st, word)) { return e; }
     RT_CUDA(cudaStreamSynchronize(st));
-    if (hs & ST_STACK) { return fail(RT_E_STACK, "a ray overflowed the 64-entry traversal stack"); }
+    if (status.read() & ST_STACK) { return fail(RT_E_STACK, "a ray overflowed the 64-entry traversal stack"); }
     return RT_OK;
 }
 

@@ -602,7 +602,7 @@ int launch_paths(PathFn fn, const TraceCtx& T, const PathJob& J, uint32_t* count
 {
     const size_t smem = (size_t)(block / 32) * sizeof(PathShare);
     const int per_sm = blocks_per_sm(reinterpret_cast<const void*>(fn), (int)block, smem);
-    // few items are spread over the resident warps (as few rays are by trace_launch)
+    // few items are spread over the resident warps (as few rays are by trace)
     const uint64_t warps = (uint64_t)device_sm_count() * (uint64_t)per_sm * (block / 32);
     const uint64_t per_warp = std::min<uint64_t>(32, (J.n + warps - 1) / warps);
     const uint64_t grid = std::min<uint64_t>((uint64_t)device_sm_count() * (uint64_t)per_sm,

@@ -275,21 +275,7 @@ int make_traversal_layout(rt_bvh* b, cudaStream_t st);
 int launch_traversal_layout(rt_bvh* b, cudaStream_t st, uint32_t max_nodes, uint32_t max_tris, const uint32_t* d_counts,
                             uint32_t* vstatus, bool tripos_ready = false, bool gnodes_ready = false);
 int trace(const rt_bvh* b, const rt_ray* d_rays, rt_hit* d_hits, uint64_t n, uint32_t flags, cudaStream_t st,
-          uint32_t* d_status);
-// Launch options of the persistent trace kernel: block size (0: default), stack entries
-// (32 or 64; 32 only for closest hits), and per-ray subtree roots (roots[rscene[i]], device).
-struct TraceRoot;
-struct TraceLaunch
-{
-    int              block = 0;
-    int              stack = 64;
-    const TraceRoot* roots = nullptr;
-    const uint32_t*  rscene = nullptr;
-};
-// Launches the persistent trace kernel; n_dev (optional) holds the ray count on the device.
-// d_counter must be zero on entry.
-int trace_launch(const rt_bvh* b, const void* d_rays, void* d_hits, uint64_t n, const uint32_t* n_dev, uint32_t flags,
-                 cudaStream_t st, uint32_t* d_status, unsigned long long* d_counter, const TraceLaunch& opt);
+          uint32_t* status);  // a word the kernel can write that is 0 on entry; ST_STACK after an overflow
 // traverse.cu: resident blocks per SM of a kernel (cached)
 int blocks_per_sm(const void* fn, int block, size_t smem);
 // render.cu

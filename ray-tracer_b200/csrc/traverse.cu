@@ -147,21 +147,18 @@ __device__ __forceinline__ void write_hit(const TraceCtx& T, float4* __restrict_
         h1 = make_float4(nrm.x, nrm.y, nrm.z, 0.f);
         flags = RT_HIT_FLAG_HIT;
     }
-    if (overflow) { flags |= RT_HIT_FLAG_OVERFLOW; atomicOr(status, ST_STACK); }
+    if (overflow) { flags |= RT_HIT_FLAG_OVERFLOW; *static_cast<volatile uint32_t*>(status) = ST_STACK; }
     h1.w = __uint_as_float(flags);
     hits[2 * ri] = h0;
     hits[2 * ri + 1] = h1;
 }
 
-// rt_ray records in, rt_hit records out (two 128-bit accesses each). n_dev, when set, holds
-// the ray count on the device (the wavefront path tracer's queue length). ROOTS: ray i
-// traces the subtree roots[rscene[i]] (a scene of a batched build). A warp holds at most
-// `per_warp` rays at a time.
-template <int MODE, int STK, bool ROOTS>
+// rt_ray records in, rt_hit records out (two 128-bit accesses each). A warp holds at most `per_warp`
+// rays at a time; without a counter it traces those of its own index only. status: a word of the host's.
+template <int MODE>
 __global__ void __launch_bounds__(256, 4)
-k_trace(TraceCtx T, const float4* __restrict__ rays, float4* __restrict__ hits, uint64_t n, const uint32_t* __restrict__ n_dev,
-        unsigned long long* __restrict__ counter, uint32_t* __restrict__ status, const TraceRoot* __restrict__ roots,
-        const uint32_t* __restrict__ rscene, int per_warp)
+k_trace(TraceCtx T, const float4* __restrict__ rays, float4* __restrict__ hits, uint64_t n,
+        unsigned long long* __restrict__ counter, uint32_t* __restrict__ status, int per_warp)
 {
     extern __shared__ __align__(16) unsigned char smem[];
     constexpr unsigned FULL = 0xffffffffu;
@@ -169,10 +166,9 @@ k_trace(TraceCtx T, const float4* __restrict__ rays, float4* __restrict__ hits, 
     const int lane = (int)(threadIdx.x & 31u);
     const unsigned lanes = per_warp >= 32 ? FULL : (1u << per_warp) - 1u;
     const int refill = per_warp >= 32 ? REFILL : (per_warp + 1) / 2;
-    if (n_dev) { n = *n_dev; }
     const bool odd_tree = *T.odd != 0u;
-    LaneTrace<MODE, STK> L;
-    uint2 stk[STK];
+    LaneTrace<MODE, STACK> L;
+    uint2 stk[STACK];
     L.live = false;
     bool pending = false, more = true;  // this lane has a result to write; rays are left
     for (;;)
@@ -188,16 +184,24 @@ k_trace(TraceCtx T, const float4* __restrict__ rays, float4* __restrict__ hits, 
             }
             if (!more) { break; }
             unsigned long long base = 0;
-            if (lane == 0) { base = atomicAdd(counter, (unsigned long long)__popc(idle)); }
-            base = __shfl_sync(FULL, base, 0);
-            if (base + __popc(idle) >= n) { more = false; }
+            if (counter)
+            {
+                if (lane == 0) { base = atomicAdd(counter, (unsigned long long)__popc(idle)); }
+                base = __shfl_sync(FULL, base, 0);
+                if (base + __popc(idle) >= n) { more = false; }
+            }
+            else
+            {
+                base = ((uint64_t)blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5)) * (uint64_t)per_warp;
+                more = false;
+            }
             if ((idle >> lane) & 1u)
             {
                 const uint64_t ri = base + __popc(idle & ((1u << lane) - 1u));
                 if (ri < n)
                 {
                     const float4 r0 = rays[2 * ri], r1 = rays[2 * ri + 1];
-                    if (ROOTS) { L.start(S, roots[rscene[ri]], r0, r1, odd_tree); } else { L.start(S, *T.root, r0, r1, odd_tree); }
+                    L.start(S, *T.root, r0, r1, odd_tree);
                     S.id[lane] = ri;
                     pending = true;
                 }
@@ -205,22 +209,19 @@ k_trace(TraceCtx T, const float4* __restrict__ rays, float4* __restrict__ hits, 
             __syncwarp();
             continue;
         }
-        warp_walk<MODE, STK>(L, stk, T, S, more ? lanes : 0u, refill);
-        warp_leaves<MODE, STK>(L, stk, T, S);
+        warp_walk<MODE, STACK>(L, stk, T, S, more ? lanes : 0u, refill);
+        warp_leaves<MODE, STACK>(L, stk, T, S);
     }
 }
 
 // The 8-wide layout's kernel: each warp claims 32 rays at a time until the batch is exhausted.
-template <int MODE, bool ROOTS>
+template <int MODE>
 __global__ void __launch_bounds__(256)
 k_trace_wide(TraceCtx T, const float4* __restrict__ rays, float4* __restrict__ hits, uint64_t n,
-             const uint32_t* __restrict__ n_dev, unsigned long long* __restrict__ counter, uint32_t* __restrict__ status,
-             const TraceRoot* __restrict__ roots, const uint32_t* __restrict__ rscene, int)
+             unsigned long long* __restrict__ counter, uint32_t* __restrict__ status, int)
 {
     const int lane = threadIdx.x & 31;
-    if (n_dev) { n = *n_dev; }
-    TraceRoot R0;
-    if (!ROOTS) { R0 = *T.root; }
+    const TraceRoot R = *T.root;
     for (;;)
     {
         unsigned long long base = 0;
@@ -230,40 +231,21 @@ k_trace_wide(TraceCtx T, const float4* __restrict__ rays, float4* __restrict__ h
         const uint64_t ri = base + (uint64_t)lane;
         if (ri >= n) { continue; }
         const float4 r0 = rays[2 * ri], r1 = rays[2 * ri + 1];
-        const TraceRoot& R = ROOTS ? roots[rscene[ri]] : R0;
         const THit H = trace_ray_wide<MODE, STACK>(T, R, mk3(r0.x, r0.y, r0.z), mk3(r1.x, r1.y, r1.z), r0.w, r1.w);
         write_hit(T, hits, ri, H.hit, H.overflow, H.t, H.u, H.v, H.tri, status);
     }
 }
 
-using TraceFn = void (*)(TraceCtx, const float4*, float4*, uint64_t, const uint32_t*, unsigned long long*, uint32_t*,
-                         const TraceRoot*, const uint32_t*, int);
+using TraceFn = void (*)(TraceCtx, const float4*, float4*, uint64_t, unsigned long long*, uint32_t*, int);
 
-TraceFn trace_fn(uint32_t flags, int stack, bool roots, bool wide)
+TraceFn trace_fn(uint32_t flags, bool wide)
 {
-    if (wide)
-    {
-        if (roots) { return (flags & 3u) == 0 ? k_trace_wide<0, true> : nullptr; }
-        switch (flags & 3u)
-        {
-        case 0: return k_trace_wide<0, false>;
-        case 1: return k_trace_wide<1, false>;
-        case 2: return k_trace_wide<2, false>;
-        default: return k_trace_wide<3, false>;
-        }
-    }
-    if (stack <= 32)
-    {
-        if (roots) { return k_trace<0, 32, true>; }
-        return (flags & 3u) == 0 ? k_trace<0, 32, false> : nullptr;
-    }
-    if (roots) { return k_trace<0, STACK, true>; }
     switch (flags & 3u)
     {
-    case 0: return k_trace<0, STACK, false>;
-    case 1: return k_trace<1, STACK, false>;
-    case 2: return k_trace<2, STACK, false>;
-    default: return k_trace<3, STACK, false>;
+    case 0: return wide ? k_trace_wide<0> : k_trace<0>;
+    case 1: return wide ? k_trace_wide<1> : k_trace<1>;
+    case 2: return wide ? k_trace_wide<2> : k_trace<2>;
+    default: return wide ? k_trace_wide<3> : k_trace<3>;
     }
 }
 
@@ -344,34 +326,6 @@ int make_traversal_layout(rt_bvh* B, cudaStream_t st)
     return RT_OK;
 }
 
-int trace_launch(const rt_bvh* B, const void* d_rays, void* d_hits, uint64_t n, const uint32_t* n_dev, uint32_t flags,
-                 cudaStream_t st, uint32_t* d_status, unsigned long long* d_counter, const TraceLaunch& opt)
-{
-    const TraceFn fn = trace_fn(flags, opt.stack, opt.roots != nullptr, B->trace_wide);
-    if (!fn) { return fail(RT_E_INVALID, "no trace kernel for this mode and stack depth"); }
-    const int block = opt.block > 0 ? opt.block : TBLK;
-    if (block % 32 || block > 256) { return fail(RT_E_INVALID, "trace block must be a multiple of 32, at most 256"); }
-    const size_t smem = B->trace_wide ? 0 : (size_t)(block / 32) * sizeof(WarpShare);
-    uint64_t grid = (uint64_t)device_sm_count() * (uint64_t)blocks_per_sm(reinterpret_cast<const void*>(fn), block, smem);
-    int per_warp = 32;
-    if (!n_dev)
-    {
-        // Few rays are spread over the resident warps, down to one ray per warp: the lanes without
-        // a ray still test its leaves' triangles (1,000 rays, 5,120-triangle hybrid tree: see
-        // trace_warp.cuh).
-        const uint64_t warps = grid * (uint64_t)(block / 32);
-        if (!B->trace_wide && n < warps * 32) { per_warp = (int)std::max<uint64_t>(1, (n + warps - 1) / warps); }
-        const uint64_t want = (n + (uint64_t)per_warp * (block / 32) - 1) / ((uint64_t)per_warp * (block / 32));
-        if (grid > want) { grid = want; }
-    }
-    if (grid == 0) { return RT_OK; }
-    const TraceCtx T = make_trace_ctx(B);
-    fn<<<(uint32_t)grid, block, smem, st>>>(T, static_cast<const float4*>(d_rays), static_cast<float4*>(d_hits), n, n_dev,
-                                            d_counter, d_status, opt.roots, opt.rscene, per_warp);
-    count_launch();
-    return check_launch("trace");
-}
-
 int launch_scene_roots(rt_bvh* B, uint32_t S, const uint32_t* d_counts, uint32_t* status, cudaStream_t st)
 {
     k_scene_roots<<<(S + 127) / 128, 128, 0, st>>>(B->nodes.as<rt_bvh_node>(), B->scene_info.as<uint32_t>(), S, d_counts,
@@ -410,15 +364,30 @@ int tree_depth(rt_bvh* B, cudaStream_t st, uint32_t* depth)
 }
 
 int trace(const rt_bvh* B, const rt_ray* d_rays, rt_hit* d_hits, uint64_t n, uint32_t flags, cudaStream_t st,
-          uint32_t* d_status)
+          uint32_t* status)
 {
     if (n == 0) { return RT_OK; }
     if (((uintptr_t)d_rays & 15) || ((uintptr_t)d_hits & 15)) { return fail(RT_E_INVALID, "rays/hits must be 16-byte aligned"); }
     rt_bvh* Bm = const_cast<rt_bvh*>(B);
     if (Bm->trace_status.ensure(64)) { return RT_E_CUDA; }
-    unsigned long long* counter = Bm->trace_status.as<unsigned long long>();
-    RT_CUDA(cudaMemsetAsync(counter, 0, 8, st));
-    return trace_launch(B, d_rays, d_hits, n, nullptr, flags, st, d_status, counter, TraceLaunch{});
+    const TraceFn fn = trace_fn(flags, B->trace_wide);
+    constexpr uint64_t WPB = TBLK / 32;
+    const size_t smem = B->trace_wide ? 0 : WPB * sizeof(WarpShare);
+    uint64_t grid = (uint64_t)device_sm_count() * (uint64_t)blocks_per_sm(reinterpret_cast<const void*>(fn), TBLK, smem);
+    // Few rays are spread over the resident warps, down to one ray per warp: the lanes without
+    // a ray still test its leaves' triangles. Every warp then has its rays at once, so they are
+    // assigned by index: no counter to clear before the launch and to wait for at its start.
+    const uint64_t warps = grid * WPB;
+    const bool few = !B->trace_wide && n <= warps * 32;
+    const uint64_t per_warp = few ? std::max<uint64_t>(1, (n + warps - 1) / warps) : 32;
+    grid = std::min(grid, (n + per_warp * WPB - 1) / (per_warp * WPB));
+    unsigned long long* counter = few ? nullptr : Bm->trace_status.as<unsigned long long>();
+    if (counter) { RT_CUDA(cudaMemsetAsync(counter, 0, 8, st)); }
+    const TraceCtx T = make_trace_ctx(B);
+    fn<<<(uint32_t)grid, TBLK, smem, st>>>(T, reinterpret_cast<const float4*>(d_rays), reinterpret_cast<float4*>(d_hits), n, counter,
+                                           status, (int)per_warp);
+    count_launch();
+    return check_launch("trace");
 }
 
 } // namespace rtb

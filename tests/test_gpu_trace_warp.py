@@ -3,6 +3,7 @@ a warp and below one ray per resident warp, leaves of one to hundreds of triangl
 vertices that are not finite. Bar: bit-equal to the oracle's restatement of bvh::trace."""
 import numpy as np
 import pytest
+import torch
 
 import rtb200
 from oracle import Baked
@@ -67,3 +68,26 @@ def test_vertices_that_are_not_finite(orc, preset):
     nodes, tris, verts = b.download()
     rays = rays_for(np.nan_to_num(v), 8192, seed=10)
     compare(b.trace(rays), orc.trace(Baked(nodes, tris, verts), rays, threads=8), preset)
+
+
+def test_traces_from_several_threads():
+    """More calls at a time than there are status words, on streams of their own."""
+    import threading
+    v, t = scenes.soup(3000, seed=8, lo=1e-2, hi=1e-1)
+    b = rtb200.Bvh.build(v, t, "hybrid")
+    rays = torch.from_numpy(scenes.incoherent_rays(777, [0, 0, 0], [1, 1, 1], seed=4)).cuda()
+    want, got = b.trace(rays).cpu(), [None] * 80
+
+    def work(k):
+        with torch.cuda.stream(torch.cuda.Stream()):
+            for _ in range(3):
+                h = b.trace(rays)
+            got[k] = h.cpu()
+
+    torch.cuda.synchronize()
+    threads = [threading.Thread(target=work, args=(k,)) for k in range(len(got))]
+    for x in threads:
+        x.start()
+    for x in threads:
+        x.join()
+    assert all(g is not None and torch.equal(g.view(torch.int32), want.view(torch.int32)) for g in got)
