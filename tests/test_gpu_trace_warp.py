@@ -91,3 +91,31 @@ def test_traces_from_several_threads():
     for x in threads:
         x.join()
     assert all(g is not None and torch.equal(g.view(torch.int32), want.view(torch.int32)) for g in got)
+
+
+@pytest.mark.parametrize("n", [1, 700, 160000])
+def test_stack_overflow_is_reported(n):
+    """A chain deeper than the 64-entry stack: the call reports it (code 5), and only that call."""
+    depth = 80
+    nodes = np.zeros(2 * depth + 1, rtb200.NODE_DTYPE)
+    nodes["bmin"][:, :3], nodes["bmax"][:, :3] = 0.0, 1.0
+    for i in range(depth):  # inner nodes 0 .. depth - 1, each with the next one and a leaf in an equal box
+        nodes["a"][i], nodes["b"][i] = i + 1, 2 * depth - i
+    nodes["is_leaf"][depth:] = 1
+    nodes["b"][depth:] = 1
+    verts = np.zeros((3, 6), np.float32)
+    verts[:, :3] = [[0, 0, 0.5], [0, 1, 0.5], [1, 0, 0.5]]
+    verts[:, 5] = 1.0
+    b = rtb200.Bvh.from_arrays(nodes, np.array([[0, 1, 2]], np.uint32), verts)
+    rays = torch.zeros(n, 8, device="cuda")
+    rays[:, 0:3] = torch.tensor([0.2, 0.2, -1.0])
+    rays[:, 6], rays[:, 7] = 1.0, float("inf")
+    off = rays.clone()
+    off[:, 0] = 9.0
+    hits = torch.empty_like(rays)
+
+    def call(r):
+        torch.cuda.synchronize()
+        return rtb200.lib().rt_trace(b.h, r.data_ptr(), hits.data_ptr(), n, 0, None)
+
+    assert [call(rays), call(off), call(rays), call(off)] == [5, 0, 5, 0]
