@@ -409,13 +409,13 @@ __device__ __forceinline__ void warp_add3(float* __restrict__ dst, uint32_t key,
 // REC: the forward pass keeps the triangles of its path, and the replay needs no more: throughput and
 // gradients follow from them (roulette's survivors are the paths with a next triangle). Without it
 // the replay traces the path again, which half of the time went to: 512 x 512 x 32, 50,000
-// triangles, 4 bounces 106 -> 57 ms, 200,000 triangles, 5 bounces 201 -> 105 ms. Paths of more than
+// triangles, 4 bounces 106 -> 54 ms, 200,000 triangles, 5 bounces 201 -> 101 ms. Paths of more than
 // REC_BOUNCES bounces are traced twice.
 //
 // Why a thread per pixel, per-lane traversal and five blocks per SM: a material's emission gradient
 // is one 32-bit sum of millions of terms, off by 1.5e-4 from the exact one at 512 x 512 x 32, and
-// where it ends up depends on which tiles are at work together. With this schedule it stays within 1.2e-5
-// of the path traced twice; warps that trace together as the renderer's do (31 ms) move it by 0.5-4e-5,
+// where it ends up depends on which tiles are at work together. With this schedule it is 0.3-1.2e-5 (1.9e-5
+// at most) from the paths traced twice, whose runs differ by 0.3-1.1e-5; warps that trace together as the renderer's do (31 ms) move it by 0.5-4e-5,
 // paths traced by k_paths and replayed by a kernel of their own (35 ms) or other numbers of blocks by up to 3e-4.
 template <bool REC>
 __global__ void __launch_bounds__(128, 5)

@@ -64,3 +64,11 @@ def test_budgets(orc, count, blades, mult):
     assert_same_tree(b.download(), ref, f"{count}x{blades}/{mult}")
     st = b.stats()
     assert st["spatial_taken"] == int(ref.stats[0]) and st["spatial_refused"] == int(ref.stats[1])
+
+
+@pytest.mark.parametrize("n", [65, 2000, 44000, 52000, 56000, 70000])
+def test_root_counts(orc, n):
+    """Hybrid bakes of one to some 1,500 SAH subtrees (one block orders up to 1,024)."""
+    v, t = scenes.soup(n, seed=n, lo=1e-3, hi=1e-1)
+    b = rtb200.Bvh.build(v, t, "hybrid")
+    assert_same_tree(b.download(), orc.build(v, t, orc_cfg("hybrid")), f"hybrid/{n}")
