@@ -97,6 +97,66 @@ int device_sm_count()
     return g_sms[d];
 }
 
+static cudaMemPool_t g_pools[64];  // (g_dev_mu)
+static std::atomic<int> g_handles{ 0 };
+
+static cudaMemPool_t scratch_pool()
+{
+    std::lock_guard<std::mutex> lk(g_dev_mu);
+    int d = 0;
+    if (cudaGetDevice(&d) != cudaSuccess || d < 0 || d >= 64) { return nullptr; }
+    if (!g_pools[d])
+    {
+        cudaMemPoolProps props;
+        std::memset(&props, 0, sizeof(props));
+        props.allocType = cudaMemAllocationTypePinned;
+        props.location.type = cudaMemLocationTypeDevice;
+        props.location.id = d;
+        cudaMemPool_t pool = nullptr;
+        if (cudaMemPoolCreate(&pool, &props) != cudaSuccess) { return nullptr; }
+        uint64_t kept = SCRATCH_KEPT;
+        int no = 0;  // a call never waits for another stream's to give memory back
+        if (cudaMemPoolSetAttribute(pool, cudaMemPoolAttrReleaseThreshold, &kept) != cudaSuccess ||
+            cudaMemPoolSetAttribute(pool, cudaMemPoolReuseAllowInternalDependencies, &no) != cudaSuccess)
+        {
+            cudaMemPoolDestroy(pool);
+            return nullptr;
+        }
+        g_pools[d] = pool;
+    }
+    return g_pools[d];
+}
+
+int CallScratch::get(size_t bytes, cudaStream_t st)
+{
+    const cudaMemPool_t pool = scratch_pool();
+    void* p = nullptr;
+    const cudaError_t e = pool ? cudaMallocFromPoolAsync(&p, bytes, pool, st) : cudaErrorMemoryAllocation;
+    if (e != cudaSuccess)
+    {
+        cudaGetLastError();
+        return fail(RT_E_CUDA, std::string("scratch of ") + std::to_string(bytes) + " bytes: " + cudaGetErrorString(e));
+    }
+    p_ = p;
+    st_ = st;
+    return RT_OK;
+}
+CallScratch::~CallScratch()
+{
+    if (p_ && cudaFreeAsync(p_, st_) != cudaSuccess) { cudaGetLastError(); }
+}
+
+HandleCount::HandleCount() { g_handles.fetch_add(1); }
+HandleCount::~HandleCount()
+{
+    if (g_handles.fetch_sub(1) != 1) { return; }
+    std::lock_guard<std::mutex> lk(g_dev_mu);
+    for (const cudaMemPool_t pool : g_pools)
+    {
+        if (pool && cudaMemPoolTrimTo(pool, 0) != cudaSuccess) { cudaGetLastError(); }
+    }
+}
+
 static int require_device()
 {
     int n = 0;

@@ -79,6 +79,30 @@ struct DevBuf
     template <typename T> T* as() const { return static_cast<T*>(p); }
 };
 
+// Device memory of one call, taken and given back in the order of the call's stream: calls on several
+// streams and host threads share none of it and do not wait for one another's. It comes from a pool
+// per device that keeps at most SCRATCH_KEPT bytes between calls, and none without a handle.
+constexpr uint64_t SCRATCH_KEPT = 512ull << 20;
+class CallScratch
+{
+    void*        p_ = nullptr;
+    cudaStream_t st_ = nullptr;
+
+public:
+    CallScratch() = default;
+    CallScratch(const CallScratch&) = delete;
+    CallScratch& operator=(const CallScratch&) = delete;
+    ~CallScratch();
+    int get(size_t bytes, cudaStream_t st);  // once; RT_E_CUDA, with nothing held, where there is no such memory
+    template <typename T> T* as() const { return static_cast<T*>(p_); }
+};
+// A member of every handle: the last one to go empties the pools.
+struct HandleCount
+{
+    HandleCount();
+    ~HandleCount();
+};
+
 // Per-device default stream and the current device's properties.
 cudaStream_t default_stream();
 int          device_sm_count();
@@ -214,6 +238,7 @@ struct rt_bvh
     uint32_t     n_wide = 0;
     uint32_t     stats[8] = {0, 0, 0, 0, 0, 0, 0, 0};
     BuildScratch s;
+    rtb::HandleCount counted;
     rtb::DevBuf  trace_status, trace_rays, trace_hits;
     // the path tracer's scratch, handed from call to call through wf_ev (render.cu)
     std::mutex   wf_mu;

@@ -368,8 +368,6 @@ int trace(const rt_bvh* B, const rt_ray* d_rays, rt_hit* d_hits, uint64_t n, uin
 {
     if (n == 0) { return RT_OK; }
     if (((uintptr_t)d_rays & 15) || ((uintptr_t)d_hits & 15)) { return fail(RT_E_INVALID, "rays/hits must be 16-byte aligned"); }
-    rt_bvh* Bm = const_cast<rt_bvh*>(B);
-    if (Bm->trace_status.ensure(64)) { return RT_E_CUDA; }
     const TraceFn fn = trace_fn(flags, B->trace_wide);
     constexpr uint64_t WPB = TBLK / 32;
     const size_t smem = B->trace_wide ? 0 : WPB * sizeof(WarpShare);
@@ -381,11 +379,16 @@ int trace(const rt_bvh* B, const rt_ray* d_rays, rt_hit* d_hits, uint64_t n, uin
     const bool few = !B->trace_wide && n <= warps * 32;
     const uint64_t per_warp = few ? std::max<uint64_t>(1, (n + warps - 1) / warps) : 32;
     grid = std::min(grid, (n + per_warp * WPB - 1) / (per_warp * WPB));
-    unsigned long long* counter = few ? nullptr : Bm->trace_status.as<unsigned long long>();
-    if (counter) { RT_CUDA(cudaMemsetAsync(counter, 0, 8, st)); }
+    // The counter is the call's own: calls on a handle may run at the same time.
+    CallScratch counter;
+    if (!few)
+    {
+        if (int e = counter.get(8, st)) { return e; }
+        RT_CUDA(cudaMemsetAsync(counter.as<void>(), 0, 8, st));
+    }
     const TraceCtx T = make_trace_ctx(B);
-    fn<<<(uint32_t)grid, TBLK, smem, st>>>(T, reinterpret_cast<const float4*>(d_rays), reinterpret_cast<float4*>(d_hits), n, counter,
-                                           status, (int)per_warp);
+    fn<<<(uint32_t)grid, TBLK, smem, st>>>(T, reinterpret_cast<const float4*>(d_rays), reinterpret_cast<float4*>(d_hits), n,
+                                           counter.as<unsigned long long>(), status, (int)per_warp);
     count_launch();
     return check_launch("trace");
 }

@@ -1,0 +1,51 @@
+"""Calls on one built handle at the same time, from host threads with streams of their own: each
+gives what it gives alone."""
+import threading
+
+import pytest
+import torch
+
+import rtb200
+from rtb200 import scenes
+
+pytestmark = pytest.mark.gpu
+
+
+def in_threads(n, work):
+    failed = []
+
+    def run(k):
+        try:
+            work(k)
+        except BaseException as e:  # noqa: BLE001 - reported by the test's own thread
+            failed.append((k, e))
+
+    torch.cuda.synchronize()
+    threads = [threading.Thread(target=run, args=(k,)) for k in range(n)]
+    for t in threads:
+        t.start()
+    for t in threads:
+        t.join()
+    assert not failed, failed
+
+
+@pytest.mark.parametrize("form", [-1, 2])
+@pytest.mark.parametrize("n", [1000, 160001])
+def test_traces(form, n):
+    """Small batches and batches of more rays than the chip holds lanes, whose warps claim rays from a
+    counter: every call's own rays are traced, each once."""
+    v, t = scenes.soup(3000, seed=8, lo=1e-2, hi=1e-1)
+    b = rtb200.Bvh.build(v, t, "lbvh63")
+    b.trace_loop(form)
+    rays = [torch.from_numpy(scenes.incoherent_rays(n, [0, 0, 0], [1, 1, 1], seed=k)).cuda() for k in range(8)]
+    want = [b.trace(r) for r in rays]
+    streams = [torch.cuda.Stream() for _ in rays]
+    hits = [[torch.full_like(r, -7.0) for _ in range(4)] for r in rays]
+
+    def work(k):
+        for h in hits[k]:
+            assert rtb200.lib().rt_trace(b.h, rays[k].data_ptr(), h.data_ptr(), n, 0, streams[k].cuda_stream) == 0
+
+    in_threads(len(rays), work)
+    for k, w in enumerate(want):
+        assert all(torch.equal(h.view(torch.int32), w.view(torch.int32)) for h in hits[k]), k
