@@ -672,6 +672,7 @@ int rt_trace_host(const rt_bvh* b, const rt_ray* rays, rt_hit* hits, uint64_t n,
     if (!b) { return fail(RT_E_NOT_LOADED, "BVH not loaded on trace()"); }
     if (n == 0) { return RT_OK; }
     rt_bvh* bm = const_cast<rt_bvh*>(b);
+    std::lock_guard<std::mutex> lk(bm->host_mu);
     if (bm->trace_rays.ensure((size_t)n * 32) || bm->trace_hits.ensure((size_t)n * 32)) { return RT_E_CUDA; }
     cudaStream_t st = default_stream();
     RT_CUDA(cudaMemcpyAsync(bm->trace_rays.p, rays, (size_t)n * 32, cudaMemcpyHostToDevice, st));

@@ -239,7 +239,9 @@ struct rt_bvh
     uint32_t     stats[8] = {0, 0, 0, 0, 0, 0, 0, 0};
     BuildScratch s;
     rtb::HandleCount counted;
-    rtb::DevBuf  trace_status, trace_rays, trace_hits;
+    rtb::DevBuf  trace_status;
+    std::mutex   host_mu;                   // rt_trace_host's staging buffers: one call at a time
+    rtb::DevBuf  trace_rays, trace_hits;
     // the path tracer's scratch, handed from call to call through wf_ev (render.cu)
     std::mutex   wf_mu;
     rtb::DevBuf  wf_buf;

@@ -49,3 +49,20 @@ def test_traces(form, n):
     in_threads(len(rays), work)
     for k, w in enumerate(want):
         assert all(torch.equal(h.view(torch.int32), w.view(torch.int32)) for h in hits[k]), k
+
+
+def test_host_traces():
+    """Rays from host memory: batches of different sizes, whose staging buffers grow on the way."""
+    v, t = scenes.soup(3000, seed=8, lo=1e-2, hi=1e-1)
+    b = rtb200.Bvh.build(v, t, "hybrid")
+    rays = [scenes.incoherent_rays(1000 * 3 ** (k % 4) + k, [0, 0, 0], [1, 1, 1], seed=k) for k in range(12)]
+    want = [rtb200.Bvh.build(v, t, "hybrid").trace(r) for r in rays]
+    got = [[] for _ in rays]
+
+    def work(k):
+        for _ in range(3):
+            got[k].append(b.trace(rays[k]))
+
+    in_threads(len(rays), work)
+    for k, w in enumerate(want):
+        assert len(got[k]) == 3 and all(g.tobytes() == w.tobytes() for g in got[k]), k
