@@ -221,6 +221,8 @@ struct PathJob
     uint32_t         sample0;  // sample of item 0, from P.sample_offset
     uint32_t         first, n; // this launch's items
     float*           rad;      // radiance per path: [sample - sample0][scene][pixel][3]
+    float*           rgb;      // the images (OWN)
+    float*           rgb2;
 };
 
 // Shared memory of one warp's paths.
@@ -230,8 +232,10 @@ struct PathShare
     float4    tp[32];  // throughput, image pixel (scene * W * H + pixel)
     float4    sum[32]; // radiance so far, sample
 };
-// The radiance of every path.
-template <int STK>
+// The radiance of every path. OWN: a lane takes whole pixels, adds their samples to the images itself,
+// in the order and with the roundings of k_sum, and needs no memory besides: for renders that may not
+// have any (run_paths). Half as fast where the pixels do not fill the chip.
+template <int STK, bool OWN>
 __global__ void __launch_bounds__(256, 4)
 k_paths(const TraceCtx T, const __grid_constant__ PathJob J, uint32_t* __restrict__ counter, int per_warp)
 {
@@ -247,12 +251,37 @@ k_paths(const TraceCtx T, const __grid_constant__ PathJob J, uint32_t* __restric
     uint2 stk[STK];
     L.live = false;
     bool pending = false, more = true;  // this lane has a ray (to shade when it is done); items are left
+    uint64_t own = 0, own_step = 0;     // OWN: the lane's pixel (an item of one sample), the way to its next
+    uint32_t smp = 0;                   // OWN: its sample
+    if (OWN)
+    {
+        const uint32_t wpb = blockDim.x >> 5;
+        own_step = (uint64_t)gridDim.x * wpb * (uint32_t)per_warp;
+        own = ((uint64_t)blockIdx.x * wpb + (threadIdx.x >> 5)) * (uint32_t)per_warp + (uint32_t)lane;
+        if (lane >= per_warp) { own = J.n; }
+    }
+    // the first ray of sample s of an item of one sample; false where the item lies outside the image
+    auto begin = [&](uint32_t item, uint32_t s, float4& r0, float4& r1) -> bool {
+        const uint32_t sc = item / J.scene_items;
+        const uint32_t q = item - sc * J.scene_items, tile = q >> 5, ty = tile / J.tiles_x;
+        const uint32_t x = (tile - ty * J.tiles_x) * 8u + (q & 7u), y = ty * 4u + ((q >> 3) & 3u);
+        if (x >= J.P.W || y >= J.P.H) { return false; }
+        const uint32_t pix = y * J.P.W + x, sidx = J.P.sample_offset + J.sample0 + s;
+        f3 o, d;
+        primary(J.P, J.cams ? J.cams[sc] : J.P.cam, x, y, pix, sidx, o, d);
+        r0 = make_float4(o.x, o.y, o.z, 1e-3f);
+        r1 = make_float4(d.x, d.y, d.z, bits2f(0x7f800000u));
+        S.tp[lane] = make_float4(1.f, 1.f, 1.f, __uint_as_float(sc * npix + pix));
+        S.sum[lane] = make_float4(0.f, 0.f, 0.f, __uint_as_float(sidx));
+        return true;
+    };
     for (;;)
     {
         // lanes whose ray is done are shaded, and those whose path is done get a new one, once enough
         // of them wait; when no paths are left, once half of the lanes still at work do
         const unsigned idle = __ballot_sync(FULL, !L.live) & lanes;
-        const unsigned takers = more ? lanes : __ballot_sync(FULL, pending);
+        const unsigned takers = OWN ? __ballot_sync(FULL, own < J.n) : more ? lanes : __ballot_sync(FULL, pending);
+        if (OWN) { more = takers == lanes; }
         const int serve = more ? refill : (__popc(takers) + 1) / 2;
         if (__popc(idle & takers) >= serve)
         {
@@ -268,7 +297,6 @@ k_paths(const TraceCtx T, const __grid_constant__ PathJob J, uint32_t* __restric
                 f3 tp = mk3(ts.x, ts.y, ts.z), sum = mk3(ss.x, ss.y, ss.z);
                 const uint32_t gpix = __float_as_uint(ts.w), sidx = __float_as_uint(ss.w);
                 const uint32_t sc = gpix / npix;
-                const size_t at = 3 * ((size_t)(sidx - J.P.sample_offset - J.sample0) * J.S * npix + gpix);
                 bounce = (uint32_t)S.w.id[lane];
                 Surf sf;
                 go = shade(T, J.P, J.sh, J.cams ? J.cams[sc].seed : J.P.cam.seed, gpix - sc * npix, sidx, bounce, L.hit, L.best, h,
@@ -279,36 +307,58 @@ k_paths(const TraceCtx T, const __grid_constant__ PathJob J, uint32_t* __restric
                     S.sum[lane] = make_float4(sum.x, sum.y, sum.z, ss.w);
                     bounce++;
                 }
-                else { J.rad[at] = sum.x; J.rad[at + 1] = sum.y; J.rad[at + 2] = sum.z; }
+                else if (OWN)
+                {
+                    const float fs = (float)J.P.spp;
+                    const bool end = smp + 1u == J.P.spp;
+#pragma unroll
+                    for (int c = 0; c < 3; c++)
+                    {
+                        const float v = get3(sum, c);
+                        float* p = J.rgb + 3 * (size_t)gpix + c;
+                        const float a = (smp ? *p : 0.f) + v;
+                        *p = end ? a / fs : a;
+                        if (J.rgb2)
+                        {
+                            float* p2 = J.rgb2 + 3 * (size_t)gpix + c;
+                            const float a2 = (smp ? *p2 : 0.f) + v * v;
+                            *p2 = end ? a2 / fs : a2;
+                        }
+                    }
+                    smp = end ? 0u : smp + 1u;
+                    if (end) { own += own_step; }
+                }
+                else
+                {
+                    const size_t at = 3 * ((size_t)(sidx - J.P.sample_offset - J.sample0) * J.S * npix + gpix);
+                    J.rad[at] = sum.x; J.rad[at + 1] = sum.y; J.rad[at + 2] = sum.z;
+                }
             }
             // new paths for the others
             const bool want = mine && !go;
-            const unsigned wants = __ballot_sync(FULL, want);
-            if (more && wants)
+            if (OWN)
             {
-                uint32_t base = 0;
-                if (lane == 0) { base = atomicAdd(counter, (uint32_t)__popc(wants)); }
-                base = __shfl_sync(FULL, base, 0);
-                if (base + (uint32_t)__popc(wants) >= J.n) { more = false; }
-                const uint32_t g = base + (uint32_t)__popc(wants & ((1u << lane) - 1u));
-                if (want && g < J.n)
+                if (want)
                 {
-                    const uint32_t G = J.first + g, per_sample = J.scene_items * J.S;
-                    const uint32_t s = G / per_sample, rem = G - s * per_sample, sc = rem / J.scene_items;
-                    const uint32_t q = rem - sc * J.scene_items, tile = q >> 5, ty = tile / J.tiles_x;
-                    const uint32_t x = (tile - ty * J.tiles_x) * 8u + (q & 7u), y = ty * 4u + ((q >> 3) & 3u);
-                    const uint32_t pix = y * J.P.W + x, gpix = sc * npix + pix;
-                    if (x < J.P.W && y < J.P.H)
+                    while (own < J.n && !(go = begin((uint32_t)own, smp, r0, r1))) { own += own_step; }
+                    bounce = 0;
+                }
+            }
+            else
+            {
+                const unsigned wants = __ballot_sync(FULL, want);
+                if (more && wants)
+                {
+                    uint32_t base = 0;
+                    if (lane == 0) { base = atomicAdd(counter, (uint32_t)__popc(wants)); }
+                    base = __shfl_sync(FULL, base, 0);
+                    if (base + (uint32_t)__popc(wants) >= J.n) { more = false; }
+                    const uint32_t g = base + (uint32_t)__popc(wants & ((1u << lane) - 1u));
+                    if (want && g < J.n)
                     {
-                        const uint32_t sidx = J.P.sample_offset + J.sample0 + s;
-                        f3 o, d;
-                        primary(J.P, J.cams ? J.cams[sc] : J.P.cam, x, y, pix, sidx, o, d);
-                        r0 = make_float4(o.x, o.y, o.z, 1e-3f);
-                        r1 = make_float4(d.x, d.y, d.z, bits2f(0x7f800000u));
-                        S.tp[lane] = make_float4(1.f, 1.f, 1.f, __uint_as_float(gpix));
-                        S.sum[lane] = make_float4(0.f, 0.f, 0.f, __uint_as_float(sidx));
+                        const uint32_t G = J.first + g, per_sample = J.scene_items * J.S, s = G / per_sample;
+                        go = begin(G - s * per_sample, s, r0, r1);
                         bounce = 0;
-                        go = true;
                     }
                 }
             }
@@ -321,7 +371,7 @@ k_paths(const TraceCtx T, const __grid_constant__ PathJob J, uint32_t* __restric
                 pending = true;
             }
             __syncwarp();
-            if (!more && !__any_sync(FULL, pending)) { break; }
+            if ((OWN || !more) && !__any_sync(FULL, pending)) { break; }
             continue;
         }
         warp_walk<0, STK>(L, stk, T, S.w, takers, serve);
@@ -607,7 +657,7 @@ int launch_paths(PathFn fn, const TraceCtx& T, const PathJob& J, uint32_t* count
     const uint64_t per_warp = std::min<uint64_t>(32, (J.n + warps - 1) / warps);
     const uint64_t grid = std::min<uint64_t>((uint64_t)device_sm_count() * (uint64_t)per_sm,
                                              (J.n + per_warp * (block / 32) - 1) / (per_warp * (block / 32)));
-    RT_CUDA(cudaMemsetAsync(counter, 0, 4, st));
+    if (counter) { RT_CUDA(cudaMemsetAsync(counter, 0, 4, st)); }
     fn<<<(uint32_t)grid, block, smem, st>>>(T, J, counter, (int)per_warp);
     count_launch();
     return check_launch("paths");
@@ -627,6 +677,19 @@ int run_paths(const rt_bvh* B, PathJob J, const Cam* h_cams, const rt_wavefront_
     const uint64_t per_sample = items * J.S;
     const uint64_t group = std::max<uint64_t>(1, std::min<uint64_t>(W.chunk_paths / per_sample, J.P.spp));
     const uint64_t rad_bytes = (group * npix * J.S * 12 + 255) / 256 * 256, cam_bytes = (J.S * sizeof(Cam) + 255) / 256 * 256;
+    const TraceCtx T = make_trace_ctx(B);
+    cudaStreamCaptureStatus cs = cudaStreamCaptureStatusNone;
+    RT_CUDA(cudaStreamIsCapturing(st, &cs));
+    if (cs != cudaStreamCaptureStatusNone && !h_cams)
+    {
+        // A captured render is one kernel node: memory nodes would keep the caller from using the
+        // graph as a child or twice at a time.
+        J.rgb = rgb; J.rgb2 = rgb2;
+        J.n = (uint32_t)per_sample;
+        return launch_paths(k_paths<STACK, true>, T, J, nullptr, W.trace_block, st);
+    }
+    // (a warm-up call loads what a captured one launches)
+    blocks_per_sm(reinterpret_cast<const void*>(k_paths<STACK, true>), (int)W.trace_block, (W.trace_block / 32) * sizeof(PathShare));
     PathScratch scratch(const_cast<rt_bvh*>(B), st);
     void* mem = nullptr;
     if (int e = scratch.get(rad_bytes + cam_bytes + 256, &mem)) { return e; }
@@ -640,8 +703,7 @@ int run_paths(const rt_bvh* B, PathJob J, const Cam* h_cams, const rt_wavefront_
         RT_CUDA(cudaMemcpyAsync(cams, h_cams, J.S * sizeof(Cam), cudaMemcpyHostToDevice, st));
         J.cams = cams;
     }
-    const TraceCtx T = make_trace_ctx(B);
-    const PathFn fn = W.stack_depth < 64 ? k_paths<32> : k_paths<STACK>;
+    const PathFn fn = W.stack_depth < 64 ? k_paths<32, false> : k_paths<STACK, false>;
     const uint64_t channels = npix * J.S * 3;
     for (uint64_t s0 = 0; s0 < J.P.spp; s0 += group)
     {
