@@ -609,40 +609,26 @@ int check_params(const rt_wavefront_params& W)
 
 // The scratch of one render: radiance of the paths in flight, per-scene cameras and
 // the item counter. It belongs to the handle and is passed from call to call through an event, so
-// calls on other streams and host threads queue up behind one another; a call that is being
-// captured into a graph owns its scratch as memory nodes of that graph.
+// calls on other streams and host threads queue up behind one another.
 class PathScratch
 {
     rt_bvh*                      B_;
     cudaStream_t                 st_;
-    bool                         capturing_ = false;
     std::unique_lock<std::mutex> lk_;
-    void*                        mem_ = nullptr;
 
 public:
     PathScratch(rt_bvh* B, cudaStream_t st) : B_(B), st_(st), lk_(B->wf_mu) {}
     int get(size_t bytes, void** p)
     {
-        cudaStreamCaptureStatus cs = cudaStreamCaptureStatusNone;
-        RT_CUDA(cudaStreamIsCapturing(st_, &cs));
-        capturing_ = cs != cudaStreamCaptureStatusNone;
-        if (capturing_)
-        {
-            RT_CUDA(cudaMallocAsync(&mem_, bytes, st_));
-            *p = mem_;
-            return RT_OK;
-        }
         if (!B_->wf_ev) { RT_CUDA(cudaEventCreateWithFlags(&B_->wf_ev, cudaEventDisableTiming)); }
         else { RT_CUDA(cudaStreamWaitEvent(st_, B_->wf_ev, 0)); }
         if (B_->wf_buf.ensure(bytes)) { return RT_E_CUDA; }
         *p = B_->wf_buf.p;
         return RT_OK;
     }
-    bool capturing() const { return capturing_; }
     ~PathScratch()
     {
-        if (mem_) { cudaFreeAsync(mem_, st_); }
-        else if (!capturing_ && B_->wf_ev) { cudaEventRecord(B_->wf_ev, st_); }
+        if (B_->wf_ev) { cudaEventRecord(B_->wf_ev, st_); }
     }
 };
 
@@ -680,8 +666,9 @@ int run_paths(const rt_bvh* B, PathJob J, const Cam* h_cams, const rt_wavefront_
     const TraceCtx T = make_trace_ctx(B);
     cudaStreamCaptureStatus cs = cudaStreamCaptureStatusNone;
     RT_CUDA(cudaStreamIsCapturing(st, &cs));
-    if (cs != cudaStreamCaptureStatusNone && !h_cams)
+    if (cs != cudaStreamCaptureStatusNone)
     {
+        if (h_cams) { return fail(RT_E_INVALID, "a render of several scenes cannot be captured"); }
         // A captured render is one kernel node: memory nodes would keep the caller from using the
         // graph as a child or twice at a time.
         J.rgb = rgb; J.rgb2 = rgb2;
@@ -698,7 +685,6 @@ int run_paths(const rt_bvh* B, PathJob J, const Cam* h_cams, const rt_wavefront_
     uint32_t* counter = reinterpret_cast<uint32_t*>(static_cast<char*>(mem) + rad_bytes + cam_bytes);
     if (h_cams)
     {
-        if (scratch.capturing()) { return fail(RT_E_INVALID, "a render of several scenes cannot be captured"); }
         // (an upload from pageable memory has left the host array when cudaMemcpyAsync returns)
         RT_CUDA(cudaMemcpyAsync(cams, h_cams, J.S * sizeof(Cam), cudaMemcpyHostToDevice, st));
         J.cams = cams;

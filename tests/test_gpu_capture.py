@@ -42,3 +42,22 @@ def test_captured_render(mode, w, h, spp):
         assert all(torch.equal(g, x) for g, x in zip(got, want))
     for _, ex in execs:
         rt.cudaGraphExecDestroy(ex)
+
+
+def test_captured_batch_is_refused():
+    """A render of several scenes uploads their cameras and cannot be captured: it says so and leaves
+    the caller's graph as it was."""
+    from cuda.bindings import runtime as rt
+    from test_gpu_batch import batch_setup, cfgs_for
+    scs, bb, mats, mot = batch_setup(n=3)
+    dm, dmot = device(mats, mot)
+    rcs = cfgs_for(scs, 32, 24, 2, max_bounce=3, rr_after=-1)
+    want = bb.render_batch(rcs, dm, dmot)[0]
+    graph = torch.cuda.CUDAGraph(keep_graph=True)
+    x = torch.zeros(8, device="cuda")
+    with torch.cuda.graph(graph):
+        x.add_(1.0)
+        with pytest.raises(rtb200.RtError, match="RT_E_INVALID"):
+            bb.render_batch(rcs, dm, dmot)
+    assert rt.cudaGraphGetNodes(graph.raw_cuda_graph())[2] == 1
+    assert torch.equal(bb.render_batch(rcs, dm, dmot)[0], want)
