@@ -222,11 +222,9 @@ static void free_bvh(rt_bvh* b)
                        &b->s.sah_lvl_a, &b->s.sah_lvl_b, &b->s.sah_dec, &b->s.sah_out, &b->s.sah_leaf_refs,
                        &b->s.sah_scan_in, &b->s.sah_scan_out, &b->s.sah_node_ids, &b->s.sah_roots_lvl, &b->s.sah_jobs, &b->s.sah_root_ord, &b->s.root_sort.keys_alt,
                        &b->s.root_sort.vals_alt, &b->s.root_sort.lookback, &b->s.root_sort.tile_counters,
-                       &b->s.in_verts, &b->s.in_tris, &b->s.gtris, &b->s.batch_off, &b->s.sah_budget, &b->s.sah_wide, &b->s.sah_tmp2, &b->s.sah_pos2, &b->s.wide_flag, &b->s.wide_par, &b->wnodes, &b->wid, &b->scene_info, &b->scene_roots,
-                       &b->wf_buf };
+                       &b->s.in_verts, &b->s.in_tris, &b->s.gtris, &b->s.batch_off, &b->s.sah_budget, &b->s.sah_wide, &b->s.sah_tmp2, &b->s.sah_pos2, &b->s.wide_flag, &b->s.wide_par, &b->wnodes, &b->wid, &b->scene_info, &b->scene_roots };
     for (DevBuf* x : bufs) { x->release(); }
     b->rootbuf.release();
-    if (b->wf_ev) { cudaEventDestroy(b->wf_ev); b->wf_ev = nullptr; }
     if (b->bake_exec) { cudaGraphExecDestroy(b->bake_exec); b->bake_exec = nullptr; }
     for (cudaEvent_t& e : b->bake_ev)
     {

@@ -607,31 +607,6 @@ int check_params(const rt_wavefront_params& W)
     return RT_OK;
 }
 
-// The scratch of one render: radiance of the paths in flight, per-scene cameras and
-// the item counter. It belongs to the handle and is passed from call to call through an event, so
-// calls on other streams and host threads queue up behind one another.
-class PathScratch
-{
-    rt_bvh*                      B_;
-    cudaStream_t                 st_;
-    std::unique_lock<std::mutex> lk_;
-
-public:
-    PathScratch(rt_bvh* B, cudaStream_t st) : B_(B), st_(st), lk_(B->wf_mu) {}
-    int get(size_t bytes, void** p)
-    {
-        if (!B_->wf_ev) { RT_CUDA(cudaEventCreateWithFlags(&B_->wf_ev, cudaEventDisableTiming)); }
-        else { RT_CUDA(cudaStreamWaitEvent(st_, B_->wf_ev, 0)); }
-        if (B_->wf_buf.ensure(bytes)) { return RT_E_CUDA; }
-        *p = B_->wf_buf.p;
-        return RT_OK;
-    }
-    ~PathScratch()
-    {
-        if (B_->wf_ev) { cudaEventRecord(B_->wf_ev, st_); }
-    }
-};
-
 using PathFn = void (*)(TraceCtx, PathJob, uint32_t*, int);
 
 int launch_paths(PathFn fn, const TraceCtx& T, const PathJob& J, uint32_t* counter, uint32_t block, cudaStream_t st)
@@ -651,7 +626,9 @@ int launch_paths(PathFn fn, const TraceCtx& T, const PathJob& J, uint32_t* count
 
 // Renders J's scenes. Samples are taken in groups
 // whose paths fit W.chunk_paths (at least one sample of every pixel), each group launched in pieces
-// of at most that many paths.
+// of at most that many paths. The call's scratch: the radiance of a group's paths, the cameras and the item
+// counter. Where the device has no memory for it, smaller groups give the same image, and at last a
+// lane per pixel does.
 int run_paths(const rt_bvh* B, PathJob J, const Cam* h_cams, const rt_wavefront_params& W, float* rgb, float* rgb2,
               cudaStream_t st)
 {
@@ -661,9 +638,12 @@ int run_paths(const rt_bvh* B, PathJob J, const Cam* h_cams, const rt_wavefront_
     J.tiles_x = (uint32_t)tiles_x;
     J.scene_items = (uint32_t)items;
     const uint64_t per_sample = items * J.S;
-    const uint64_t group = std::max<uint64_t>(1, std::min<uint64_t>(W.chunk_paths / per_sample, J.P.spp));
-    const uint64_t rad_bytes = (group * npix * J.S * 12 + 255) / 256 * 256, cam_bytes = (J.S * sizeof(Cam) + 255) / 256 * 256;
     const TraceCtx T = make_trace_ctx(B);
+    auto own_pixels = [&]() {
+        J.rgb = rgb; J.rgb2 = rgb2;
+        J.n = (uint32_t)per_sample;
+        return launch_paths(k_paths<STACK, true>, T, J, nullptr, W.trace_block, st);
+    };
     cudaStreamCaptureStatus cs = cudaStreamCaptureStatusNone;
     RT_CUDA(cudaStreamIsCapturing(st, &cs));
     if (cs != cudaStreamCaptureStatusNone)
@@ -671,24 +651,26 @@ int run_paths(const rt_bvh* B, PathJob J, const Cam* h_cams, const rt_wavefront_
         if (h_cams) { return fail(RT_E_INVALID, "a render of several scenes cannot be captured"); }
         // A captured render is one kernel node: memory nodes would keep the caller from using the
         // graph as a child or twice at a time.
-        J.rgb = rgb; J.rgb2 = rgb2;
-        J.n = (uint32_t)per_sample;
-        return launch_paths(k_paths<STACK, true>, T, J, nullptr, W.trace_block, st);
+        return own_pixels();
     }
     // (a warm-up call loads what a captured one launches)
     blocks_per_sm(reinterpret_cast<const void*>(k_paths<STACK, true>), (int)W.trace_block, (W.trace_block / 32) * sizeof(PathShare));
-    PathScratch scratch(const_cast<rt_bvh*>(B), st);
-    void* mem = nullptr;
-    if (int e = scratch.get(rad_bytes + cam_bytes + 256, &mem)) { return e; }
-    J.rad = static_cast<float*>(mem);
-    Cam* cams = reinterpret_cast<Cam*>(static_cast<char*>(mem) + rad_bytes);
-    uint32_t* counter = reinterpret_cast<uint32_t*>(static_cast<char*>(mem) + rad_bytes + cam_bytes);
+    // cameras, item counter, radiance
+    const uint64_t cam_bytes = h_cams ? (J.S * sizeof(Cam) + 255) / 256 * 256 : 0, head = cam_bytes + 256;
+    uint64_t group = std::max<uint64_t>(1, std::min<uint64_t>(W.chunk_paths / per_sample, J.P.spp));
+    CallScratch scratch;
+    int missing = 0;
+    while ((missing = scratch.get(head + group * npix * J.S * 12, st)) != 0 && group > 0) { group /= 2; }
+    if (missing && h_cams) { return missing; }
     if (h_cams)
     {
         // (an upload from pageable memory has left the host array when cudaMemcpyAsync returns)
-        RT_CUDA(cudaMemcpyAsync(cams, h_cams, J.S * sizeof(Cam), cudaMemcpyHostToDevice, st));
-        J.cams = cams;
+        RT_CUDA(cudaMemcpyAsync(scratch.as<void>(), h_cams, J.S * sizeof(Cam), cudaMemcpyHostToDevice, st));
+        J.cams = scratch.as<Cam>();
     }
+    if (group == 0) { return own_pixels(); }
+    uint32_t* counter = reinterpret_cast<uint32_t*>(scratch.as<char>() + cam_bytes);
+    J.rad = reinterpret_cast<float*>(scratch.as<char>() + head);
     const PathFn fn = W.stack_depth < 64 ? k_paths<32, false> : k_paths<STACK, false>;
     const uint64_t channels = npix * J.S * 3;
     for (uint64_t s0 = 0; s0 < J.P.spp; s0 += group)

@@ -242,10 +242,6 @@ struct rt_bvh
     rtb::DevBuf  trace_status;
     std::mutex   host_mu;                   // rt_trace_host's staging buffers: one call at a time
     rtb::DevBuf  trace_rays, trace_hits;
-    // the path tracer's scratch, handed from call to call through wf_ev (render.cu)
-    std::mutex   wf_mu;
-    rtb::DevBuf  wf_buf;
-    cudaEvent_t  wf_ev = nullptr;
     // an LBVH bake's launch sequence, captured on the second call with the same key (sizes,
     // settings, inputs, buffer addresses) and replayed on bake_stream (fenced with the caller's
     // stream by bake_ev); its key, and the key the last plain bake left

@@ -1,0 +1,123 @@
+"""Renders' device memory: no more is kept than the documented bound however many handles render, all is
+given back with the last handle, renders on different streams do not wait for one another, and a render
+that finds less memory than it would like still gives the same image. The cases that fill the device or look
+at all of its memory run in a process of their own."""
+import os
+import subprocess
+import sys
+
+import pytest
+import torch
+
+import rtb200
+from test_gpu_paths import VIEW, scene
+
+pytestmark = pytest.mark.gpu
+HERE = os.path.dirname(os.path.abspath(__file__))
+
+PRELUDE = """
+import ctypes, gc, sys
+import numpy as np, torch
+import rtb200
+from cuda.bindings import runtime as rt
+from test_gpu_paths import VIEW, scene
+
+def free():
+    torch.cuda.synchronize()
+    return torch.cuda.mem_get_info()[0]
+
+def cfg(w, h, spp):
+    return rtb200.render_cfg(w, h, spp, max_bounce=3, rr_after=-1, env_kind=1, env_color=(0.1, 0.2, 0.3), seed=w, lookat=VIEW)
+"""
+
+
+def in_process(code):
+    env = dict(os.environ, PYTHONPATH=os.pathsep.join([HERE, *sys.path]))
+    r = subprocess.run([sys.executable, "-c", PRELUDE + code], env=env, capture_output=True, text=True, timeout=300)
+    assert r.returncode == 0, r.stdout + r.stderr
+
+
+def test_scratch_is_bounded_and_given_back():
+    in_process("""
+b, mats, mot = scene()
+dm, dmot = torch.from_numpy(rtb200.materials_array(mats)).cuda(), torch.from_numpy(mot.astype(np.int32)).cuda()
+b.render(cfg(64, 64, 1), dm, dmot)
+handles = [scene()[0] for _ in range(5)]
+before = free()
+imgs = [x.render(cfg(1024, 1024, 32), dm, dmot)[0] for x in handles]  # 403 MB each while it runs
+torch.cuda.synchronize()
+kept = before - free()
+assert kept < (512 + 96) << 20, kept  # and the images
+for x in handles + [b]:
+    x.free()
+del imgs
+gc.collect()
+torch.cuda.empty_cache()
+assert before - free() < 32 << 20, before - free()
+""")
+
+
+def test_little_memory_left():
+    """Enough for some samples a launch, then not even for one."""
+    in_process("""
+b, mats, mot = scene()
+dm, dmot = torch.from_numpy(rtb200.materials_array(mats)).cuda(), torch.from_numpy(mot.astype(np.int32)).cuda()
+sh = rtb200.api.Shading()
+sh.mats, sh.n_mats, sh.mat_of_tri = dm.data_ptr(), dm.shape[0], dmot.data_ptr()
+
+def render(c, out, out2, handle):
+    code = rtb200.lib().rt_render_ex(handle.h, ctypes.byref(c), ctypes.byref(sh), 0, out.data_ptr(), out2.data_ptr(), None)
+    rtb200.lib().rt_device_sync(None)
+    return code
+
+jobs = []
+for w, h, spp in ((1024, 1024, 32), (3001, 2200, 2)):
+    jobs.append((cfg(w, h, spp), [torch.zeros(h, w, 3, device="cuda") for _ in range(4)]))
+torch.cuda.synchronize()  # (the renders run on the library's own stream)
+for c, t in jobs:
+    assert render(c, t[0], t[1], b) == 0
+graph = torch.cuda.CUDAGraph()  # loads the form without scratch
+with torch.cuda.graph(graph):
+    x = b.render(cfg(32, 32, 1), dm, dmot)[0]
+graph.replay()
+other = scene()[0]
+b.free()
+other.free()  # the last handles: the scratch is gone
+b = scene()[0]
+held, room = [], 48 << 20
+for size in (1 << 30, 64 << 20, 8 << 20):
+    while free() > size + room:
+        err, p = rt.cudaMalloc(size)
+        if err != rt.cudaError_t.cudaSuccess:
+            break
+        held.append(p)
+assert 16 << 20 < free() < 79 << 20, free()  # 403 MB and 79 MB (a sample of every pixel) would be taken
+for c, t in jobs:
+    assert render(c, t[2], t[3], b) == 0, rtb200.lib().rt_last_error()
+for p in held:
+    rt.cudaFree(p)
+for c, t in jobs:
+    assert torch.equal(t[0], t[2]) and torch.equal(t[1], t[3])
+""")
+
+
+def test_streams_do_not_wait_for_one_another():
+    b, mats, mot = scene()
+    import numpy as np
+    dm, dmot = torch.from_numpy(rtb200.materials_array(mats)).cuda(), torch.from_numpy(mot.astype(np.int32)).cuda()
+    rc = rtb200.render_cfg(64, 48, 4, max_bounce=3, rr_after=-1, env_kind=1, seed=1, lookat=VIEW)
+    want = b.render(rc, dm, dmot)[0]
+    s0, s1 = torch.cuda.Stream(), torch.cuda.Stream()
+    for s in (s0, s1):
+        with torch.cuda.stream(s):
+            b.render(rc, dm, dmot)
+    torch.cuda.synchronize()
+    with torch.cuda.stream(s0):
+        torch.cuda._sleep(1 << 30)  # about half a second before this stream's render
+        first = b.render(rc, dm, dmot)[0]
+    with torch.cuda.stream(s1):
+        second = b.render(rc, dm, dmot)[0]
+    s1.synchronize()
+    assert not s0.query()
+    torch.cuda.synchronize()
+    assert torch.equal(first, want) and torch.equal(second, want)
