@@ -138,8 +138,8 @@ void rt_bvh_free(rt_bvh* bvh);
  * they choose the loop of rt_adjoint's traversal (0 one loop, 1 while-while, -1 while-while when
  * leaves hold 6 or more triangles on average), traces and renders have one form for all. 2: the 8-wide layout (128-byte
  * nodes of up to eight children with 8-bit quantised, conservative child boxes), built now and
- * again after every rebuild of the handle; rt_trace, RT_RENDER_WAVEFRONT and rt_render_batch use it
- * (RT_RENDER_PLAIN keeps the binary tree). It is not the reference's visiting order: the closest hit's distance is the same, but on an exact tie
+ * again after every rebuild of the handle; rt_trace uses it (renders keep the binary tree). It is
+ * not the reference's visiting order: the closest hit's distance is the same, but on an exact tie
  * in distance the reported triangle may differ, and a triangle that the binary boxes cull -- one
  * an exact box test loses by rounding at a face, or, in trees with spatial splits, one outside a
  * collapsed intermediate node's box -- may be found. */

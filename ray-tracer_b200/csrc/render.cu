@@ -234,10 +234,9 @@ struct PathShare
 };
 // The radiance of every path. OWN: a lane takes whole pixels, adds their samples to the images itself,
 // in the order and with the roundings of k_sum, and needs no memory besides: for renders that may not
-// have any (run_paths). Half as fast where the pixels do not fill the chip. WIDE: each lane traces its ray by
-// itself over the 8-wide layout (a handle in form 2).
-template <int STK, bool OWN, bool WIDE>
-__global__ void __launch_bounds__(256, WIDE ? 2 : 4)
+// have any (run_paths). Half as fast where the pixels do not fill the chip.
+template <int STK, bool OWN>
+__global__ void __launch_bounds__(256, 4)
 k_paths(const TraceCtx T, const __grid_constant__ PathJob J, uint32_t* __restrict__ counter, int per_warp)
 {
     extern __shared__ __align__(16) unsigned char smem[];
@@ -368,14 +367,6 @@ k_paths(const TraceCtx T, const __grid_constant__ PathJob J, uint32_t* __restric
                 const TraceRoot* R = T.root;
                 if (J.roots) { R = J.roots + __float_as_uint(S.tp[lane].w) / npix; }
                 L.start(S.w, *R, r0, r1, odd_tree);
-                if (WIDE && L.live)
-                {
-                    const THit H = trace_ray_wide<0, STK>(T, *R, mk3(r0.x, r0.y, r0.z), mk3(r1.x, r1.y, r1.z), r0.w, r1.w);
-                    L.live = false;
-                    L.hit = H.hit;
-                    L.best = H.t;
-                    S.w.hit[lane] = make_float4(H.u, H.v, __uint_as_float(H.tri), 0.f);
-                }
                 S.w.id[lane] = bounce;
                 pending = true;
             }
@@ -383,11 +374,8 @@ k_paths(const TraceCtx T, const __grid_constant__ PathJob J, uint32_t* __restric
             if ((OWN || !more) && !__any_sync(FULL, pending)) { break; }
             continue;
         }
-        if (!WIDE)
-        {
-            warp_walk<0, STK>(L, stk, T, S.w, takers, serve);
-            warp_leaves<0, STK>(L, stk, T, S.w);
-        }
+        warp_walk<0, STK>(L, stk, T, S.w, takers, serve);
+        warp_leaves<0, STK>(L, stk, T, S.w);
     }
 }
 
@@ -621,13 +609,6 @@ int check_params(const rt_wavefront_params& W)
 
 using PathFn = void (*)(TraceCtx, PathJob, uint32_t*, int);
 
-PathFn path_fn(uint32_t stack, bool own, bool wide)
-{
-    if (own) { return wide ? k_paths<STACK, true, true> : k_paths<STACK, true, false>; }
-    if (stack < 64) { return wide ? k_paths<32, false, true> : k_paths<32, false, false>; }
-    return wide ? k_paths<STACK, false, true> : k_paths<STACK, false, false>;
-}
-
 int launch_paths(PathFn fn, const TraceCtx& T, const PathJob& J, uint32_t* counter, uint32_t block, cudaStream_t st)
 {
     const size_t smem = (size_t)(block / 32) * sizeof(PathShare);
@@ -648,7 +629,7 @@ int launch_paths(PathFn fn, const TraceCtx& T, const PathJob& J, uint32_t* count
 // of at most that many paths. The call's scratch: the radiance of a group's paths, the cameras and the item
 // counter. Where the device has no memory for it, smaller groups give the same image, and at last a
 // lane per pixel does.
-int run_paths(const rt_bvh* B, PathJob J, const Cam* h_cams, const rt_wavefront_params& W, bool wide, float* rgb, float* rgb2,
+int run_paths(const rt_bvh* B, PathJob J, const Cam* h_cams, const rt_wavefront_params& W, float* rgb, float* rgb2,
               cudaStream_t st)
 {
     const uint64_t npix = (uint64_t)J.P.W * J.P.H;
@@ -661,7 +642,7 @@ int run_paths(const rt_bvh* B, PathJob J, const Cam* h_cams, const rt_wavefront_
     auto own_pixels = [&]() {
         J.rgb = rgb; J.rgb2 = rgb2;
         J.n = (uint32_t)per_sample;
-        return launch_paths(path_fn(STACK, true, wide), T, J, nullptr, W.trace_block, st);
+        return launch_paths(k_paths<STACK, true>, T, J, nullptr, W.trace_block, st);
     };
     cudaStreamCaptureStatus cs = cudaStreamCaptureStatusNone;
     RT_CUDA(cudaStreamIsCapturing(st, &cs));
@@ -673,8 +654,7 @@ int run_paths(const rt_bvh* B, PathJob J, const Cam* h_cams, const rt_wavefront_
         return own_pixels();
     }
     // (a warm-up call loads what a captured one launches)
-    blocks_per_sm(reinterpret_cast<const void*>(path_fn(STACK, true, wide)), (int)W.trace_block,
-                  (W.trace_block / 32) * sizeof(PathShare));
+    blocks_per_sm(reinterpret_cast<const void*>(k_paths<STACK, true>), (int)W.trace_block, (W.trace_block / 32) * sizeof(PathShare));
     // cameras, item counter, radiance
     const uint64_t cam_bytes = h_cams ? (J.S * sizeof(Cam) + 255) / 256 * 256 : 0, head = cam_bytes + 256;
     uint64_t group = std::max<uint64_t>(1, std::min<uint64_t>(W.chunk_paths / per_sample, J.P.spp));
@@ -691,7 +671,7 @@ int run_paths(const rt_bvh* B, PathJob J, const Cam* h_cams, const rt_wavefront_
     if (group == 0) { return own_pixels(); }
     uint32_t* counter = reinterpret_cast<uint32_t*>(scratch.as<char>() + cam_bytes);
     J.rad = reinterpret_cast<float*>(scratch.as<char>() + head);
-    const PathFn fn = path_fn(W.stack_depth, false, wide);
+    const PathFn fn = W.stack_depth < 64 ? k_paths<32, false> : k_paths<STACK, false>;
     const uint64_t channels = npix * J.S * 3;
     for (uint64_t s0 = 0; s0 < J.P.spp; s0 += group)
     {
@@ -735,7 +715,7 @@ int render(const rt_bvh* B, const rt_render_cfg& cfg, const rt_shading& sh, int 
     J.sh = Shade{ sh.mats, sh.mat_of_tri, sh.tri_albedo, sh.n_mats };
     rt_wavefront_params W = mode == RT_RENDER_WAVEFRONT ? pick_params(B, nullptr) : default_params();
     W.stack_depth = 64;  // tuned for a batch; a plain handle keeps the full stack
-    return run_paths(B, J, nullptr, W, mode == RT_RENDER_WAVEFRONT && B->trace_wide, rgb, rgb2, st);
+    return run_paths(B, J, nullptr, W, rgb, rgb2, st);
 }
 
 int render_batch(rt_bvh* B, const rt_render_cfg* cfgs, uint32_t S, const rt_shading& sh, const rt_wavefront_params* params,
@@ -758,7 +738,7 @@ int render_batch(rt_bvh* B, const rt_render_cfg* cfgs, uint32_t S, const rt_shad
     J.S = S;
     J.sh = Shade{ sh.mats, sh.mat_of_tri, sh.tri_albedo, sh.n_mats };
     J.roots = S > 1 ? B->scene_roots.as<TraceRoot>() : nullptr;  // one scene: the whole tree
-    return run_paths(B, J, S > 1 ? cams.data() : nullptr, W, B->trace_wide, rgb, rgb2, st);
+    return run_paths(B, J, S > 1 ? cams.data() : nullptr, W, rgb, rgb2, st);
 }
 
 int autotune_wavefront(rt_bvh* B, const rt_render_cfg* cfgs, uint32_t S, const rt_shading& sh, rt_wavefront_params* best,

@@ -352,7 +352,7 @@ class Bvh:
 
     def trace_loop(self, form: int = -1):
         """Traversal form: -1, 0 and 1 the reference's visiting order over the binary tree; 2 the
-        8-wide layout for trace(), wavefront and batched renders (same closest distance, ties may report another triangle; kept up
+        8-wide layout for trace() (same closest distance, ties may report another triangle; kept up
         to date across rebuilds)."""
         _check(lib().rt_bvh_trace_loop(self.h, int(form)))
 
