@@ -374,7 +374,7 @@ k_paths(const TraceCtx T, const __grid_constant__ PathJob J, uint32_t* __restric
             if ((OWN || !more) && !__any_sync(FULL, pending)) { break; }
             continue;
         }
-        warp_walk<0, STK>(L, stk, T, S.w, takers, serve);
+        warp_walk<0, STK>(L, stk, T, takers, serve);
         warp_leaves<0, STK>(L, stk, T, S.w);
     }
 }

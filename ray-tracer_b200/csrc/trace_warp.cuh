@@ -128,7 +128,7 @@ struct LaneTrace
     }
 
     // One inner node: both children's boxes, the nearer child next, the farther one on the stack.
-    __device__ __forceinline__ void step(uint2 (&stk)[STK], const rt_gnode* __restrict__ gn, const WarpShare& S)
+    __device__ __forceinline__ void step(uint2 (&stk)[STK], const rt_gnode* __restrict__ gn)
     {
         const quad64 A = ldg256(gn + ref), B = ldg256(reinterpret_cast<const char*>(gn + ref) + 32);
         uint32_t lref, rref, lcnt, rcnt;
@@ -141,8 +141,7 @@ struct LaneTrace
             float l0, l1, l2, l3, l4, l5, r0, r1, r2, r3, r4, r5;
             unpack2(A.x, l0, l3); unpack2(A.y, l1, l4); unpack2(A.z, l2, l5);
             unpack2(A.w, r0, r3); unpack2(B.x, r1, r4); unpack2(B.y, r2, r5);
-            const float4 q = S.a[threadIdx.x & 31u], w = S.b[threadIdx.x & 31u];
-            const f3 o = mk3(q.x, q.y, q.z), inv = mk3(1.f / w.x, 1.f / w.y, 1.f / w.z);
+            const f3 o = mk3(ox, oy, oz), inv = mk3(ix, iy, iz);
             tl = ray_box(o, inv, tmin, best, l0, l1, l2, l3, l4, l5);
             tr = ray_box(o, inv, tmin, best, r0, r1, r2, r3, r4, r5);
         }
@@ -288,8 +287,8 @@ __device__ __forceinline__ void warp_leaves(LaneTrace<MODE, STK>& L, uint2 (&stk
 // Walks inner nodes until every live lane stands at a leaf, or few lanes walk and others wait at a
 // leaf or, `serve` or more of `takers`, to be served by the caller (a new ray).
 template <int MODE, int STK>
-__device__ __forceinline__ void warp_walk(LaneTrace<MODE, STK>& L, uint2 (&stk)[STK], const TraceCtx& T, const WarpShare& S,
-                                          unsigned takers, int serve)
+__device__ __forceinline__ void warp_walk(LaneTrace<MODE, STK>& L, uint2 (&stk)[STK], const TraceCtx& T, unsigned takers,
+                                          int serve)
 {
     constexpr unsigned FULL = 0xffffffffu;
     uint32_t it = 0;
@@ -303,7 +302,7 @@ __device__ __forceinline__ void warp_walk(LaneTrace<MODE, STK>& L, uint2 (&stk)[
             const unsigned live = __ballot_sync(FULL, L.live);
             if (live != walking || __popc(takers & ~live) >= serve) { break; }
         }
-        if (walk) { L.step(stk, T.gn, S); }
+        if (walk) { L.step(stk, T.gn); }
         __syncwarp();
     }
     // A validated BVH is a DAG with children after parents; the cap only bounds the work a

@@ -209,7 +209,7 @@ k_trace(TraceCtx T, const float4* __restrict__ rays, float4* __restrict__ hits, 
             __syncwarp();
             continue;
         }
-        warp_walk<MODE, STACK>(L, stk, T, S, more ? lanes : 0u, refill);
+        warp_walk<MODE, STACK>(L, stk, T, more ? lanes : 0u, refill);
         warp_leaves<MODE, STACK>(L, stk, T, S);
     }
 }

@@ -119,3 +119,29 @@ def test_stack_overflow_is_reported(n):
         return rtb200.lib().rt_trace(b.h, r.data_ptr(), hits.data_ptr(), n, 0, None)
 
     assert [call(rays), call(off), call(rays), call(off)] == [5, 0, 5, 0]
+
+
+def test_axis_parallel_rays_cost_what_others_do():
+    """Orthographic rays (two direction components 0) take the general box test at every node, with the
+    reciprocals of the ray's start: the same grid tilted a little takes the same nodes without it. 1.09-1.11 times
+    the time on a B200; 1.27-1.36 while the reciprocals were taken again at every node."""
+    v, t = scenes.icosphere(6, seed=2)
+    b = rtb200.Bvh.build(v, t, "sah4")
+    n = 1024
+    y, x = torch.meshgrid(torch.linspace(-1, 1, n, device="cuda"), torch.linspace(-1, 1, n, device="cuda"), indexing="ij")
+    rays = torch.zeros(n * n, 8, device="cuda")
+    rays[:, 0], rays[:, 1], rays[:, 2], rays[:, 6], rays[:, 7] = x.reshape(-1), y.reshape(-1), -2.0, 1.0, float("inf")
+    tilted = rays.clone()
+    tilted[:, 4], tilted[:, 5] = 1e-3, 2e-3
+    hits = torch.empty_like(rays)
+
+    def once(r):
+        a, e = torch.cuda.Event(enable_timing=True), torch.cuda.Event(enable_timing=True)
+        a.record()
+        assert rtb200.lib().rt_trace(b.h, r.data_ptr(), hits.data_ptr(), n * n, 0, 1) == 0  # (torch's default stream)
+        e.record()
+        e.synchronize()
+        return a.elapsed_time(e)
+
+    times = np.array([[once(rays), once(tilted)] for _ in range(24)])[4:]
+    assert np.median(times[:, 0] / times[:, 1]) < 1.2, times
