@@ -207,7 +207,7 @@ struct BuildScratch
     rtb::DevBuf sah_roots;     // SAH subtree roots
     // SAH builder state
     rtb::DevBuf sah_refs_a, sah_refs_b, sah_tmp, sah_pos, sah_lvl_a, sah_lvl_b, sah_dec, sah_out, sah_leaf_refs,
-        sah_scan_in, sah_scan_out, sah_node_ids, sah_roots_lvl, sah_jobs;
+        sah_scan_in, sah_scan_out, sah_node_ids, sah_roots_lvl;
     rtb::DevBuf sah_root_ord;       // the roots' sort keys, order, counts and their scan, per-depth runs
     rtb::SortScratch root_sort;     // (their sort's own scratch: the bake's sorted keys stay live)
     rtb::DevBuf in_verts, in_tris;  // staging for host geometry

@@ -3070,7 +3070,7 @@ int sah_build(rt_bvh* B, const rt_build_cfg& cfg, const SahInput& in, cudaStream
         S.sah_refs_a.ensure((size_t)cap * 4) || S.sah_refs_b.ensure((size_t)cap * 4) || S.sah_tmp.ensure((size_t)cap * 4) ||
         S.sah_pos.ensure((size_t)cap * 4) || S.sah_scan_in.ensure((size_t)cap) || S.sah_dec.ensure((size_t)cap * sizeof(Dec)) ||
         S.sah_out.ensure((size_t)2 * cap * sizeof(OutNode)) || S.sah_leaf_refs.ensure((size_t)cap * 4) ||
-        S.sah_scan_out.ensure((size_t)3 * cap * 4 + (size_t)2 * nr * 4 + 80) || S.sah_jobs.ensure((size_t)cap * sizeof(ClipJob)))
+        S.sah_scan_out.ensure((size_t)3 * cap * 4 + (size_t)2 * nr * 4 + 80))
     {
         return RT_E_CUDA;
     }
@@ -3239,7 +3239,9 @@ int sah_build(rt_bvh* B, const rt_build_cfg& cfg, const SahInput& in, cudaStream
         }
         const uint32_t eval_blocks = std::min<uint32_t>((n_cur + EVAL_WPB - 1) / EVAL_WPB, 8u * (uint32_t)device_sm_count());
         const uint32_t sms = (uint32_t)device_sm_count();
-        ClipJob* jobs = S.sah_jobs.as<ClipJob>();
+        // the clip jobs of a level (at most one a node) lie where its split writes the next level
+        static_assert(sizeof(ClipJob) <= sizeof(LvlNode) && alignof(ClipJob) <= alignof(LvlNode));
+        ClipJob* jobs = reinterpret_cast<ClipJob*>(lv_next);
         k_sah_eval_warp<true><<<eval_blocks, EVAL_WPB * 32, 0, st>>>(lv_cur, refs_cur, C, S.sah_dec.as<Dec>(), n_cur, io, jobs);
         if (n_cur <= CLIP_FEW * sms)
         {
