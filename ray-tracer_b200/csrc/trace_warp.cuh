@@ -171,13 +171,12 @@ struct LaneTrace
             cnt = left ? lcnt : rcnt;
             if (ft < best)
             {
-                // (the reference's 64-entry stack holds the nearer child too)
+                // (the reference's 64-entry stack holds the nearer child too; alone it always fits)
                 if (top + 1 >= STK) { overflow = true; live = false; return; }
                 stk[top++] = make_uint2(tref, __float_as_uint(ttn));
                 tref = (fcnt & LEAF_BIT) ? at : fref;
                 ttn = ft;
             }
-            else if (top >= STK) { overflow = true; live = false; }
         }
         else { pop(stk, gn); }
     }
@@ -291,8 +290,7 @@ __device__ __forceinline__ void warp_walk(LaneTrace<MODE, STK>& L, uint2 (&stk)[
                                           int serve)
 {
     constexpr unsigned FULL = 0xffffffffu;
-    uint32_t it = 0;
-    for (; it < 1024u; it++)
+    for (uint32_t it = 0; it < 1024u; it++)
     {
         const bool walk = L.live && !(L.cnt & LEAF_BIT);
         const unsigned walking = __ballot_sync(FULL, walk);
@@ -302,12 +300,15 @@ __device__ __forceinline__ void warp_walk(LaneTrace<MODE, STK>& L, uint2 (&stk)[
             const unsigned live = __ballot_sync(FULL, L.live);
             if (live != walking || __popc(takers & ~live) >= serve) { break; }
         }
-        if (walk) { L.step(stk, T.gn); }
+        if (walk)
+        {
+            L.step(stk, T.gn);
+            L.steps++;
+        }
         __syncwarp();
     }
     // A validated BVH is a DAG with children after parents; the cap only bounds the work a
-    // malformed one could cause.
-    L.steps += it;
+    // malformed one could cause. (Only the lane's own nodes count, not its waits for others.)
     if (L.live && L.steps > MAX_POPS) { L.overflow = true; L.live = false; }
 }
 

@@ -145,3 +145,41 @@ def test_axis_parallel_rays_cost_what_others_do():
 
     times = np.array([[once(rays), once(tilted)] for _ in range(24)])[4:]
     assert np.median(times[:, 0] / times[:, 1]) < 1.2, times
+
+
+def test_long_rays_among_others():
+    """The cap on a ray's steps counts its own nodes only. A few rays with 32,768 leaves share a warp with
+    rays of eight million nodes, for which they wait at every leaf: 2^24 rounds of the warp in all, and no
+    ray near the cap of 2^24. (The tree is a DAG: chains of nodes whose children are the next one.)"""
+    far = np.array([[100.0, 0, 0], [101.0, 1, 1]])
+
+    def box(x0, x1, z0, z1):
+        return np.array([[x0, 0.0, z0], [x1, 1.0, z1]])
+
+    recs = [[box(0, 3, 0, 3), 0, 0, 0], [box(1, 3, 0, 3), 0, 0, 0], [box(2, 3, 0, 3), 0, 0, 0]]
+
+    def chain(depth, b, leaf_box):  # `depth` inner nodes, the last with two equal leaves: 2^depth - 1 visits
+        first = len(recs)
+        recs.extend([b, 0, first + k + 1, first + k + 1] for k in range(depth))
+        recs.append([leaf_box, 1, 0, 1])
+        return first
+
+    near, deep = 15, 23
+    recs[0][2:] = [chain(near, box(0, 1, 0, 1), box(0, 1, 0, 1)), 1]
+    recs[1][2:] = [chain(deep, box(1, 2, 2, 3), far), 2]
+    recs[2][2:] = [chain(near - 1, box(2, 3, 0, 1), box(2, 3, 0, 1)), chain(deep, box(2, 3, 2, 3), far)]
+    nodes = np.zeros(len(recs), rtb200.NODE_DTYPE)
+    for i, (b, leaf, left, right) in enumerate(recs):
+        nodes["bmin"][i, :3], nodes["bmax"][i, :3] = b
+        nodes["is_leaf"][i], nodes["a"][i], nodes["b"][i] = leaf, left, right
+    verts = np.zeros((3, 6), np.float32)  # no area: every leaf is tested, none is hit
+    b = rtb200.Bvh.from_arrays(nodes, np.array([[0, 1, 2]], np.uint32), verts)
+    n = 151552  # a ray for each resident lane, by index: the first warp has the first 32
+    rays = torch.zeros(n, 8, device="cuda")
+    rays[:, 0], rays[:, 1], rays[:, 2], rays[:, 7] = 9.0, 0.5, -1.0, float("inf")
+    rays[:, 4], rays[:, 5], rays[:, 6] = 1e-3, 1e-3, 1.0
+    rays[:4, 0], rays[4:18, 0], rays[18:32, 0] = 0.5, 1.5, 2.5
+    hits = torch.full_like(rays, -1.0)
+    torch.cuda.synchronize()
+    assert rtb200.lib().rt_trace(b.h, rays.data_ptr(), hits.data_ptr(), n, 0, None) == 0, rtb200.lib().rt_last_error()
+    assert int(hits.view(torch.int32)[:, 7].abs().max()) == 0
