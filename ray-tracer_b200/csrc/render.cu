@@ -468,7 +468,7 @@ __device__ __forceinline__ void warp_add3(float* __restrict__ dst, uint32_t key,
 // at most) from the paths traced twice, whose runs differ by 0.3-1.1e-5; warps that trace together as the renderer's do (31 ms) move it by 0.5-4e-5,
 // paths traced by k_paths and replayed by a kernel of their own (35 ms) or other numbers of blocks by up to 3e-4.
 template <bool REC>
-__global__ void __launch_bounds__(128, 5)
+__global__ void __launch_bounds__(128, REC ? 5 : 1)
 k_adjoint(TraceCtx T, RP P, Shade S, const float* __restrict__ dimg, float* __restrict__ g_alb, float* __restrict__ g_em)
 {
     const uint32_t x = blockIdx.x * 16 + (threadIdx.x & 15);
