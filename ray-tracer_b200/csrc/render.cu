@@ -653,8 +653,13 @@ int run_paths(const rt_bvh* B, PathJob J, const Cam* h_cams, const rt_wavefront_
         // graph as a child or twice at a time.
         return own_pixels();
     }
-    // (a warm-up call loads what a captured one launches)
-    blocks_per_sm(reinterpret_cast<const void*>(k_paths<STACK, true>), (int)W.trace_block, (W.trace_block / 32) * sizeof(PathShare));
+    // (Asked for in every call: a warm-up also loads the kernel that a captured call launches.)
+    // One sample of an image that the chip holds at once: the lanes own their pixels just as well, and that
+    // needs one launch instead of two, a clear and scratch.
+    const uint64_t warps = (uint64_t)device_sm_count() *
+                           blocks_per_sm(reinterpret_cast<const void*>(k_paths<STACK, true>), (int)W.trace_block,
+                                         (W.trace_block / 32) * sizeof(PathShare)) * (W.trace_block / 32);
+    if (J.P.spp == 1 && !h_cams && per_sample <= warps * 32) { return own_pixels(); }
     // cameras, item counter, radiance
     const uint64_t cam_bytes = h_cams ? (J.S * sizeof(Cam) + 255) / 256 * 256 : 0, head = cam_bytes + 256;
     uint64_t group = std::max<uint64_t>(1, std::min<uint64_t>(W.chunk_paths / per_sample, J.P.spp));

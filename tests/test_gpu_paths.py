@@ -102,3 +102,24 @@ def test_short_albedo_table():
     a = b.render(rc, mats, mot, tri_albedo=full)[0]
     c = b.render(rc, mats, mot, tri_albedo=full[:n // 2])[0]
     assert torch.equal(a, c)
+
+
+@pytest.mark.parametrize("w,h", [(1, 1), (8, 4), (61, 43), (256, 256)])
+def test_one_sample_of_a_small_image(w, h):
+    """One launch, and the sample that an image of two samples has."""
+    import torch
+    b, mats, mot = scene("hybrid")
+    dm, dmot = torch.from_numpy(rtb200.materials_array(mats)).cuda(), torch.from_numpy(mot.astype(np.int32)).cuda()
+
+    def render(spp, offset):
+        rc = rtb200.render_cfg(w, h, spp, max_bounce=4, rr_after=1, env_kind=1, env_color=(0.1, 0.2, 0.3), seed=w, sample_offset=offset,
+                               lookat=VIEW)
+        n = rtb200.lib().rt_kernel_launches()
+        out = b.render(rc, dm, dmot, want_sq=True)
+        return out, rtb200.lib().rt_kernel_launches() - n
+
+    (x, x2), n0 = render(1, 3)
+    (y, y2), n1 = render(1, 4)
+    (z, z2), _ = render(2, 3)
+    assert (n0, n1) == (1, 1)
+    assert torch.equal((x + y) / 2, z) and torch.equal((x2 + y2) / 2, z2)
