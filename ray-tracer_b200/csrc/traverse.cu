@@ -214,22 +214,26 @@ k_trace(TraceCtx T, const float4* __restrict__ rays, float4* __restrict__ hits, 
     }
 }
 
-// The 8-wide layout's kernel: each warp claims 32 rays at a time until the batch is exhausted.
+// The 8-wide layout's kernel: each warp claims 32 rays at a time until the batch is exhausted; without a
+// counter it traces the `per_warp` of its own index.
 template <int MODE>
 __global__ void __launch_bounds__(256)
 k_trace_wide(TraceCtx T, const float4* __restrict__ rays, float4* __restrict__ hits, uint64_t n,
-             unsigned long long* __restrict__ counter, uint32_t* __restrict__ status, int)
+             unsigned long long* __restrict__ counter, uint32_t* __restrict__ status, int per_warp)
 {
     const int lane = threadIdx.x & 31;
     const TraceRoot R = *T.root;
-    for (;;)
+    for (bool more = true; more; more = counter != nullptr)
     {
-        unsigned long long base = 0;
-        if (lane == 0) { base = atomicAdd(counter, 32ull); }
-        base = __shfl_sync(0xffffffffu, base, 0);
+        unsigned long long base = ((uint64_t)blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5)) * (uint64_t)per_warp;
+        if (counter)
+        {
+            if (lane == 0) { base = atomicAdd(counter, 32ull); }
+            base = __shfl_sync(0xffffffffu, base, 0);
+        }
         if (base >= n) { return; }
         const uint64_t ri = base + (uint64_t)lane;
-        if (ri >= n) { continue; }
+        if (ri >= n || lane >= per_warp) { continue; }
         const float4 r0 = rays[2 * ri], r1 = rays[2 * ri + 1];
         const THit H = trace_ray_wide<MODE, STACK>(T, R, mk3(r0.x, r0.y, r0.z), mk3(r1.x, r1.y, r1.z), r0.w, r1.w);
         write_hit(T, hits, ri, H.hit, H.overflow, H.t, H.u, H.v, H.tri, status);
@@ -376,7 +380,7 @@ int trace(const rt_bvh* B, const rt_ray* d_rays, rt_hit* d_hits, uint64_t n, uin
     // a ray still test its leaves' triangles. Every warp then has its rays at once, so they are
     // assigned by index: no counter to clear before the launch and to wait for at its start.
     const uint64_t warps = grid * WPB;
-    const bool few = !B->trace_wide && n <= warps * 32;
+    const bool few = n <= warps * 32;
     const uint64_t per_warp = few ? std::max<uint64_t>(1, (n + warps - 1) / warps) : 32;
     grid = std::min(grid, (n + per_warp * WPB - 1) / (per_warp * WPB));
     // The counter is the call's own: calls on a handle may run at the same time.

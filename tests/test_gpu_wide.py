@@ -221,3 +221,13 @@ def test_wide_batched_roots():
     a, c = img_bin.cpu().numpy(), img_wide.cpu().numpy()
     assert np.mean(np.abs(a - c)) <= 1e-3 * max(float(np.mean(np.abs(a))), 1e-6)
     assert np.mean(np.isclose(a, c, rtol=1e-5, atol=1e-6)) > 0.999
+
+
+@pytest.mark.parametrize("n", [1, 31, 33, 1000, 4737, 151553])
+def test_wide_ray_counts(orc, n):
+    """Few rays, spread over the resident warps, and more than a chip full, claimed from a counter."""
+    v, t = SCENES["soup20k"]
+    b = rtb200.Bvh.build(v, t, "sah4")
+    b.trace_loop(2)
+    rays = rays_for(v, max(n, 8), seed=n)[:n]
+    check_wide(b.trace(rays), orc.trace(Baked(*b.download()), rays, threads=8), f"n={n}")
