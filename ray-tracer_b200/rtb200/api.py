@@ -394,7 +394,7 @@ class Bvh:
         import torch
         rgb = torch.empty((rcfg.height, rcfg.width, 3), dtype=torch.float32, device="cuda")
         rgb2 = torch.empty_like(rgb) if want_sq else None
-        sh, keep = _shading(mats, mat_of_tri, tri_albedo, env_map, self.counts()[1])
+        sh, keep = _shading(mats, mat_of_tri, tri_albedo, env_map, bvh=self)
         _check(lib().rt_render_ex(self.h, C.byref(rcfg), C.byref(sh), mode, _ptr(rgb), _ptr(rgb2),
                                   _stream_ptr(stream, True)))
         del keep
@@ -410,7 +410,7 @@ class Bvh:
         assert d_rgb.is_cuda and d_rgb.numel() == rcfg.width * rcfg.height * 3
         g_alb = torch.zeros((nt, 3), dtype=torch.float32, device="cuda")
         g_em = torch.zeros((len(mats), 3), dtype=torch.float32, device="cuda") if mats is not None else None
-        sh, keep = _shading(mats, mat_of_tri, tri_albedo, n_tris=nt)
+        sh, keep = _shading(mats, mat_of_tri, tri_albedo, bvh=self)
         _check(lib().rt_adjoint(self.h, C.byref(rcfg), C.byref(sh), _ptr(d_rgb), _ptr(g_alb), _ptr(g_em),
                                 _stream_ptr(stream, True)))
         del keep
@@ -427,7 +427,7 @@ class Bvh:
         c0 = rcfgs[0]
         rgb = torch.empty((n, c0.height, c0.width, 3), dtype=torch.float32, device="cuda")
         rgb2 = torch.empty_like(rgb) if want_sq else None
-        sh, keep = _shading(mats, mat_of_tri, tri_albedo, n_tris=self.counts()[1])
+        sh, keep = _shading(mats, mat_of_tri, tri_albedo, bvh=self)
         _check(lib().rt_render_batch(self.h, arr, n, C.byref(sh), C.byref(params) if params is not None else None,
                                      _ptr(rgb), _ptr(rgb2), _stream_ptr(stream, True)))
         del keep
@@ -498,9 +498,9 @@ def _device_u32(x):
     return torch.from_numpy(np.ascontiguousarray(x, np.uint32).view(np.int32)).cuda()
 
 
-def _shading(mats, mat_of_tri, tri_albedo, env_map=None, n_tris=0):
+def _shading(mats, mat_of_tri, tri_albedo, env_map=None, bvh=None):
     """An rt_shading record over device copies of the inputs (kept alive by the caller). An albedo
-    table with fewer than n_tris rows (baked triangles: spatial splits add some) is continued in
+    table with fewer rows than bvh has triangles (baked ones: spatial splits add some) is continued in
     black, so that no kernel reads past it."""
     import torch
     sh = Shading()
@@ -521,6 +521,7 @@ def _shading(mats, mat_of_tri, tri_albedo, env_map=None, n_tris=0):
     if tri_albedo is not None:
         ta = tri_albedo.detach() if _is_torch(tri_albedo) else torch.from_numpy(np.ascontiguousarray(tri_albedo, np.float32))
         ta = ta.to(device="cuda", dtype=torch.float32).contiguous()
+        n_tris = bvh.counts()[1]
         if ta.numel() < 3 * n_tris:
             ta = torch.cat([ta.reshape(-1), ta.new_zeros(3 * n_tris - ta.numel())])
         keep.append(ta)
