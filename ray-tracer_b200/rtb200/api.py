@@ -394,7 +394,7 @@ class Bvh:
         import torch
         rgb = torch.empty((rcfg.height, rcfg.width, 3), dtype=torch.float32, device="cuda")
         rgb2 = torch.empty_like(rgb) if want_sq else None
-        sh, keep = _shading(mats, mat_of_tri, tri_albedo, env_map, bvh=self)
+        sh, keep = _shading(mats, mat_of_tri, tri_albedo, env_map, bvh=self, stream=stream)
         _check(lib().rt_render_ex(self.h, C.byref(rcfg), C.byref(sh), mode, _ptr(rgb), _ptr(rgb2),
                                   _stream_ptr(stream, True)))
         del keep
@@ -406,11 +406,12 @@ class Bvh:
         CUDA tensors, indexed like tri_albedo / mats."""
         import torch
         _, nt, _ = self.counts()
-        d_rgb = d_rgb.contiguous().to(torch.float32)
+        given, d_rgb = d_rgb, d_rgb.contiguous().to(torch.float32)
         assert d_rgb.is_cuda and d_rgb.numel() == rcfg.width * rcfg.height * 3
         g_alb = torch.zeros((nt, 3), dtype=torch.float32, device="cuda")
         g_em = torch.zeros((len(mats), 3), dtype=torch.float32, device="cuda") if mats is not None else None
-        sh, keep = _shading(mats, mat_of_tri, tri_albedo, bvh=self)
+        made = [t for t in (g_alb, g_em, d_rgb) if t is not None and t.data_ptr() != given.data_ptr()]
+        sh, keep = _shading(mats, mat_of_tri, tri_albedo, bvh=self, stream=stream, made=made)
         _check(lib().rt_adjoint(self.h, C.byref(rcfg), C.byref(sh), _ptr(d_rgb), _ptr(g_alb), _ptr(g_em),
                                 _stream_ptr(stream, True)))
         del keep
@@ -427,7 +428,7 @@ class Bvh:
         c0 = rcfgs[0]
         rgb = torch.empty((n, c0.height, c0.width, 3), dtype=torch.float32, device="cuda")
         rgb2 = torch.empty_like(rgb) if want_sq else None
-        sh, keep = _shading(mats, mat_of_tri, tri_albedo, bvh=self)
+        sh, keep = _shading(mats, mat_of_tri, tri_albedo, bvh=self, stream=stream)
         _check(lib().rt_render_batch(self.h, arr, n, C.byref(sh), C.byref(params) if params is not None else None,
                                      _ptr(rgb), _ptr(rgb2), _stream_ptr(stream, True)))
         del keep
@@ -437,7 +438,7 @@ class Bvh:
         n = len(rcfgs)
         arr = (RenderCfg * n)(*rcfgs)
         best = WavefrontParams()
-        sh, keep = _shading(mats, mat_of_tri, None)
+        sh, keep = _shading(mats, mat_of_tri, None, stream=stream)
         _check(lib().rt_autotune_wavefront(self.h, arr, n, C.byref(sh), C.byref(best), _stream_ptr(stream, True)))
         del keep
         return best
@@ -498,25 +499,46 @@ def _device_u32(x):
     return torch.from_numpy(np.ascontiguousarray(x, np.uint32).view(np.int32)).cuda()
 
 
-def _shading(mats, mat_of_tri, tri_albedo, env_map=None, bvh=None):
-    """An rt_shading record over device copies of the inputs (kept alive by the caller). An albedo
+def _hand_over(stream, made):
+    """Tensors that a call has made on torch's current stream, to the stream it runs on: that one waits
+    for them, and their memory is not used again before it is done."""
+    if stream is None or not made:
+        return
+    import torch
+    s = stream if hasattr(stream, "cuda_stream") else torch.cuda.ExternalStream(int(stream))
+    current = torch.cuda.current_stream()
+    if s.cuda_stream != current.cuda_stream:
+        s.wait_stream(current)
+        for t in made:
+            t.record_stream(s)
+
+
+def _shading(mats, mat_of_tri, tri_albedo, env_map=None, bvh=None, stream=None, made=()):
+    """An rt_shading record over device copies of the inputs (kept alive by the caller), handed over to
+    the call's stream with the tensors in `made`. An albedo
     table with fewer rows than bvh has triangles (baked ones: spatial splits add some) is continued in
     black, so that no kernel reads past it."""
     import torch
     sh = Shading()
-    keep = []
+    keep, made = [], list(made)
+
+    def add(t, given):
+        keep.append(t)
+        if not (_is_torch(given) and given.data_ptr() == t.data_ptr()):
+            made.append(t)
+
     if env_map is not None:
         em = env_map if _is_torch(env_map) else torch.from_numpy(np.ascontiguousarray(env_map, np.float32))
         em = em.to(device="cuda", dtype=torch.float32).contiguous()
-        keep.append(em)
+        add(em, env_map)
         sh.env_map, sh.env_h, sh.env_w = em.data_ptr(), int(em.shape[0]), int(em.shape[1])
     if mats is not None:
         dm = mats.contiguous().cuda() if _is_torch(mats) else torch.from_numpy(materials_array(mats)).cuda()
-        keep.append(dm)
+        add(dm, mats)
         sh.mats, sh.n_mats = dm.data_ptr(), int(dm.shape[0])
         if mat_of_tri is not None:
             dmot = _device_u32(mat_of_tri)
-            keep.append(dmot)
+            add(dmot, mat_of_tri)
             sh.mat_of_tri = dmot.data_ptr()
     if tri_albedo is not None:
         ta = tri_albedo.detach() if _is_torch(tri_albedo) else torch.from_numpy(np.ascontiguousarray(tri_albedo, np.float32))
@@ -524,8 +546,9 @@ def _shading(mats, mat_of_tri, tri_albedo, env_map=None, bvh=None):
         n_tris = bvh.counts()[1]
         if ta.numel() < 3 * n_tris:
             ta = torch.cat([ta.reshape(-1), ta.new_zeros(3 * n_tris - ta.numel())])
-        keep.append(ta)
+        add(ta, tri_albedo)
         sh.tri_albedo = ta.data_ptr()
+    _hand_over(stream, made)
     return sh, keep
 
 

@@ -123,3 +123,28 @@ def test_one_sample_of_a_small_image(w, h):
     (z, z2), _ = render(2, 3)
     assert (n0, n1) == (1, 1)
     assert torch.equal((x + y) / 2, z) and torch.equal((x2 + y2) / 2, z2)
+
+
+def test_tensors_made_for_a_call_on_another_stream():
+    """The rest of a short albedo table and the gradients' zeros are made on the current stream, which
+    is busy, and used on the call's; their memory is not handed out again while that one works."""
+    import torch
+    b, mats, mot = scene()
+    rc = rtb200.render_cfg(64, 48, 64, max_bounce=4, rr_after=-1, env_kind=1, env_color=(0.4, 0.5, 0.6), seed=2, lookat=VIEW)
+    n = mot.shape[0]
+    mats, mot = torch.from_numpy(rtb200.materials_array(mats)).cuda(), torch.from_numpy(mot.astype(np.int32)).cuda()
+    alb = torch.rand(n // 2, 3, device="cuda")
+    d = torch.ones(48, 64, 3, device="cuda")
+    want = b.render(rc, mats, mot, tri_albedo=alb)[0]
+    grad = b.adjoint(rc, d, mats, mot, tri_albedo=alb)
+    side = torch.cuda.Stream()
+    torch.cuda.synchronize()
+    torch.cuda._sleep(1 << 28)  # the current stream is busy for about 0.15 s
+    got = b.render(rc, mats, mot, tri_albedo=alb, stream=side)[0]
+    fill = [torch.full((n, 3), 7.0, device="cuda") for _ in range(8)]
+    g = b.adjoint(rc, d, mats, mot, tri_albedo=alb, stream=side.cuda_stream)
+    fill += [torch.full((n, 3), 7.0, device="cuda") for _ in range(8)]
+    torch.cuda.synchronize()
+    assert torch.equal(got, want)
+    for x, y in zip(g, grad):  # float sums of the same terms in other orders
+        assert float((x.double() - y.double()).norm()) <= 1e-4 * float(y.double().norm())
