@@ -274,10 +274,12 @@ typedef struct rt_wavefront_params
  * handle from rt_build renders as one scene. */
 int rt_render_batch(rt_bvh* bvh, const rt_render_cfg* cfgs, uint32_t n_scenes, const rt_shading* shading,
                     const rt_wavefront_params* params, float* rgb, float* rgb2, void* stream);
-/* Times each candidate parameter set (trace block 64/128/256, chunk 1-8 Mi paths, stack
- * 32/64 where the tree allows) on a short render of the batch -- enough samples per pixel for
- * 8 Mi paths, at most the configuration's own -- and keeps the fastest in the handle (and in
- * *best). */
+/* Times candidate parameter sets -- the default, each trace block (64/128/256) with each stack (32 where
+ * the tree allows, 64), then the best of these with chunks of 1 to 32 Mi paths -- on a short render of
+ * the batch -- enough samples per pixel for 32 Mi paths, at most the configuration's own -- and keeps the
+ * fastest in the handle (and in *best), the default unless another is at least 2 % faster. Of chunks
+ * that hold the whole render the smallest tried is reported; a later render of more paths takes the
+ * default's chunk where it is larger. */
 int rt_autotune_wavefront(rt_bvh* bvh, const rt_render_cfg* cfgs, uint32_t n_scenes, const rt_shading* shading,
                           rt_wavefront_params* best, void* stream);
 

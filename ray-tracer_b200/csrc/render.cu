@@ -607,6 +607,12 @@ int check_params(const rt_wavefront_params& W)
     return RT_OK;
 }
 
+// Items of one sample of S images (tiles cover them).
+uint64_t sample_items(const rt_render_cfg& c, uint32_t S)
+{
+    return ((uint64_t)c.width + 7) / 8 * (((uint64_t)c.height + 3) / 4) * 32 * S;
+}
+
 using PathFn = void (*)(TraceCtx, PathJob, uint32_t*, int);
 
 int launch_paths(PathFn fn, const TraceCtx& T, const PathJob& J, uint32_t* counter, uint32_t block, cudaStream_t st)
@@ -698,13 +704,20 @@ int run_paths(const rt_bvh* B, PathJob J, const Cam* h_cams, const rt_wavefront_
     return RT_OK;
 }
 
-// A valid parameter set for this handle: the tuned one, else the defaults (with the
-// stack the tree needs).
-rt_wavefront_params pick_params(const rt_bvh* B, const rt_wavefront_params* W)
+// A valid parameter set for a render of this handle: the tuned one, else the defaults (with the
+// stack the tree needs). A larger job than the tuning's has no measurement of its own launches: it takes
+// the default's at least.
+rt_wavefront_params pick_params(const rt_bvh* B, const rt_wavefront_params* W, const rt_render_cfg& c, uint32_t S)
 {
     if (W) { return *W; }
-    if (B->wf_tuned_valid) { return B->wf_tuned; }
-    return default_params();
+    rt_wavefront_params P = default_params();
+    if (B->wf_tuned_valid)
+    {
+        const uint32_t chunk = P.chunk_paths;
+        P = B->wf_tuned;
+        if (sample_items(c, S) * c.spp > B->wf_tuned_paths) { P.chunk_paths = std::max(P.chunk_paths, chunk); }
+    }
+    return P;
 }
 
 } // namespace
@@ -718,7 +731,7 @@ int render(const rt_bvh* B, const rt_render_cfg& cfg, const rt_shading& sh, int 
     J.P = make_rp(cfg, sh);
     J.S = 1;
     J.sh = Shade{ sh.mats, sh.mat_of_tri, sh.tri_albedo, sh.n_mats };
-    rt_wavefront_params W = mode == RT_RENDER_WAVEFRONT ? pick_params(B, nullptr) : default_params();
+    rt_wavefront_params W = mode == RT_RENDER_WAVEFRONT ? pick_params(B, nullptr, cfg, 1) : default_params();
     W.stack_depth = 64;  // tuned for a batch; a plain handle keeps the full stack
     return run_paths(B, J, nullptr, W, rgb, rgb2, st);
 }
@@ -728,7 +741,7 @@ int render_batch(rt_bvh* B, const rt_render_cfg* cfgs, uint32_t S, const rt_shad
 {
     const rt_render_cfg& c0 = cfgs[0];
     if (c0.max_bounce > MAX_WAVEFRONT_BOUNCE) { return fail(RT_E_INVALID, "max_bounce must be below 63 for the wavefront"); }
-    const rt_wavefront_params W = pick_params(B, params);
+    const rt_wavefront_params W = pick_params(B, params, c0, S);
     if (int e = check_params(W)) { return e; }
     if (W.stack_depth < 64)
     {
@@ -751,58 +764,71 @@ int autotune_wavefront(rt_bvh* B, const rt_render_cfg* cfgs, uint32_t S, const r
 {
     uint32_t depth = 0;
     if (int e = tree_depth(B, st, &depth)) { return e; }
-    const uint32_t blocks[] = { 64, 128, 256 };
-    const uint32_t chunks[] = { 1u << 20, 1u << 21, 1u << 22, 1u << 23 };
+    const uint32_t chunks[] = { 1u << 20, 1u << 21, 1u << 22, 1u << 23, 1u << 24, 1u << 25 };
     // trial renders with enough samples per pixel that the largest chunk fills (a one-sample
     // trial of a small image cannot tell the chunk sizes apart), at most the configs' own
-    uint64_t px = 0;
-    for (uint32_t k = 0; k < S; k++) { px += (uint64_t)cfgs[k].width * cfgs[k].height; }
-    const uint64_t want = px ? (((uint64_t)chunks[3] + px - 1) / px) : 1;
+    const uint64_t items = sample_items(cfgs[0], S), largest = chunks[5];
     std::vector<rt_render_cfg> c1(cfgs, cfgs + S);
     for (auto& c : c1)
     {
-        c.spp = (uint32_t)std::max<uint64_t>(1, std::min<uint64_t>(want, c.spp));
+        c.spp = (uint32_t)std::max<uint64_t>(1, std::min<uint64_t>((largest + items - 1) / items, c.spp));
         c.sample_offset = 0;
     }
-    const uint32_t stacks[] = { 32, 64 };
+    // chunks that hold the whole trial launch the same: the smallest of them stands for all, the default's too
+    uint32_t whole = 0;
+    while (chunks[whole] < items * c1[0].spp && whole < 5) { whole++; }
     cudaEvent_t a, b;
     RT_CUDA(cudaEventCreate(&a));
     RT_CUDA(cudaEventCreate(&b));
-    float best_ms = 1e30f;
-    rt_wavefront_params bw = default_params();
     int err = RT_OK;
-    for (uint32_t stack : stacks)
-    {
-        if (stack < 64 && depth + 1 > stack) { continue; }
-        for (uint32_t blk : blocks)
+    auto time = [&](const rt_wavefront_params& W) {  // the faster of two runs
+        float best_ms = 1e30f;
+        for (int rep = 0; rep < 2 && !err; rep++)
         {
-            for (uint32_t ch : chunks)
-            {
-                rt_wavefront_params W = default_params();
-                W.trace_block = blk; W.chunk_paths = ch; W.stack_depth = stack;
-                float ms = 0.f;
-                for (int rep = 0; rep < 2 && !err; rep++)  // the first run warms up
-                {
-                    if (cudaEventRecord(a, st) != cudaSuccess) { err = fail(RT_E_CUDA, "event"); break; }
-                    err = render_batch(B, c1.data(), S, sh, &W, scratch_rgb, nullptr, st);
-                    if (err) { break; }
-                    if (cudaEventRecord(b, st) != cudaSuccess || cudaEventSynchronize(b) != cudaSuccess)
-                    {
-                        err = fail(RT_E_CUDA, "event"); break;
-                    }
-                    cudaEventElapsedTime(&ms, a, b);
-                }
-                if (err) { break; }
-                if (ms < best_ms) { best_ms = ms; bw = W; }
-            }
+            if (cudaEventRecord(a, st) != cudaSuccess) { err = fail(RT_E_CUDA, "event"); break; }
+            err = render_batch(B, c1.data(), S, sh, &W, scratch_rgb, nullptr, st);
             if (err) { break; }
+            if (cudaEventRecord(b, st) != cudaSuccess || cudaEventSynchronize(b) != cudaSuccess) { err = fail(RT_E_CUDA, "event"); break; }
+            float ms = 0.f;
+            cudaEventElapsedTime(&ms, a, b);
+            best_ms = std::min(best_ms, ms);
         }
-        if (err) { break; }
+        return best_ms;
+    };
+    rt_wavefront_params bw = default_params();
+    bw.chunk_paths = chunks[whole];
+    const rt_wavefront_params dw = bw;
+    time(bw);
+    const float default_ms = time(bw);
+    float best_ms = default_ms;
+    auto trial = [&](const rt_wavefront_params& W) {
+        if (err || std::memcmp(&W, &dw, sizeof(W)) == 0) { return; }
+        const float ms = time(W);
+        if (!err && ms < best_ms) { best_ms = ms; bw = W; }
+    };
+    // the block and the stack at the default's chunk, then the chunk
+    for (const uint32_t stack : { 32u, 64u })
+    {
+        for (const uint32_t block : { 64u, 128u, 256u })
+        {
+            rt_wavefront_params W = dw;
+            W.trace_block = block; W.stack_depth = stack;
+            if (stack == 64 || depth + 1 <= stack) { trial(W); }
+        }
     }
+    const rt_wavefront_params shape = bw;
+    for (uint32_t k = 0; k < whole; k++)
+    {
+        rt_wavefront_params W = shape;
+        W.chunk_paths = chunks[k];
+        trial(W);
+    }
+    if (best_ms > 0.98f * default_ms) { bw = dw; }  // (closer times are the runs' own spread)
     cudaEventDestroy(a);
     cudaEventDestroy(b);
     if (err) { return err; }
     B->wf_tuned = bw;
+    B->wf_tuned_paths = c1[0].spp < cfgs[0].spp ? ~0ull : items * cfgs[0].spp;
     B->wf_tuned_valid = true;
     if (best) { *best = bw; }
     return RT_OK;

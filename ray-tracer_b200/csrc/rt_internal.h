@@ -254,6 +254,7 @@ struct rt_bvh
     cudaEvent_t  bake_ev[2] = { nullptr, nullptr };
     rt_wavefront_params wf_tuned = { 0, 0, 0, 0 };
     bool         wf_tuned_valid = false;
+    uint64_t     wf_tuned_paths = 0;        // jobs of up to this many were measured
     // stage timing (rt_bvh_profile): events at the stage boundaries of a build
     bool         prof = false;
     cudaEvent_t  ev[8] = { nullptr, nullptr, nullptr, nullptr, nullptr, nullptr, nullptr, nullptr };
