@@ -207,9 +207,28 @@ __device__ __forceinline__ bool shade(const TraceCtx& T, const RP& P, const Shad
     return true;
 }
 
-// What one launch of k_paths works on. Items are numbered sample by sample, scene by scene, and in
-// 8 x 4 pixel tiles (neighbouring lanes start with neighbouring pixels); items of a tile that lie
-// outside the image are skipped.
+// Pixels of an image in tiles of 32: 8 x 4 (neighbouring lanes start with neighbouring pixels), or one
+// pixel wide or high where that takes fewer items (a very narrow or low image would take up to
+// eight times its pixels).
+struct Tiles
+{
+    uint32_t lw, tiles_x;  // log2 of a tile's width, tiles in a row
+    uint64_t items;        // all tiles' pixels
+};
+
+Tiles make_tiles(uint32_t w, uint32_t h)
+{
+    Tiles best{ 0, 0, ~0ull };
+    for (const uint32_t lw : { 3u, 0u, 5u })
+    {
+        const uint64_t tx = ((uint64_t)w + (1u << lw) - 1) >> lw, ty = ((uint64_t)h + (32u >> lw) - 1) >> (5 - lw);
+        if (tx * ty * 32 < best.items) { best = Tiles{ lw, (uint32_t)tx, tx * ty * 32 }; }
+    }
+    return best;
+}
+
+// What one launch of k_paths works on. Items are numbered sample by sample, scene by scene and tile by
+// tile; items of a tile that lie outside the image are skipped.
 struct PathJob
 {
     RP               P;
@@ -217,7 +236,7 @@ struct PathJob
     const Cam*       cams;     // per scene (nullptr: P.cam)
     const TraceRoot* roots;    // per scene (nullptr: the handle's root)
     uint32_t         S;        // scenes
-    uint32_t         tiles_x, scene_items;
+    uint32_t         tile_lw, tiles_x, scene_items;
     uint32_t         sample0;  // sample of item 0, from P.sample_offset
     uint32_t         first, n; // this launch's items
     float*           rad;      // radiance per path: [sample - sample0][scene][pixel][3]
@@ -264,7 +283,8 @@ k_paths(const TraceCtx T, const __grid_constant__ PathJob J, uint32_t* __restric
     auto begin = [&](uint32_t item, uint32_t s, float4& r0, float4& r1) -> bool {
         const uint32_t sc = item / J.scene_items;
         const uint32_t q = item - sc * J.scene_items, tile = q >> 5, ty = tile / J.tiles_x;
-        const uint32_t x = (tile - ty * J.tiles_x) * 8u + (q & 7u), y = ty * 4u + ((q >> 3) & 3u);
+        const uint32_t lw = J.tile_lw, p = q & 31u;
+        const uint32_t x = ((tile - ty * J.tiles_x) << lw) + (p & ((1u << lw) - 1u)), y = (ty << (5u - lw)) + (p >> lw);
         if (x >= J.P.W || y >= J.P.H) { return false; }
         const uint32_t pix = y * J.P.W + x, sidx = J.P.sample_offset + J.sample0 + s;
         f3 o, d;
@@ -607,12 +627,6 @@ int check_params(const rt_wavefront_params& W)
     return RT_OK;
 }
 
-// Items of one sample of S images (tiles cover them).
-uint64_t sample_items(const rt_render_cfg& c, uint32_t S)
-{
-    return ((uint64_t)c.width + 7) / 8 * (((uint64_t)c.height + 3) / 4) * 32 * S;
-}
-
 using PathFn = void (*)(TraceCtx, PathJob, uint32_t*, int);
 
 int launch_paths(PathFn fn, const TraceCtx& T, const PathJob& J, uint32_t* counter, uint32_t block, cudaStream_t st)
@@ -639,11 +653,12 @@ int run_paths(const rt_bvh* B, PathJob J, const Cam* h_cams, const rt_wavefront_
               cudaStream_t st)
 {
     const uint64_t npix = (uint64_t)J.P.W * J.P.H;
-    const uint64_t tiles_x = ((uint64_t)J.P.W + 7) / 8, items = tiles_x * (((uint64_t)J.P.H + 3) / 4) * 32;
-    if (items * J.S > 0xffffffffull) { return fail(RT_E_CAPACITY, "more than 2^32 pixels"); }
-    J.tiles_x = (uint32_t)tiles_x;
-    J.scene_items = (uint32_t)items;
-    const uint64_t per_sample = items * J.S;
+    const Tiles tiles = make_tiles(J.P.W, J.P.H);
+    if (tiles.items > 0xffffffffull / J.S) { return fail(RT_E_CAPACITY, "more than 2^32 pixels"); }
+    J.tile_lw = tiles.lw;
+    J.tiles_x = tiles.tiles_x;
+    J.scene_items = (uint32_t)tiles.items;
+    const uint64_t per_sample = tiles.items * J.S;
     const TraceCtx T = make_trace_ctx(B);
     auto own_pixels = [&]() {
         J.rgb = rgb; J.rgb2 = rgb2;
@@ -715,7 +730,7 @@ rt_wavefront_params pick_params(const rt_bvh* B, const rt_wavefront_params* W, c
     {
         const uint32_t chunk = P.chunk_paths;
         P = B->wf_tuned;
-        if (sample_items(c, S) * c.spp > B->wf_tuned_paths) { P.chunk_paths = std::max(P.chunk_paths, chunk); }
+        if (make_tiles(c.width, c.height).items * S * c.spp > B->wf_tuned_paths) { P.chunk_paths = std::max(P.chunk_paths, chunk); }
     }
     return P;
 }
@@ -767,7 +782,7 @@ int autotune_wavefront(rt_bvh* B, const rt_render_cfg* cfgs, uint32_t S, const r
     const uint32_t chunks[] = { 1u << 20, 1u << 21, 1u << 22, 1u << 23, 1u << 24, 1u << 25 };
     // trial renders with enough samples per pixel that the largest chunk fills (a one-sample
     // trial of a small image cannot tell the chunk sizes apart), at most the configs' own
-    const uint64_t items = sample_items(cfgs[0], S), largest = chunks[5];
+    const uint64_t items = make_tiles(cfgs[0].width, cfgs[0].height).items * S, largest = chunks[5];
     std::vector<rt_render_cfg> c1(cfgs, cfgs + S);
     for (auto& c : c1)
     {

@@ -148,3 +148,27 @@ def test_tensors_made_for_a_call_on_another_stream():
     assert torch.equal(got, want)
     for x, y in zip(g, grad):  # float sums of the same terms in other orders
         assert float((x.double() - y.double()).norm()) <= 1e-4 * float(y.double().norm())
+
+
+@pytest.mark.parametrize("w,h", [(1, 33), (3, 70), (7, 4), (33, 1), (100, 3), (9, 5)])
+def test_narrow_and_low_images_match_oracle(orc, w, h):
+    b, mats, mot = scene()
+    rc = rtb200.render_cfg(w, h, 8, max_bounce=3, rr_after=1, env_kind=1, env_color=(0.1, 0.2, 0.3), seed=w, lookat=VIEW)
+    rgb, rgb2 = b.render(rc, mats, mot, want_sq=True)
+    ref, ref2 = orc.render(Baked(*b.download()), orc_cfg_from(rc), mats, mot, threads=8, want_sq=True)
+    compare(rgb, rgb2, ref, ref2, 8, f"{w}x{h}", min_equal=0.0)
+
+
+@pytest.mark.parametrize("w,h", [(1, 600_000_000), (1_200_000_000, 1)])
+def test_long_thin_images(w, h):
+    """Every pixel of an image far longer than wide is rendered: the background, with the scene behind the
+    camera."""
+    import torch
+    b, _, _ = scene()
+    rc = rtb200.render_cfg(w, h, 1, max_bounce=1, rr_after=-1, env_kind=1, env_color=(0.25, 0.5, 0.75), seed=1,
+                           lookat=((0.0, 0.0, -9.0), (0.0, 0.0, -10.0), 45.0))
+    img = b.render(rc)[0].reshape(-1, 3)
+    for c in range(3):
+        assert torch.aminmax(img[:, c]) == (0.25 * (c + 1), 0.25 * (c + 1))
+    del img
+    torch.cuda.empty_cache()
