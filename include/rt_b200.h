@@ -188,8 +188,8 @@ void rt_camera_quat(const float pos[3], const float q_wxyz[4], float focal, rt_r
  * (rt_autotune_wavefront), RT_RENDER_PLAIN the defaults. Calls on one handle may come from several
  * streams and host threads. A render takes device memory for the time it runs: 12 bytes for each of
  * the paths of a launch (chunk_paths, by default 2^25; at least one per pixel), at most 403 MB up to 2^25 pixels.
- * It is stream-ordered memory of a pool per device, which keeps at most 512 MB between calls and is emptied
- * when the last handle is freed. With less memory left a render takes smaller launches, at last
+ * It is stream-ordered memory of a pool per device, which keeps at most 512 MB between calls and 64 MB
+ * once the last handle is freed. With less memory left a render takes smaller launches, at last
  * none. A render that is captured into a CUDA graph takes none; one of several scenes
  * (rt_render_batch) cannot be captured. */
 enum rt_render_mode { RT_RENDER_PLAIN = 0, RT_RENDER_WAVEFRONT = 1 };

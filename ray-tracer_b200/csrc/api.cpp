@@ -153,7 +153,7 @@ HandleCount::~HandleCount()
     std::lock_guard<std::mutex> lk(g_dev_mu);
     for (const cudaMemPool_t pool : g_pools)
     {
-        if (pool && cudaMemPoolTrimTo(pool, 0) != cudaSuccess) { cudaGetLastError(); }
+        if (pool && cudaMemPoolTrimTo(pool, SCRATCH_IDLE) != cudaSuccess) { cudaGetLastError(); }
     }
 }
 

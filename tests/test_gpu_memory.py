@@ -1,5 +1,5 @@
 """Device memory of renders and bakes. Renders: no more is kept than the documented bound however many
-handles render, all is given back with the last handle, renders on different streams do not wait for one
+handles render, most is given back with the last handle, renders on different streams do not wait for one
 another, and a render that finds less memory than it would like still gives the same image. Bakes: the
 scratch per triangle. The cases that fill the device or look at all of its memory run in a process of
 their own."""
@@ -54,7 +54,7 @@ for x in handles + [b]:
 del imgs
 gc.collect()
 torch.cuda.empty_cache()
-assert before - free() < 32 << 20, before - free()
+assert before - free() < (64 + 32) << 20, before - free()
 """)
 
 
@@ -72,7 +72,7 @@ def render(c, out, out2, handle):
     return code
 
 jobs = []
-for w, h, spp in ((1024, 1024, 32), (3001, 2200, 2)):
+for w, h, spp in ((1024, 1024, 32), (5001, 3000, 2)):
     jobs.append((cfg(w, h, spp), [torch.zeros(h, w, 3, device="cuda") for _ in range(4)]))
 torch.cuda.synchronize()  # (the renders run on the library's own stream)
 for c, t in jobs:
@@ -83,7 +83,7 @@ with torch.cuda.graph(graph):
 graph.replay()
 other = scene()[0]
 b.free()
-other.free()  # the last handles: the scratch is gone
+other.free()  # the last handles: most of the scratch is gone
 b = scene()[0]
 held, room = [], 48 << 20
 for size in (1 << 30, 64 << 20, 8 << 20):
@@ -92,7 +92,7 @@ for size in (1 << 30, 64 << 20, 8 << 20):
         if err != rt.cudaError_t.cudaSuccess:
             break
         held.append(p)
-assert 16 << 20 < free() < 79 << 20, free()  # 403 MB and 79 MB (a sample of every pixel) would be taken
+assert 16 << 20 < free() < 79 << 20, free()  # 403 MB and 180 MB (a sample of every pixel) would be taken; 64 MB may be in the pool
 for c, t in jobs:
     assert render(c, t[2], t[3], b) == 0, rtb200.lib().rt_last_error()
 for p in held:
