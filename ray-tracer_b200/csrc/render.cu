@@ -414,7 +414,7 @@ __device__ __forceinline__ f3 path_sample(const TraceCtx& T, const RP& P, const 
     f3 tp = mk3(1.f, 1.f, 1.f), L = mk3(0.f, 0.f, 0.f);
     for (uint32_t bounce = 0; bounce <= P.max_bounce; bounce++)
     {
-        const THit H = trace_ray<0>(T, o, d, tmin, bits2f(0x7f800000u));
+        const THit H = trace_ray(T, o, d, tmin, bits2f(0x7f800000u));
         if (REC) { rec[bounce] = H.hit ? H.tri : NO_TRI; }
         if (!H.hit)
         {
@@ -524,7 +524,7 @@ k_adjoint(TraceCtx T, RP P, Shade S, const float* __restrict__ dimg, float* __re
                 if (REC) { tri = rec[bounce]; }
                 else
                 {
-                    H = trace_ray<0>(T, o, d, tmin, bits2f(0x7f800000u));
+                    H = trace_ray(T, o, d, tmin, bits2f(0x7f800000u));
                     tri = H.hit ? H.tri : NO_TRI;
                 }
                 if (tri == NO_TRI) { alive = false; }

@@ -121,13 +121,12 @@ struct THit
 // re-test its entry distance against the best t, then test a leaf's triangles or push both
 // children, farther first. Used for trees with small leaves, where the while-while form's
 // meeting points cost more than they save.
-template <int MODE, int STK>
 __device__ __forceinline__ THit trace_ray_oneloop(const TraceCtx& T, const TraceRoot& R, rtd::f3 o, rtd::f3 d, float tmin,
                                                   float tmax)
 {
     using namespace rtd;
-    uint32_t sref[STK], scnt[STK];
-    float stn[STK];
+    uint32_t sref[STACK], scnt[STACK];
+    float stn[STACK];
     const f3 inv = mk3(1.f / d.x, 1.f / d.y, 1.f / d.z);
     THit H;
     H.t = tmax; H.u = 0.f; H.v = 0.f; H.tri = 0; H.hit = false; H.overflow = false;
@@ -147,22 +146,17 @@ __device__ __forceinline__ THit trace_ray_oneloop(const TraceCtx& T, const Trace
         if (cnt & LEAF_BIT)
         {
             const uint32_t c = cnt & ~LEAF_BIT;
-            bool done = false;
             for (uint32_t k = 0; k < c; k++)
             {
                 const uint32_t ti = ref + k;
                 const float4 p0 = __ldg(&T.tp[3 * ti]), p1 = __ldg(&T.tp[3 * ti + 1]), p2 = __ldg(&T.tp[3 * ti + 2]);
                 const f3 v0 = mk3(p0.x, p0.y, p0.z), v1 = mk3(p0.w, p1.x, p1.y), v2 = mk3(p1.z, p1.w, p2.x);
                 float t, u, v;
-                const bool acc = (MODE & 2) ? ray_tri_watertight(o, d, tmin, tmax, v0, v1, v2, t, u, v)
-                                            : ray_tri(o, d, tmin, tmax, v0, v1, v2, t, u, v);
-                if (acc && t < best)
+                if (ray_tri(o, d, tmin, tmax, v0, v1, v2, t, u, v) && t < best)
                 {
                     best = t; H.u = u; H.v = v; H.tri = ti; H.hit = true;
-                    if (MODE & 1) { done = true; break; }
                 }
             }
-            if (done) { break; }
         }
         else
         {
@@ -178,12 +172,12 @@ __device__ __forceinline__ THit trace_ray_oneloop(const TraceCtx& T, const Trace
             else { fr = dd.x; fc = dd.z; ft = tl; nr = dd.y; nc = dd.w; nt = tr; }
             if (ft < best)
             {
-                if (top >= STK) { H.overflow = true; break; }
+                if (top >= STACK) { H.overflow = true; break; }
                 sref[top] = fr; scnt[top] = fc; stn[top] = ft; top++;
             }
             if (nt < best)
             {
-                if (top >= STK) { H.overflow = true; break; }
+                if (top >= STACK) { H.overflow = true; break; }
                 sref[top] = nr; scnt[top] = nc; stn[top] = nt; top++;
             }
         }
@@ -200,12 +194,11 @@ __device__ __forceinline__ THit trace_ray_oneloop(const TraceCtx& T, const Trace
 // {reference, count, entry distance}. The visiting order, the pop-time test "entry distance >=
 // best t" and the points where a 64-entry stack would overflow (the held node counts as its
 // stack entry) are those of the one-loop form of the reference's traverse().
-template <int MODE, int STK>
 __device__ __forceinline__ THit trace_ray_ww(const TraceCtx& T, const TraceRoot& R, rtd::f3 o, rtd::f3 d, float tmin,
                                              float tmax)
 {
     using namespace rtd;
-    uint4 stk[STK];
+    uint4 stk[STACK];
     const f3 inv = mk3(1.f / d.x, 1.f / d.y, 1.f / d.z);
     THit H;
     H.t = tmax; H.u = 0.f; H.v = 0.f; H.tri = 0; H.hit = false; H.overflow = false;
@@ -247,10 +240,10 @@ __device__ __forceinline__ THit trace_ray_ww(const TraceCtx& T, const TraceRoot&
             {
                 if (ft < best)
                 {
-                    if (top >= STK) { H.overflow = true; have = false; break; }
+                    if (top >= STACK) { H.overflow = true; have = false; break; }
                     stk[top++] = make_uint4(fr, fc, __float_as_uint(ft), 0u);
                 }
-                if (top >= STK) { H.overflow = true; have = false; break; }
+                if (top >= STACK) { H.overflow = true; have = false; break; }
                 cref = nr; ccnt = nc;
             }
             else { pop(); }
@@ -258,22 +251,17 @@ __device__ __forceinline__ THit trace_ray_ww(const TraceCtx& T, const TraceRoot&
         if (!have) { break; }
         // a leaf: its triangles in order, strict "t < best" (bvh_traverse.cpp:112-142)
         const uint32_t cnt = ccnt & ~LEAF_BIT;
-        bool done = false;
         for (uint32_t k = 0; k < cnt; k++)
         {
             const uint32_t ti = cref + k;
             const float4 p0 = __ldg(&T.tp[3 * ti]), p1 = __ldg(&T.tp[3 * ti + 1]), p2 = __ldg(&T.tp[3 * ti + 2]);
             const f3 v0 = mk3(p0.x, p0.y, p0.z), v1 = mk3(p0.w, p1.x, p1.y), v2 = mk3(p1.z, p1.w, p2.x);
             float t, u, v;
-            const bool acc = (MODE & 2) ? ray_tri_watertight(o, d, tmin, tmax, v0, v1, v2, t, u, v)
-                                        : ray_tri(o, d, tmin, tmax, v0, v1, v2, t, u, v);
-            if (acc && t < best)
+            if (ray_tri(o, d, tmin, tmax, v0, v1, v2, t, u, v) && t < best)
             {
                 best = t; H.u = u; H.v = v; H.tri = ti; H.hit = true;
-                if (MODE & 1) { done = true; break; }
             }
         }
-        if (done) { break; }
         pop();
     }
     H.t = best;
@@ -384,24 +372,13 @@ __device__ __forceinline__ THit trace_ray_wide(const TraceCtx& T, const TraceRoo
     return H;
 }
 
-// Closest hit (MODE bit 0 clear) or first accepted hit (bit 0 set); bit 1 selects the
-// watertight triangle test. Reproduces the reference's visiting order exactly, in either loop
-// form (T.ww picks one per tree; both visit the same nodes in the same order). STK entries of
-// stack: the loop holds at most one entry per level of the tree plus one, so a stack deeper
-// than the tree never overflows (overflow is reported, never silent). R: the subtree to trace.
-template <int MODE, int STK = STACK>
-__device__ __forceinline__ THit trace_ray(const TraceCtx& T, const TraceRoot& R, rtd::f3 o, rtd::f3 d, float tmin,
-                                          float tmax)
-{
-    return T.ww ? trace_ray_ww<MODE, STK>(T, R, o, d, tmin, tmax) : trace_ray_oneloop<MODE, STK>(T, R, o, d, tmin, tmax);
-}
-
-// The whole tree (the handle's root record).
-template <int MODE, int STK = STACK>
+// The closest hit in the whole tree, in the reference's visiting order in either loop form (T.ww picks
+// one per tree; both visit the same nodes in the same order). The loop holds at most one stack entry
+// per level of the tree plus one (overflow is reported, never silent).
 __device__ __forceinline__ THit trace_ray(const TraceCtx& T, rtd::f3 o, rtd::f3 d, float tmin, float tmax)
 {
     const TraceRoot R = *T.root;
-    return trace_ray<MODE, STK>(T, R, o, d, tmin, tmax);
+    return T.ww ? trace_ray_ww(T, R, o, d, tmin, tmax) : trace_ray_oneloop(T, R, o, d, tmin, tmax);
 }
 
 // Interpolated shading normal of a hit: normalize(w n0 + u n1 + v n2), bvh_traverse.cpp:135-139.

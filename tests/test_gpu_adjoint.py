@@ -193,3 +193,27 @@ def test_adjoint_skips_zero_weight_pixels_and_validates():
     assert not g.any() and not e.any()
     with pytest.raises(rtb200.RtError):
         b.adjoint(rtb200.render_cfg(0, 16, 4), torch.zeros((0, 16, 3), device="cuda"))
+
+
+@pytest.mark.parametrize("loop", [0, 1])
+@pytest.mark.parametrize("preset", ["lbvh30", "sah4", "hybrid"])
+def test_adjoint_in_both_loop_forms_matches_oracle_fp64(orc, preset, loop):
+    """The adjoint's traversal has a loop for small leaves and one for large ones (rt_bvh_trace_loop 0 and
+    1): each gives the oracle's gradients on trees of either kind."""
+    sc = small_scene(3)
+    b = rtb200.Bvh.build(sc.verts, sc.tris, preset)
+    b.trace_loop(loop)
+    prim = b.prim_ids()
+    mot = sc.baked_materials(prim)
+    rng = np.random.default_rng(5)
+    talb = rng.uniform(0.2, 0.8, size=(sc.tris.shape[0], 3)).astype(np.float32)[prim]
+    rc = rcfg(40, 32, 8, max_bounce=4, rr_after=1)
+    d = rng.uniform(0.5, 1.5, size=(rc.height, rc.width, 3)).astype(np.float32)
+    g, e = b.adjoint(rc, torch.from_numpy(d).cuda(), sc.mats, mot, tri_albedo=talb)
+    go, eo = orc.adjoint(Baked(*b.download()), orc_cfg_from(rc), d, sc.mats, mot, talb, threads=8)
+    g, e = g.cpu().numpy().astype(np.float64), e.cpu().numpy().astype(np.float64)
+    # the bars of the case above: the same paths but where host and device cosf/sinf differ by an ulp
+    assert np.linalg.norm(g - go) / np.linalg.norm(go) < 2e-3
+    close = np.abs(g - go) <= 1e-4 * np.abs(go) + 1e-6 * np.abs(go).max()
+    assert close.mean() > 0.97, close.mean()
+    assert np.allclose(e, eo, rtol=2e-3, atol=1e-6 * np.abs(eo).max()), (e, eo)
