@@ -14,7 +14,7 @@ reference's own CPU bake timed on this host, and under "render" the path-loop wo
 plain path tracing (256x256, 16 spp, depth 4, Cornell box + 20,480-triangle icosphere + two
 spheres; plain vs wavefront, and the CPU restatement on all host cores), the batched workload
 (64 scenes of 1,000-500,000 triangles built in one launch sequence and rendered at 512x512,
-4 spp, depth 5 by the graph-replayed wavefront vs the plain kernel per scene), the adjoint
+4 spp, depth 5 in one call vs scene by scene), the adjoint
 (512x512, 32 spp, depth 4, Cornell box + 50,000-triangle icosphere: adjoint / forward time)
 and the large render (1920x1080, 64 spp, depth 8, roulette after bounce 2, 5,000,000
 triangles, binned SAH with spatial splits).
@@ -550,7 +550,7 @@ def _trace_ceiling(b, verts, stream, dev, n=1 << 22):
 
 
 def profiled_render_counters(key):
-    """Issue-slot and cache figures of a path-loop kernel from the committed ncu summaries
+    """Issue-slot and cache figures of the path kernel from the committed ncu summaries
     (profiles/render_kernels_<workload>.md: lines `key: name=value, ...`), if present."""
     path = os.path.join(HERE, "profiles", f"render_kernels_{key.split('_')[0]}.md")
     try:
@@ -562,7 +562,7 @@ def profiled_render_counters(key):
     return None
 
 
-def _render_roofline(counts, samples_counted, samples, ms, ceiling, kernel, counters_key=None):
+def _render_roofline(counts, samples_counted, samples, ms, ceiling, kernel, counters_key=None, counters_of=None):
     """Traversal roofline of a path-loop workload: segments traced per second against the
     incoherent-ray closest-hit rate on the same BVH; the traversal work per sample (nodes
     popped and triangles tested, 48 bytes each: a node's two child boxes and references, a
@@ -579,6 +579,7 @@ def _render_roofline(counts, samples_counted, samples, ms, ceiling, kernel, coun
            "counted_samples": int(samples_counted)}
     if counters_key:
         out["ncu"] = profiled_render_counters(counters_key)
+        out["ncu_of"] = f"k_paths, {counters_of}"
     return out
 
 
@@ -626,7 +627,7 @@ def render_c1(stream, dev):
         "wavefront_ms": round(tw, 3),
         "wavefront_vs_plain_max_rel_diff": float(((iw64 - ip64).abs().max() / ip64.abs().max()).item()),
         "roofline": _render_roofline(counts, 256 * rows * 16, n, min(tp, tw), ceiling,
-                                     "wavefront" if tw < tp else "plain", "c1_wavefront_trace"),
+                                     "wavefront" if tw < tp else "plain", "c1_wavefront_trace", "this image"),
         "cpu_baseline": {"value": round(256 * rows * 16 / cpu_s / 1e6, 4), "unit": "Mpx*spp/s", "cores": cores,
                          "kind": "port (the oracle's restated path loop over the reference traversal)",
                          "sample": f"{rows} image rows (of 256) at 16 spp, scaled to the metric"},
@@ -638,8 +639,8 @@ def render_c1(stream, dev):
 
 def render_c3(stream, dev):
     """Batched: 64 scenes of 1,000-500,000 triangles built in one launch sequence and rendered
-    at 512 x 512, 4 spp, depth 5 by the graph-replayed wavefront (autotuned) vs the plain kernel
-    per scene; CPU leg: the reference's bake plus the restated path loop per scene, on a subset."""
+    at 512 x 512, 4 spp, depth 5 in one call (autotuned) vs a plain render per
+    scene; CPU leg: the reference's bake plus the restated path loop per scene, on a subset."""
     import numpy as np
     import torch
     import rtb200
@@ -716,7 +717,8 @@ def render_c3(stream, dev):
         "autotuned": tuned.as_dict(), "autotune_s": round(tune_s, 2),
         "batched_vs_plain_max_rel_diff": max(diffs),
         "roofline": _render_roofline(counts, len(sub) * 8 * 512 * 4, nb, tbr, statistics.mean(ceil),
-                                     "batched wavefront (autotuned)", "c3_wavefront_trace"),
+                                     "batched wavefront (autotuned)", "c3_wavefront_trace",
+                                     "16 scenes of 1,000-100,000 triangles at 256x256"),
         "cpu_baseline": {"value": round(nb / cpu_total_s / 1e6, 4), "unit": "Mpx*spp/s (bake + render)", "cores": cores,
                          "kind": "reference bake + port (the oracle's restated path loop)",
                          "sample": f"scenes {sub}: the reference's bake of each (1 thread, {bake_s:.2f} s) and the "
@@ -804,7 +806,7 @@ def render_c5(stream, dev):
         "plain_ms": round(tlp, 1), "wavefront_ms": round(tlw, 1), "wavefront_tuned_ms": round(tlt, 1),
         "roofline": _render_roofline(counts, 1920 * (rows[1] - rows[0]) * 64, nl, best, ceiling,
                                      {tlp: "plain", tlw: "wavefront", tlt: "wavefront (autotuned)"}[best],
-                                     "c5_wavefront_trace"),
+                                     "c5_wavefront_trace", "400 icospheres x 2,500 triangles, 4 spp"),
         "cpu_baseline": {"value": round(1920 * (rows[1] - rows[0]) * 64 / cpu_s / 1e6, 4), "unit": "Mpx*spp/s",
                          "cores": cores, "kind": "port (the oracle's restated path loop over the reference traversal)",
                          "sample": f"rows {rows[0]}-{rows[1] - 1} of 1080 at 64 spp, scaled to the metric"}}

@@ -253,7 +253,8 @@ struct PathShare
 };
 // The radiance of every path. OWN: a lane takes whole pixels, adds their samples to the images itself,
 // in the order and with the roundings of k_sum, and needs no memory besides: for renders that may not
-// have any (run_paths). Half as fast where the pixels do not fill the chip.
+// have any, and single samples (run_paths). Small Cornell box, 4 bounces: 256 x 256 x 16 4.2 ms against 1.5, where its
+// pixels leave half of the lanes idle, 1080p x 16 39 against 29 ms.
 template <int STK, bool OWN>
 __global__ void __launch_bounds__(256, 4)
 k_paths(const TraceCtx T, const __grid_constant__ PathJob J, uint32_t* __restrict__ counter, int per_warp)

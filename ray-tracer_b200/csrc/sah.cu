@@ -3052,7 +3052,9 @@ k_sah_emit(const OutNode* __restrict__ out, uint32_t n_out, const SahRoot* __res
     }
 }
 
-// Levels of at most this many nodes per SM clip with 12 warps a node.
+// Levels of at most this many nodes per SM clip with 12 warps a node. Hybrid bake of a 300,000-triangle
+// mesh, rebuilt on the device: 4.09 ms, 4.61 with 4 warps everywhere and 4.08 with 12; its SAH leaf 4 bake 6.90, 6.92
+// and 7.86; 1M soup, SAH leaf 4: 11.9, 11.9 and 12.5.
 constexpr uint32_t CLIP_FEW = 32;
 
 inline uint32_t nblk(uint64_t n) { return (uint32_t)((n + SBLK - 1) / SBLK); }

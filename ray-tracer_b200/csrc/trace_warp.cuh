@@ -16,8 +16,8 @@
 // 2,097,152 incoherent rays, 1M-triangle soup: LBVH (leaf 16) 15.7 -> 6.5 ms, SAH (leaf 4)
 // 11.4 -> 6.0 ms; 1080p primary plus shadow rays, 1M triangles, hybrid tree: 3.07 -> 1.96 ms.
 //
-// The rest of the time goes to L1 (node and triangle fetches, stacks: 55-73 % of its wavefronts)
-// and issue slots (50-70 %) with 17-21 lanes busy. Hence the 8-byte stack entries (16 bytes: 8.2 ms on the
+// The rest of the time goes to L1 (node and triangle fetches, stacks: 60-78 % of its wavefronts)
+// and issue slots (49-74 %) with 17-21 lanes busy. Hence the 8-byte stack entries (16 bytes: 8.2 ms on the
 // SAH tree -- the stacks of an SM alone filled its L1), the top entry kept in registers, nodes
 // fetched with two 256-bit loads, and rays and hits kept in shared memory rather than in
 // registers (64 registers, four blocks of 256 threads per SM; 80 registers 5-10 % slower). Slower too:
