@@ -17,7 +17,7 @@ namespace
 
 // Two tile shapes (threads, keys per thread, blocks per SM): up to 2^21 keys 4,096 keys on 512
 // threads (100,000 keys: 50 us a sort, 54 on 256 threads of 16 keys); above, 4,608 keys on 384
-// threads. A pass is bound by issue slots (65 % used; ranking, not memory, takes most of them), so
+// threads. A pass is bound by issue slots (51 % used at 4M keys, 18 % of the DRAM rate; ranking, not memory, takes most of them), so
 // the long passes want both many warps and few instructions per key for the tile's own work: at
 // 16.8M keys a sort takes 0.75 ms with 384 x 12, 0.77 with 384 x 13, 0.81 with 384 x 10, 0.83 with
 // 256 x 13 or 512 x 12 and 0.86 with 256 x 8.
@@ -404,6 +404,54 @@ __global__ void __launch_bounds__(256) k_settle(const K* __restrict__ kin, const
 {
     if (*path == SORT_RUNS) { return; }
     for (uint32_t i = blockIdx.x * 256u + threadIdx.x; i < n; i += gridDim.x * 256u) { kout[i] = kin[i]; vout[i] = vin[i]; }
+}
+
+// A large sort of 7 or 8 digits: the top four by passes, then the runs, or all digits (above).
+template <typename K>
+int sort_by_runs(K* keys, uint32_t* vals, bool vals_identity, uint32_t n, int passes, const uint32_t* hist, K* kalt,
+                 uint32_t* valt, uint32_t* lookback, size_t lbw, uint32_t* tickets, uint32_t* status, cudaStream_t st,
+                 K** keys_out, uint32_t** vals_out, bool scratch_zeroed)
+{
+    const int identity = vals_identity ? 1 : 0;
+    const int low_bits = 8 * (passes - TOP_PASSES);
+    uint32_t* path = tickets + 64;
+    static PerDeviceOnce attr;  // per key type and device
+    if (int e = attr.once([] {
+            RT_CUDA(cudaFuncSetAttribute(k_crowded<K>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)(CR_TABLE * 8)));
+            return (int)RT_OK;
+        }))
+    {
+        return e;
+    }
+    k_crowded<K><<<1, 1024, CR_TABLE * 8, st>>>(keys, n, low_bits, path);
+    K* ktop = nullptr;
+    uint32_t* vtop = nullptr;
+    if (int e = onesweep_passes<K, RS_LB, RS_LI, RS_LM>(keys, vals, identity, n, passes - TOP_PASSES, passes, hist, kalt, valt,
+                                                        lookback, tickets, status, st, &ktop, &vtop, path, SORT_CROWDED,
+                                                        scratch_zeroed))
+    {
+        return e;
+    }
+    // an even number of passes: the keys are back in their own buffers
+    k_runs<K><<<(n + 255) / 256, 256, 0, st>>>(ktop, vtop, n, low_bits, n / RUN_DIV, kalt, valt, path);
+    const uint32_t blocks = 8u * (uint32_t)device_sm_count();
+    k_undone<<<blocks, 256, 0, st>>>(lookback, lbw, tickets, path);
+    count_launch(3);
+    K* klsd = nullptr;
+    uint32_t* vlsd = nullptr;
+    if (int e = onesweep_passes<K, RS_LB, RS_LI, RS_LM>(keys, vals, identity ? 2 : 0, n, 0, passes, hist, kalt, valt, lookback,
+                                                        tickets, status, st, &klsd, &vlsd, path, SORT_RUNS, true))
+    {
+        return e;
+    }
+    if (klsd != kalt)
+    {
+        k_settle<K><<<blocks, 256, 0, st>>>(klsd, vlsd, n, kalt, valt, path);
+        count_launch();
+    }
+    *keys_out = kalt;
+    *vals_out = valt;
+    return check_launch("radix sort");
 }
 
 // ---- MSD path: one onesweep pass on the most significant digit, then every bucket of that
@@ -847,53 +895,17 @@ int radix_sort_pairs(K* keys, uint32_t* vals, bool vals_identity, uint32_t n, in
     }
     uint32_t* lookback = s.lookback.as<uint32_t>();
     uint32_t* tickets = s.tile_counters.as<uint32_t>();
-    K* kalt = s.keys_alt.as<K>();
-    uint32_t* valt = s.vals_alt.as<uint32_t>();
-    const int identity = vals_identity ? 1 : 0;
-    if (passes < TOP_PASSES + 3)
+    if constexpr (sizeof(K) == 8)  // (32-bit keys have too few digits)
     {
-        return onesweep_passes<K, RS_LB, RS_LI, RS_LM>(keys, vals, identity, n, 0, passes, hist, kalt, valt, lookback, tickets,
-                                                       status, st, keys_out, vals_out, nullptr, 0u, scratch_zeroed);
+        if (passes >= TOP_PASSES + 3)
+        {
+            return sort_by_runs<K>(keys, vals, vals_identity, n, passes, hist, s.keys_alt.as<K>(), s.vals_alt.as<uint32_t>(),
+                                   lookback, lbw, tickets, status, st, keys_out, vals_out, scratch_zeroed);
+        }
     }
-    const int low_bits = 8 * (passes - TOP_PASSES);
-    uint32_t* path = tickets + 64;
-    static PerDeviceOnce attr;  // per key type and device
-    if (int e = attr.once([] {
-            RT_CUDA(cudaFuncSetAttribute(k_crowded<K>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)(CR_TABLE * 8)));
-            return (int)RT_OK;
-        }))
-    {
-        return e;
-    }
-    k_crowded<K><<<1, 1024, CR_TABLE * 8, st>>>(keys, n, low_bits, path);
-    K* ktop = nullptr;
-    uint32_t* vtop = nullptr;
-    if (int e = onesweep_passes<K, RS_LB, RS_LI, RS_LM>(keys, vals, identity, n, passes - TOP_PASSES, passes, hist, kalt, valt,
-                                                        lookback, tickets, status, st, &ktop, &vtop, path, SORT_CROWDED,
-                                                        scratch_zeroed))
-    {
-        return e;
-    }
-    // an even number of passes: the keys are back in their own buffers
-    k_runs<K><<<(n + 255) / 256, 256, 0, st>>>(ktop, vtop, n, low_bits, n / RUN_DIV, kalt, valt, path);
-    const uint32_t blocks = 8u * (uint32_t)device_sm_count();
-    k_undone<<<blocks, 256, 0, st>>>(lookback, lbw, tickets, path);
-    count_launch(3);
-    K* klsd = nullptr;
-    uint32_t* vlsd = nullptr;
-    if (int e = onesweep_passes<K, RS_LB, RS_LI, RS_LM>(keys, vals, identity ? 2 : 0, n, 0, passes, hist, kalt, valt, lookback,
-                                                        tickets, status, st, &klsd, &vlsd, path, SORT_RUNS, true))
-    {
-        return e;
-    }
-    if (klsd != kalt)
-    {
-        k_settle<K><<<blocks, 256, 0, st>>>(klsd, vlsd, n, kalt, valt, path);
-        count_launch();
-    }
-    *keys_out = kalt;
-    *vals_out = valt;
-    return check_launch("radix sort");
+    return onesweep_passes<K, RS_LB, RS_LI, RS_LM>(keys, vals, vals_identity ? 1 : 0, n, 0, passes, hist, s.keys_alt.as<K>(),
+                                                   s.vals_alt.as<uint32_t>(), lookback, tickets, status, st, keys_out,
+                                                   vals_out, nullptr, 0u, scratch_zeroed);
 }
 
 template int radix_sort_pairs<uint64_t>(uint64_t*, uint32_t*, bool, uint32_t, int, const uint32_t*, const uint32_t*,
