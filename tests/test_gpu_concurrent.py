@@ -66,3 +66,25 @@ def test_host_traces():
     in_threads(len(rays), work)
     for k, w in enumerate(want):
         assert len(got[k]) == 3 and all(g.tobytes() == w.tobytes() for g in got[k]), k
+
+
+def test_renders():
+    """Images of different sizes and sample counts, whose scratch differs, some without any."""
+    import numpy as np
+    from test_gpu_paths import VIEW, scene
+    b, mats, mot = scene("hybrid")
+    dm, dmot = torch.from_numpy(rtb200.materials_array(mats)).cuda(), torch.from_numpy(mot.astype(np.int32)).cuda()
+    cfgs = [rtb200.render_cfg(64 + 48 * k, 40 + 8 * k, 1 + k % 5, max_bounce=4, rr_after=1, env_kind=1, seed=k, lookat=VIEW)
+            for k in range(8)]
+    want = [b.render(c, dm, dmot, want_sq=True) for c in cfgs]
+    got = [[] for _ in cfgs]
+
+    def work(k):
+        with torch.cuda.stream(torch.cuda.Stream()):
+            for i in range(6):
+                got[k].append(b.render(cfgs[k], dm, dmot, mode=i % 2, want_sq=True))
+            torch.cuda.current_stream().synchronize()
+
+    in_threads(len(cfgs), work)
+    for k, w in enumerate(want):
+        assert len(got[k]) == 6 and all(torch.equal(g[0], w[0]) and torch.equal(g[1], w[1]) for g in got[k]), k

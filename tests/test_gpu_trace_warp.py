@@ -123,8 +123,8 @@ def test_stack_overflow_is_reported(n):
 
 def test_axis_parallel_rays_cost_what_others_do():
     """Orthographic rays (two direction components 0) take the general box test at every node, with the
-    reciprocals of the ray's start: the same grid tilted a little takes the same nodes without it. 1.09-1.11 times
-    the time on a B200; 1.27-1.36 while the reciprocals were taken again at every node."""
+    reciprocals of the ray's start: the same grid tilted a little takes the same nodes without it. 1.11-1.12 times
+    the time on a B200; 1.40 while the reciprocals were taken again at every node."""
     v, t = scenes.icosphere(6, seed=2)
     b = rtb200.Bvh.build(v, t, "sah4")
     n = 1024
