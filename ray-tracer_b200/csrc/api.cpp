@@ -53,6 +53,7 @@ int DevBuf::ensure(size_t n)
     if (e != cudaSuccess)
     {
         p = nullptr;
+        cudaGetLastError();  // (a later call's launch check would report it again)
         set_error(std::string("cudaMalloc(") + std::to_string(want) + "): " + cudaGetErrorString(e));
         return RT_E_CUDA;
     }

@@ -137,3 +137,32 @@ before = free()
 b = rtb200.Bvh.build(*g, "hybrid")
 assert (before - free()) / n < 1470, (before - free()) / n
 """)
+
+
+def test_a_failed_allocation_fails_its_own_call_only():
+    in_process("""
+from rtb200 import scenes
+small, large = scenes.soup(3000, seed=1), scenes.soup(1 << 20, seed=2)
+b = rtb200.Bvh.build(*small, "lbvh63")
+rays = torch.from_numpy(scenes.incoherent_rays(5000, [0, 0, 0], [1, 1, 1], seed=4)).cuda()
+want = b.trace(rays)
+held = []
+for size in (1 << 30, 64 << 20):
+    while free() > size + (96 << 20):
+        err, p = rt.cudaMalloc(size)
+        if err != rt.cudaError_t.cudaSuccess:
+            break
+        held.append(p)
+assert free() < 300 << 20  # a 1M-triangle bake takes about 900 MB
+code = None
+try:
+    rtb200.Bvh.build(*large, "lbvh63")
+except rtb200.RtError as e:
+    code = e.code
+assert code == 6, code
+got = b.trace(rays)
+assert torch.equal(got.view(torch.int32), want.view(torch.int32))
+for p in held:
+    rt.cudaFree(p)
+rtb200.Bvh.build(*large, "lbvh63")
+""")
